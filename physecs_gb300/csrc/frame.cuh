@@ -80,10 +80,10 @@ struct FrameBuf {
     // colouring
     unsigned long long* claim;  // [n_dyn] (hashed priority << 32 | contact index)
     int* color_of;        // [man_cap]
-    int* corder;          // [man_cap] manifolds sorted by (scene, colour, index)
+    int* corder;          // [man_cap] manifolds sorted by (scene, colour, points)
     int* scene_ncolor;    // [S]
-    int* color_start;     // [S * (kMaxColors+1)]
-    int* claim_pos;       // [S * (kMaxColors+1)] scatter counters
+    int* color_start;     // [S * kColorBins] contacts per bin of a scene solved by several blocks
+    int* claim_pos;       // [S * kColorBins] scatter counters of the same scenes
     // per-substep contact records of scenes whose records do not fit in shared memory
     int* pt_off;          // [man_cap] first point of each contact, colour order
     int2* cbody;          // [man_cap] colouring: scene-local dynamic bodies of each contact

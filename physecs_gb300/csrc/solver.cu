@@ -362,50 +362,62 @@ __device__ void row_presolve(const World& w, Row& r, bool simd) {
     }
 }
 
-// Body velocities the iterations work on, as six float arrays of n entries:
-//   - in this block's shared memory (s != null, body d at index d - off);
-//   - spread over the blocks of a thread-block cluster (rs != null: body d at block
-//     (d - off) mod 2^lg, index (d - off) >> lg, through distributed shared memory);
-//   - else the world's vt arrays.
-struct VelRef {
-    float* s;
+// The dynamic shared memory of the solver kernels: velocities, then contact records.
+extern __shared__ float4 smem[];
+
+// Body velocities the iterations work on, by scene-local dynamic body:
+//   - SmemVel: in this block's shared memory, 24 bytes a body from its start, read and
+//     written as three 8-byte words;
+//   - ClusterVel: spread over the blocks of a thread-block cluster through distributed
+//     shared memory (body i at block i mod 2^lg, index i >> lg), six float arrays of n;
+//   - GlobVel: the world's vt arrays from the scene's first body on.
+// Each view is its own type so that every access has one known address space.
+struct SmemVel {
+    __device__ __forceinline__ void ld(int i, V3& v, V3& w) const {
+        const float2* p = (const float2*)smem + 3 * i;
+        const float2 a = p[0], b = p[1], c = p[2];
+        v = {a.x, a.y, b.x};
+        w = {b.y, c.x, c.y};
+    }
+    __device__ __forceinline__ void st(int i, V3 v, V3 w) const {
+        float2* p = (float2*)smem + 3 * i;
+        p[0] = make_float2(v.x, v.y);
+        p[1] = make_float2(v.z, w.x);
+        p[2] = make_float2(w.y, w.z);
+    }
+};
+struct ClusterVel {
     float* const* rs;
-    float4* v;
-    float4* w;
-    int off, n, lg;
-    __device__ __forceinline__ float* base(int d, int& j) const {
-        int i = d - off;
-        if (rs) { j = i >> lg; return rs[i & ((1 << lg) - 1)]; }
-        j = i;
-        return s;
+    int n, lg;
+    __device__ __forceinline__ void ld(int i, V3& v, V3& w) const {
+        const float* b = rs[i & ((1 << lg) - 1)] + (i >> lg);
+        v = {b[0], b[n], b[2 * n]};
+        w = {b[3 * n], b[4 * n], b[5 * n]};
     }
-    __device__ __forceinline__ V3 lv(int d) const {
-        if (s || rs) { int j; const float* b = base(d, j); return {b[j], b[n + j], b[2 * n + j]}; }
-        return ld3(v[d]);
+    __device__ __forceinline__ void st(int i, V3 v, V3 w) const {
+        float* b = rs[i & ((1 << lg) - 1)] + (i >> lg);
+        b[0] = v.x; b[n] = v.y; b[2 * n] = v.z;
+        b[3 * n] = w.x; b[4 * n] = w.y; b[5 * n] = w.z;
     }
-    __device__ __forceinline__ V3 lw(int d) const {
-        if (s || rs) { int j; const float* b = base(d, j); return {b[3 * n + j], b[4 * n + j], b[5 * n + j]}; }
-        return ld3(w[d]);
-    }
-    __device__ __forceinline__ void sv(int d, V3 x) const {
-        if (s || rs) { int j; float* b = base(d, j); b[j] = x.x; b[n + j] = x.y; b[2 * n + j] = x.z; }
-        else v[d] = st4(x);
-    }
-    __device__ __forceinline__ void sw(int d, V3 x) const {
-        if (s || rs) { int j; float* b = base(d, j); b[3 * n + j] = x.x; b[4 * n + j] = x.y; b[5 * n + j] = x.z; }
-        else w[d] = st4(x);
-    }
+};
+struct GlobVel {
+    float4* v_;
+    float4* w_;
+    __device__ __forceinline__ void ld(int i, V3& v, V3& w) const { v = ld3(v_[i]); w = ld3(w_[i]); }
+    __device__ __forceinline__ void st(int i, V3 v, V3 w) const { v_[i] = st4(v); w_[i] = st4(w); }
 };
 
 // Constraint1D(W)::solve for one row (Constraint1D.cpp:54-127 / Constraint1DW.cpp:117-233)
-__device__ void row_solve(const World& w, Row& r, float h, bool warm, bool simd, const VelRef vr) {
+template <class V>
+__device__ void row_solve(Row& r, float h, bool warm, bool simd, int ds, const V vr) {
     int fl = r.flags;
     bool angf = fl & 2, soft = fl & 1, lim = fl & 4;
     float inv = r.angular1t.w;
     if (!simd && !inv) return;
+    // an angular row neither uses nor changes the linear velocities
     V3 v0 = {0, 0, 0}, w0 = {0, 0, 0}, v1 = {0, 0, 0}, w1 = {0, 0, 0};
-    if (r.b0 >= 0) { if (!angf) v0 = vr.lv(r.b0); w0 = vr.lw(r.b0); }
-    if (r.b1 >= 0) { if (!angf) v1 = vr.lv(r.b1); w1 = vr.lw(r.b1); }
+    if (r.b0 >= 0) vr.ld(r.b0 - ds, v0, w0);
+    if (r.b1 >= 0) vr.ld(r.b1 - ds, v1, w1);
     V3 l0t = ld3(r.linear0t), l1t = ld3(r.linear1t), a0t = ld3(r.angular0t), a1t = ld3(r.angular1t);
     float c = r.angular0.w;
     if (!soft && warm) {
@@ -467,20 +479,20 @@ __device__ void row_solve(const World& w, Row& r, float h, bool warm, bool simd,
     if (!simd) {
         // the scalar row applies only this iteration's impulse (Constraint1D.cpp:158-168)
         if (r.b0 >= 0) {
-            if (!angf) vr.sv(r.b0, vr.lv(r.b0) + lambda * l0t);
-            vr.sw(r.b0, vr.lw(r.b0) + lambda * a0t);
+            vr.ld(r.b0 - ds, v0, w0);
+            vr.st(r.b0 - ds, angf ? v0 : v0 + lambda * l0t, w0 + lambda * a0t);
         }
         if (r.b1 >= 0) {
-            if (!angf) vr.sv(r.b1, vr.lv(r.b1) - lambda * l1t);
-            vr.sw(r.b1, vr.lw(r.b1) - lambda * a1t);
+            vr.ld(r.b1 - ds, v1, w1);
+            vr.st(r.b1 - ds, angf ? v1 : v1 - lambda * l1t, w1 - lambda * a1t);
         }
         return;
     }
     if (!angf) { v0 += lambda * l0t; v1 -= lambda * l1t; }
     w0 += lambda * a0t;
     w1 -= lambda * a1t;
-    if (r.b0 >= 0) { if (!angf) vr.sv(r.b0, v0); vr.sw(r.b0, w0); }
-    if (r.b1 >= 0) { if (!angf) vr.sv(r.b1, v1); vr.sw(r.b1, w1); }
+    if (r.b0 >= 0) vr.st(r.b0 - ds, v0, w0);
+    if (r.b1 >= 0) vr.st(r.b1 - ds, v1, w1);
 }
 
 __constant__ int c_flag_order[6] = {0, 2, 1, 4, 3, 6};
@@ -493,12 +505,13 @@ __device__ void joint_presolve(const World& w, int j) {
             if (J.rowflags[k] == c_flag_order[fi]) row_presolve(w, R[k], J.simd != 0);
 }
 
-__device__ void joint_solve(const World& w, int j, float h, bool warm, const VelRef vr) {
+template <class V>
+__device__ void joint_solve(const World& w, int j, float h, bool warm, int ds, const V vr) {
     JointDev& J = w.joints[j];
     Row* R = w.rows + j * kMaxRowsPerJoint;
     for (int fi = 0; fi < 6; ++fi)
         for (int k = 0; k < J.nrows; ++k)
-            if (J.rowflags[k] == c_flag_order[fi]) row_solve(w, R[k], h, warm, J.simd != 0, vr);
+            if (J.rowflags[k] == c_flag_order[fi]) row_solve(R[k], h, warm, J.simd != 0, ds, vr);
 }
 
 // ---------------------------------------------------------------- contacts (ContactConstraints.cpp)
@@ -509,7 +522,7 @@ __device__ __forceinline__ M3 world_invI(const World& w, int d) {
 
 
 // update contact rows (src/Physecs.cpp:366-427)
-__device__ void contact_update(const World& w, Contact& c, SHdr& H, SPt* P) {
+__device__ void contact_update(const World& w, Contact& c, int ds, SHdr& H, SPt* P) {
     int4 i0 = w.info[c.body0], i1 = w.info[c.body1];
     Q4 q0 = ld4(w.quat[c.body0]), q1 = ld4(w.quat[c.body1]);
     V3 com0 = {0, 0, 0}, v0 = {0, 0, 0}, w0 = {0, 0, 0}, com1 = {0, 0, 0}, v1 = {0, 0, 0}, w1 = {0, 0, 0};
@@ -518,8 +531,8 @@ __device__ void contact_update(const World& w, Contact& c, SHdr& H, SPt* P) {
     V3 n = ld3(c.n);
     H.n = c.n;
     H.m = make_float4(c.b0 >= 0 ? w.com[c.b0].w : 0.f, c.b1 >= 0 ? w.com[c.b1].w : 0.f, c.frequency, c.damping);
-    H.i.x = c.b0;
-    H.i.y = c.b1;
+    H.i.x = c.b0 >= 0 ? c.b0 - ds : -1;
+    H.i.y = c.b1 >= 0 ? c.b1 - ds : -1;
     H.i.z = c.np | (c.soft << 8);
     for (int k = 0; k < c.np; ++k) {
         ContactPt& p = c.p[k];
@@ -544,8 +557,8 @@ __device__ void contact_update(const World& w, Contact& c, SHdr& H, SPt* P) {
 
 // ContactConstraints::preSolve (src/ContactConstraints.cpp:4-31) and the per-substep
 // constants of solve (:33-101)
-__device__ void contact_presolve(const World& w, SHdr& H, SPt* P, float h) {
-    const int b0 = H.i.x, b1 = H.i.y, np = H.i.z & 0xff;
+__device__ void contact_presolve(const World& w, int ds, SHdr& H, SPt* P, float h) {
+    const int b0 = H.i.x >= 0 ? ds + H.i.x : -1, b1 = H.i.y >= 0 ? ds + H.i.y : -1, np = H.i.z & 0xff;
     const bool soft = (H.i.z >> 8) != 0;
     const float im0 = H.m.x, im1 = H.m.y;
     M3 I0 = m3zero(), I1 = m3zero();
@@ -588,43 +601,42 @@ __device__ void contact_presolve(const World& w, SHdr& H, SPt* P, float h) {
     }
 }
 
-// ContactConstraints::solve (src/ContactConstraints.cpp:33-124).  No other thread touches
-// the contact's bodies within its colour, so their velocities stay in registers from the
-// first point to the last; every value equals a reload after each point.
-// The step is one dependent chain of up to eight rows, so it is written for latency:
-//   * the header and the velocity view come by value (a store through a record pointer
-//     then cannot alias them, and nothing is reloaded after it);
+// ContactConstraints::solve (src/ContactConstraints.cpp:33-124) of a contact with at most
+// N points; SOFT: the contact may be soft.  No other thread touches the contact's bodies
+// within its colour, so their velocities stay in registers from the first point to the
+// last; every value equals a reload after each point.
+// The step is one dependent chain of up to 2 N rows, so it is written for latency:
 //   * the records are read ahead of the chain (the normal rows' all at once, then the
 //     friction rows') and the accumulated impulses are written after the last row;
-//   * all four rows of each kind are evaluated and a row is kept only when it is live
-//     (the reference skips a row whose inverse effective mass is zero; a contact has
-//     fewer than four points), so the chain has no branches.  A live row's operations
-//     and their order are the reference's.  Branching on the point count instead costs
-//     registers that the solver kernels do not have.
-__device__ __noinline__ void contact_solve(const SHdr H, SPt* __restrict__ P, bool useBias, const VelRef vr) {
+//   * all N rows of each kind are evaluated and a row is kept only when it is live (the
+//     reference skips a row whose inverse effective mass is zero; a contact may have
+//     fewer than N points), so the chain has no branches.  A live row's operations and
+//     their order are the reference's.
+template <int N, bool SOFT, class V>
+__device__ __forceinline__ void contact_solve(const SHdr& H, SPt* __restrict__ P, bool useBias, const V vr) {
     const V3 n = ld3(H.n);
     const float friction = H.n.w;
     const float im0 = H.m.x, im1 = H.m.y;
     const int b0 = H.i.x, b1 = H.i.y, np = H.i.z & 0xff;
-    const bool soft = (H.i.z >> 8) != 0;
+    const bool soft = SOFT && (H.i.z >> 8) != 0;
     V3 v0 = {0, 0, 0}, w0 = {0, 0, 0}, v1 = {0, 0, 0}, w1 = {0, 0, 0};
-    if (b0 >= 0) { v0 = vr.lv(b0); w0 = vr.lw(b0); }
-    if (b1 >= 0) { v1 = vr.lv(b1); w1 = vr.lw(b1); }
+    if (b0 >= 0) vr.ld(b0, v0, w0);
+    if (b1 >= 0) vr.ld(b1, v1, w1);
     // every normal record of the contact is read before the chain; rows past the
     // contact's points read its first point and stay dead
-    float4 A[4], B[4], C[4], D[4];
-    int live[4];
+    float4 A[N], B[N], C[N], D[N];
+    int live[N];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < N; ++i) {
         const bool has = i < np;
         const SPt* q = P + (has ? i : 0);
         A[i] = q->a; B[i] = q->b; C[i] = q->c; D[i] = q->d;
         live[i] = has ? __float_as_int(q->g.w) : 0;
     }
     bool touched = false;
-    float lamN[4], lamT[4];
+    float lamN[N], lamT[N];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < N; ++i) {
         const bool on = (live[i] & 1) != 0;
         const V3 r0xn = ld3(A[i]), r1xn = ld3(B[i]);
         float rv = dot(-n, v0) + dot(-r0xn, w0) + dot(n, v1) + dot(r1xn, w1);
@@ -642,14 +654,14 @@ __device__ __noinline__ void contact_solve(const SHdr H, SPt* __restrict__ P, bo
         if (on && b1 >= 0) { v1 = nv1; w1 = nw1; }
         touched |= on;
     }
-    float4 E[4], F[4], G[4];
+    float4 E[N], F[N], G[N];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < N; ++i) {
         const int q = i < np ? i : 0;
         E[i] = P[q].e; F[i] = P[q].f; G[i] = P[q].g;
     }
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < N; ++i) {
         const bool on = (live[i] & 2) != 0;
         const V3 t = ld3(E[i]);
         float lambda = F[i].w;
@@ -666,20 +678,39 @@ __device__ __noinline__ void contact_solve(const SHdr H, SPt* __restrict__ P, bo
         touched |= on;
     }
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < N; ++i) {
         if (live[i] & 1) P[i].a.w = lamN[i];
         if (live[i] & 2) P[i].e.w = lamT[i];
     }
     if (touched) {
-        if (b0 >= 0) { vr.sv(b0, v0); vr.sw(b0, w0); }
-        if (b1 >= 0) { vr.sv(b1, v1); vr.sw(b1, w1); }
+        if (b0 >= 0) vr.st(b0, v0, w0);
+        if (b1 >= 0) vr.st(b1, v1, w1);
     }
+}
+
+// One contact of a colour step by the form that its warp needs: the contacts of a colour
+// lie by point count (solve_scene), so a warp's contacts mostly have the same number, and
+// most contacts of mixed shapes have one point (1.24 on average on the batched scenes).
+// The vote only chooses among forms that all give this contact's result.
+template <class V>
+__device__ __forceinline__ void contact_step(const SHdr* __restrict__ Hp, SPt* __restrict__ points, bool useBias, const V vr) {
+    const SHdr H = *Hp;
+    const int np = H.i.z & 0xff;
+    const bool soft = (H.i.z >> 8) != 0;
+    if (soft && !useBias) return;   // the relaxation skips soft contacts
+    SPt* P = points + H.i.w;
+    const unsigned lanes = __activemask();
+    if (__any_sync(lanes, soft)) contact_solve<4, true>(H, P, useBias, vr);
+    else if (!__any_sync(lanes, np > 1)) contact_solve<1, false>(H, P, useBias, vr);
+    else if (!__any_sync(lanes, np > 2)) contact_solve<2, false>(H, P, useBias, vr);
+    else contact_solve<4, false>(H, P, useBias, vr);
 }
 
 // ---------------------------------------------------------------- bodies
 
 // integrate velocities (src/Physecs.cpp:441-469)
-__device__ void integrate_velocity(const World& w, int d, float h, float g, const VelRef& vr) {
+template <class V>
+__device__ void integrate_velocity(const World& w, int d, int ds, float h, float g, const V vr) {
     int b = w.dyn_body[d];
     if (w.info[b].y & BODY_KIN) return;
     M3 rot = mat3_cast(ld4(w.quat[b]));
@@ -695,8 +726,7 @@ __device__ void integrate_velocity(const World& w, int d, float h, float g, cons
     ang = mv(rot, wl);
     w.vel[d] = st4(vel);
     w.ang[d] = st4(ang);
-    vr.sv(d, vel);
-    vr.sw(d, ang);
+    vr.st(d - ds, vel, ang);
     w.pv_v[d] = make_float4(0, 0, 0, 0);
     w.pv_w[d] = make_float4(0, 0, 0, 0);
     M3 wi = mm(mm(rot, invIl), invRot);
@@ -706,7 +736,8 @@ __device__ void integrate_velocity(const World& w, int d, float h, float g, cons
 }
 
 // integrate positions (src/Physecs.cpp:492-512)
-__device__ void integrate_position(const World& w, int d, float h, const VelRef& vr) {
+template <class V>
+__device__ void integrate_position(const World& w, int d, int ds, float h, const V vr) {
     int b = w.dyn_body[d];
     if (w.info[b].y & BODY_KIN) return;
     float4 pv = w.pv_v[d];
@@ -714,9 +745,11 @@ __device__ void integrate_position(const World& w, int d, float h, const VelRef&
     V3 pos = ld3(w.pos[b]);
     Q4 q = ld4(w.quat[b]);
     V3 com = ld3(w.com[d]);
-    pos += h * vr.lv(d) + s * ld3(pv);
+    V3 lin, rot;
+    vr.ld(d - ds, lin, rot);
+    pos += h * lin + s * ld3(pv);
     V3 prevCom = qrot(q, com);
-    V3 wv = 0.5f * (h * vr.lw(d) + s * ld3(w.pv_w[d]));
+    V3 wv = 0.5f * (h * rot + s * ld3(w.pv_w[d]));
     q = qadd(q, qmul(Q4{wv.x, wv.y, wv.z, 0.f}, q));
     q = qnormalize(q);
     pos += prevCom - qrot(q, com);
@@ -727,7 +760,7 @@ __device__ void integrate_position(const World& w, int d, float h, const VelRef&
 // ---------------------------------------------------------------- frame kernel
 
 struct BlockSync {
-    static constexpr bool kCluster = false;
+    static constexpr bool kCluster = false, kBlock = true;
     __device__ __forceinline__ void sync() const { __syncthreads(); }
     __device__ __forceinline__ int tid() const { return threadIdx.x; }
     __device__ __forceinline__ int nth() const { return blockDim.x; }
@@ -747,31 +780,9 @@ struct BlockSync {
         __syncthreads();
         return r;
     }
-    // first point of each contact (colour order) packed without gaps; returns the point count
-    __device__ int point_offsets(FrameBuf& f, int ms, int nc) const {
-        __shared__ int part[513];   // solver blocks have at most 512 threads
-        const int t = threadIdx.x, T = blockDim.x;
-        const int chunk = (nc + T - 1) / T;
-        const int k0 = min(nc, t * chunk), k1 = min(nc, k0 + chunk);
-        int sum = 0;
-        for (int k = k0; k < k1; ++k) sum += f.contacts[f.corder[ms + k]].np;
-        part[t] = sum;
-        __syncthreads();
-        if (t == 0) {
-            int acc = 0;
-            for (int i = 0; i < T; ++i) { int v = part[i]; part[i] = acc; acc += v; }
-            part[T] = acc;
-        }
-        __syncthreads();
-        int acc = part[t];
-        for (int k = k0; k < k1; ++k) { f.pt_off[ms + k] = acc; acc += f.contacts[f.corder[ms + k]].np; }
-        const int total = part[T];
-        __syncthreads();
-        return total;
-    }
 };
 struct GridSync {
-    static constexpr bool kCluster = false;
+    static constexpr bool kCluster = false, kBlock = false;
     GridBarrier bar;
     int* flag;
     __device__ __forceinline__ void sync() const { bar.sync(); }
@@ -798,19 +809,13 @@ struct GridSync {
         bar.sync();
         return r;
     }
-    // four point slots per contact (no cross-block scan in grid mode)
-    __device__ int point_offsets(FrameBuf& f, int ms, int nc) const {
-        for (int k = tid(); k < nc; k += nth()) f.pt_off[ms + k] = 4 * k;
-        bar.sync();
-        return 4 * nc;
-    }
 };
 
 // A thread-block cluster working on one scene: the hardware cluster barrier orders
 // shared, distributed-shared and global memory for all its threads; reductions go
 // through a small array in block 0's shared memory.
 struct ClusterSync {
-    static constexpr bool kCluster = true;
+    static constexpr bool kCluster = true, kBlock = false;
     int rank, R, lg;
     float* const* bases;   // every block's dynamic shared memory, mapped
     int* red;              // R ints in block 0's shared memory, mapped
@@ -841,12 +846,6 @@ struct ClusterSync {
         for (int i = 0; i < R; ++i) r = max(r, red[i]);
         sync();
         return r;
-    }
-    // four point slots per contact, as in grid mode
-    __device__ int point_offsets(FrameBuf& f, int ms, int nc) const {
-        for (int k = tid(); k < nc; k += nth()) f.pt_off[ms + k] = 4 * k;
-        sync();
-        return 4 * nc;
     }
 };
 
@@ -934,17 +933,121 @@ __device__ int colour_contacts(const World& w, FrameBuf& f, int ms, int nc, int 
     return ncol;
 }
 
+// A scene's contacts in solve order: its first manifold, contacts, point slots, colours,
+// whether the last colour is serial, and each colour's first contact.
+struct SortedContacts {
+    int ms, ncl, npts, ncol;
+    bool serial_last;
+    const int* colstart;
+};
+
+// All substeps of one scene.  SREC: contact records in shared memory (smem) from rec_f4 to
+// smem_f4 as far as they fit, header and points of a contact together, in solve order; the
+// contacts from ks on keep theirs in the world's buffers, so a scene slightly too big for
+// shared memory loses only its tail.
+template <bool SREC, class S, class V>
+__device__ void solve_substeps(const World& w, FrameBuf& f, int s, const S& sy, const SortedContacts sc, int rec_f4,
+                               int smem_f4, const V vr) {
+    const int tid = sy.tid(), nth = sy.nth();
+    const int ds = w.scene_dyn[s], de = w.scene_dyn[s + 1];
+    const int ms = sc.ms, ncl = sc.ncl, ncol = sc.ncol;
+    const float4 kn = w.knobs[s];
+    const int substeps = (int)kn.x, iterations = (int)kn.y;
+    const float g = kn.z, h = kn.w / substeps;
+    int ks = 0;
+    if constexpr (SREC) {
+        const int room = smem_f4 - rec_f4;
+        if (kHdrF4 * ncl + kPtF4 * sc.npts <= room) {
+            ks = ncl;
+        } else {
+            int fit = 0;
+            for (int k = tid; k < ncl; k += nth) {
+                const int end = k + 1 < ncl ? f.pt_off[ms + k + 1] : sc.npts;
+                if (kHdrF4 * (k + 1) + kPtF4 * end <= room) fit = k + 1;
+            }
+            ks = sy.max_int(fit);
+        }
+    }
+    SHdr* const Hg = f.s_hdr + ms;
+    SPt* const Pg = f.s_pts + 4 * (size_t)ms;
+    auto HK = [&](int k) -> SHdr& { return SREC && k < ks ? ((SHdr*)(smem + rec_f4))[k] : Hg[k]; };
+    auto PK = [&](int k) -> SPt* { return SREC && k < ks ? (SPt*)(smem + rec_f4 + kHdrF4 * ks) : Pg; };
+    for (int k = tid; k < ncl; k += nth) HK(k).i.w = f.pt_off[ms + k];
+    sy.sync();
+    const int js0 = w.scene_jsteps[s], js1 = w.scene_jsteps[s + 1];
+    const int jb = w.scene_joint[s], je = w.scene_joint[s + 1];
+    for (int sub = 0; sub < substeps; ++sub) {
+        for (int k = tid; k < ncl; k += nth) {
+            SHdr& H = HK(k);
+            contact_update(w, f.contacts[f.corder[ms + k]], ds, H, PK(k) + H.i.w);
+        }
+        for (int j = jb + tid; j < je; j += nth) make_joint_rows(w, j);
+        sy.sync();
+        for (int d = ds + tid; d < de; d += nth) integrate_velocity(w, d, ds, h, g, vr);
+        sy.sync();
+        for (int k = tid; k < ncl; k += nth) {
+            SHdr& H = HK(k);
+            contact_presolve(w, ds, H, PK(k) + H.i.w, h);
+        }
+        for (int st = js0; st < js1; ++st) {
+            for (int k = w.jstep_start[st] + tid; k < w.jstep_start[st + 1]; k += nth) joint_presolve(w, w.jsched[k]);
+            sy.sync();
+        }
+        sy.sync();
+        // the iterations, then the positions and the relaxation (the sweep without bias)
+        for (int it = 0; it <= iterations; ++it) {
+            const bool bias = it < iterations;
+            if (!bias) {
+                for (int d = ds + tid; d < de; d += nth) integrate_position(w, d, ds, h, vr);
+                sy.sync();
+            }
+            for (int cl = 0; cl < ncol; ++cl) {
+                const bool serial = sc.serial_last && cl == ncol - 1;
+                const int k1 = sc.colstart[cl + 1], stride = serial ? 1 : nth;
+                int k = sc.colstart[cl] + tid;
+                if (serial && tid != 0) k = k1;
+                if constexpr (SREC) {
+                    const int k2 = min(k1, ks);
+                    for (; k < k2; k += stride)
+                        contact_step((const SHdr*)(smem + rec_f4) + k, (SPt*)(smem + rec_f4 + kHdrF4 * ks), bias, vr);
+                }
+                for (; k < k1; k += stride) contact_step(Hg + k, Pg, bias, vr);
+                sy.sync();
+            }
+            if (bias)
+                for (int st = js0; st < js1; ++st) {
+                    for (int k = w.jstep_start[st] + tid; k < w.jstep_start[st + 1]; k += nth)
+                        joint_solve(w, w.jsched[k], h, it == 0, ds, vr);
+                    sy.sync();
+                }
+        }
+        for (int d = ds + tid; d < de; d += nth) {
+            int b = w.dyn_body[d];
+            if (w.info[b].y & BODY_KIN) continue;
+            V3 lin, rot;
+            vr.ld(d - ds, lin, rot);
+            w.vel[d] = st4(lin);
+            w.ang[d] = st4(rot);
+        }
+        sy.sync();
+    }
+    // accumulated impulses back into the frame's contacts (inspection only)
+    for (int k = tid; k < ncl; k += nth) {
+        Contact& c = f.contacts[f.corder[ms + k]];
+        const SPt* q = PK(k) + HK(k).i.w;
+        for (int i = 0; i < c.np; ++i) { c.p[i].r0xn.w = q[i].a.w; c.p[i].r1xn.w = q[i].e.w; }
+    }
+}
+
 template <class S>
-__device__ void solve_scene(const World& w, FrameBuf& f, int s, const S& sy, float4* smem, int smem_f4) {
+__device__ void solve_scene(const World& w, FrameBuf& f, int s, const S& sy, int smem_f4) {
     if (w.scene_active && !w.scene_active[s]) return;
     const int tid = sy.tid(), nth = sy.nth();
     int ds = w.scene_dyn[s], de = w.scene_dyn[s + 1];
     int ms = f.scene_man[s], me = f.scene_man[s + 1];
-    float4 kn = w.knobs[s];
-    int substeps = (int)kn.x, iterations = (int)kn.y;
-    float g = kn.z, dt = kn.w;
-    int* colstart_g = f.color_start + s * (kMaxColors + 1);
-    __shared__ int colstart[kMaxColors + 1];   // this block's copy, read by every colour step
+    // bins of the counting sort: bin_a counts, then cursors; bin_b as written by the scan
+    __shared__ int bin_a[kColorBins], bin_b[kColorBins], bin_total[2];
+    __shared__ int colstart[kMaxColors + 1];   // first contact of each colour, read by every colour step
     // ---- graph colouring of the contacts.  Each colour is a maximal set of contacts with
     // no dynamic body in common, grown in rounds: every uncoloured contact whose bodies
     // the colour does not hold yet claims them with a hashed priority, and the contacts
@@ -961,133 +1064,89 @@ __device__ void solve_scene(const World& w, FrameBuf& f, int s, const S& sy, flo
     int ncol = colour_contacts(w, f, ms, nc, ds, nd, sy, claim, cmask, cb, col);
     const bool serial_last = ncol < 0;
     if (serial_last) ncol = -ncol;
-    // counting sort of the scene's contacts by colour
-    for (int k = tid; k <= kMaxColors; k += nth) colstart_g[k] = 0;
+    // Counting sort of the scene's contacts by colour and, within a colour, by point count
+    // (four points first), one bin each: contacts of one colour touch disjoint bodies and
+    // may be solved in any order, and a warp of contacts with the same point count runs no
+    // row it does not need.  A contact's first point follows from its bin, so the records
+    // are packed without a scan over the contacts.  A block keeps the bins in shared
+    // memory, a grid or cluster counts in global memory and scans once per block.
+    const int nbins = kPointBins * ncol;
+    int* const hist = S::kBlock ? bin_a : f.color_start + (size_t)s * kColorBins;
+    int* const cursor = S::kBlock ? bin_a : f.claim_pos + (size_t)s * kColorBins;
+    auto bin_of = [&](int cl, int k) {
+        if (serial_last && cl == ncol - 1) return kPointBins * cl;
+        return kPointBins * cl + 4 - min(4, max(1, f.contacts[ms + k].np));
+    };
+    for (int b = tid; b < nbins; b += nth) { hist[b] = 0; if (!S::kBlock) cursor[b] = 0; }
     sy.sync();
-    for (int k = tid; k < nc; k += nth) { int cl = col[k]; if (cl >= 0) atomicAdd(&colstart_g[cl + 1], 1); }
+    for (int k = tid; k < nc; k += nth) { const int cl = col[k]; if (cl >= 0) atomicAdd(&hist[bin_of(cl, k)], 1); }
     sy.sync();
-    if (tid == 0) {
-        for (int k = 0; k < kMaxColors; ++k) colstart_g[k + 1] += colstart_g[k];
-        f.scene_ncolor[s] = ncol;
+    if (threadIdx.x < 32) {
+        // bin_a: first contact of the bin; bin_b: its first point less (points per contact)
+        // times that, so that a contact's first point is bin_b + k * points
+        int c0 = 0, p0 = 0;
+        for (int base = 0; base < nbins; base += 32) {
+            const int b = base + (int)threadIdx.x, per = 4 - (b & (kPointBins - 1));
+            const int n = b < nbins ? (S::kBlock ? bin_a[b] : ((volatile int*)hist)[b]) : 0;
+            int cs = n, ps = n * per;
+            for (int o = 1; o < 32; o <<= 1) {
+                const int x = __shfl_up_sync(~0u, cs, o), y = __shfl_up_sync(~0u, ps, o);
+                if ((int)threadIdx.x >= o) { cs += x; ps += y; }
+            }
+            if (b < nbins) {
+                bin_a[b] = c0 + cs - n;
+                bin_b[b] = p0 + ps - n * per - (c0 + cs - n) * per;
+            }
+            c0 += __shfl_sync(~0u, cs, 31);
+            p0 += __shfl_sync(~0u, ps, 31);
+        }
+        if (threadIdx.x == 0) { bin_total[0] = c0; bin_total[1] = p0; }
     }
-    sy.sync();
-    for (int k = threadIdx.x; k <= kMaxColors; k += blockDim.x) colstart[k] = colstart_g[k];
+    if (tid == 0) f.scene_ncolor[s] = ncol;
+    __syncthreads();
+    const int ncl = bin_total[0], npts = bin_total[1];   // coloured contacts (all of them) and their point slots
+    for (int c = threadIdx.x; c <= ncol; c += blockDim.x) colstart[c] = c < ncol ? bin_a[kPointBins * c] : ncl;
     __syncthreads();
     for (int k = tid; k < nc; k += nth) {
-        int cl = col[k];
-        if (col_smem) f.color_of[ms + k] = cl;   // kept for inspection
+        const int cl = col[k];
+        if (S::kBlock) f.color_of[ms + k] = cl;   // kept for inspection
         if (cl < 0 || (serial_last && cl == ncol - 1)) continue;
-        // contacts of one colour touch disjoint bodies and may be solved in any order
-        int pos = atomicAdd(&f.claim_pos[s * (kMaxColors + 1) + cl], 1);
-        f.corder[ms + colstart[cl] + pos] = ms + k;
+        const int b = bin_of(cl, k), per = 4 - (b & (kPointBins - 1));
+        const int pos = atomicAdd(&cursor[b], 1) + (S::kBlock ? 0 : bin_a[b]);
+        f.corder[ms + pos] = ms + k;
+        f.pt_off[ms + pos] = bin_b[b] + pos * per;
     }
     if (serial_last && tid == 0) {
         // the serial colour keeps contact order
-        int pos = 0;
-        for (int k = 0; k < nc; ++k) if (col[k] == ncol - 1) f.corder[ms + colstart[ncol - 1] + pos++] = ms + k;
+        int pos = colstart[ncol - 1];
+        for (int k = 0; k < nc; ++k)
+            if (col[k] == ncol - 1) {
+                f.corder[ms + pos] = ms + k;
+                f.pt_off[ms + pos] = bin_b[kPointBins * (ncol - 1)] + pos * 4;
+                ++pos;
+            }
     }
     sy.sync();
-    // ---- where the substep data lives: velocities and contact records in shared memory
-    // when they fit, velocities alone when only they fit, else the world's buffers
-    const int ncl = colstart[kMaxColors];   // coloured contacts (all, unless the colour cap was hit)
-    int npts = sy.point_offsets(f, ms, ncl);   // first point of each contact -> f.pt_off[ms + k]
+    const SortedContacts sc{ms, ncl, npts, ncol, serial_last, colstart};
     const int vel_f4 = (6 * nd + 3) / 4;
-    const bool vel_smem = !S::kCluster && vel_f4 <= smem_f4;
-    // contact headers in shared memory when they fit beside the velocities; point records
-    // fill what is left, in colour order, up to the first contact whose points no longer
-    // fit (contacts ks.. keep theirs in the world's buffer), so a scene slightly too big
-    // for shared memory loses only its tail, not every record
-    const bool hdr_smem = vel_smem && vel_f4 + kHdrF4 * ncl <= smem_f4;
-    const int pbase_f4 = vel_f4 + (hdr_smem ? kHdrF4 * ncl : 0);
-    const int pcap = vel_smem ? max(0, (smem_f4 - pbase_f4) / kPtF4) : 0;
-    int ks = 0;
-    if (vel_smem) {
-        int fit = 0;
-        for (int k = tid; k < ncl; k += nth) {
-            const int end = k + 1 < ncl ? f.pt_off[ms + k + 1] : npts;
-            if (end <= pcap) fit = k + 1;
-        }
-        ks = sy.max_int(fit);
-    }
-    VelRef vr = vel_smem ? VelRef{(float*)smem, nullptr, nullptr, nullptr, ds, nd, 0}
-                         : VelRef{nullptr, nullptr, w.vt_v, w.vt_w, 0, 0, 0};
-    if constexpr (S::kCluster) {
+    if constexpr (S::kBlock) {
+        if (vel_f4 <= smem_f4) solve_substeps<true>(w, f, s, sy, sc, vel_f4, smem_f4, SmemVel{});
+        else solve_substeps<false>(w, f, s, sy, sc, 0, 0, GlobVel{w.vt_v + ds, w.vt_w + ds});
+    } else if constexpr (S::kCluster) {
         // velocities spread over the cluster's blocks; records and colouring stay global
         const int per = (nd + sy.R - 1) >> sy.lg;
-        if (6 * per <= 4 * smem_f4) vr = VelRef{nullptr, sy.bases, nullptr, nullptr, ds, per, sy.lg};
-        else vr = VelRef{nullptr, nullptr, w.vt_v, w.vt_w, 0, 0, 0};
-    }
-    SHdr* H = hdr_smem ? (SHdr*)(smem + vel_f4) : f.s_hdr + ms;
-    SPt* const Ps = (SPt*)(smem + pbase_f4);
-    SPt* const Pg = f.s_pts + 4 * (size_t)ms;
-    auto PK = [&](int k) -> SPt* { return (k < ks ? Ps : Pg) + H[k].i.w; };
-    for (int k = tid; k < ncl; k += nth) H[k].i.w = f.pt_off[ms + k];
-    sy.sync();
-    int js0 = w.scene_jsteps[s], js1 = w.scene_jsteps[s + 1];
-    int jb = w.scene_joint[s], je = w.scene_joint[s + 1];
-    float h = dt / substeps;
-    for (int sub = 0; sub < substeps; ++sub) {
-        for (int k = tid; k < ncl; k += nth) contact_update(w, f.contacts[f.corder[ms + k]], H[k], PK(k));
-        for (int j = jb + tid; j < je; j += nth) make_joint_rows(w, j);
-        sy.sync();
-        for (int d = ds + tid; d < de; d += nth) integrate_velocity(w, d, h, g, vr);
-        sy.sync();
-        for (int k = tid; k < ncl; k += nth) contact_presolve(w, H[k], PK(k), h);
-        for (int st = js0; st < js1; ++st) {
-            for (int k = w.jstep_start[st] + tid; k < w.jstep_start[st + 1]; k += nth) joint_presolve(w, w.jsched[k]);
-            sy.sync();
-        }
-        sy.sync();
-        for (int it = 0; it < iterations; ++it) {
-            for (int cl = 0; cl < ncol; ++cl) {
-                if (serial_last && cl == ncol - 1) {
-                    if (tid == 0)
-                        for (int k = colstart[cl]; k < colstart[cl + 1]; ++k) contact_solve(H[k], PK(k), true, vr);
-                } else {
-                    for (int k = colstart[cl] + tid; k < colstart[cl + 1]; k += nth) contact_solve(H[k], PK(k), true, vr);
-                }
-                sy.sync();
-            }
-            for (int st = js0; st < js1; ++st) {
-                for (int k = w.jstep_start[st] + tid; k < w.jstep_start[st + 1]; k += nth) joint_solve(w, w.jsched[k], h, it == 0, vr);
-                sy.sync();
-            }
-        }
-        for (int d = ds + tid; d < de; d += nth) integrate_position(w, d, h, vr);
-        sy.sync();
-        for (int cl = 0; cl < ncol; ++cl) {
-            if (serial_last && cl == ncol - 1) {
-                if (tid == 0)
-                    for (int k = colstart[cl]; k < colstart[cl + 1]; ++k)
-                        if (!(H[k].i.z >> 8)) contact_solve(H[k], PK(k), false, vr);
-            } else {
-                for (int k = colstart[cl] + tid; k < colstart[cl + 1]; k += nth)
-                    if (!(H[k].i.z >> 8)) contact_solve(H[k], PK(k), false, vr);
-            }
-            sy.sync();
-        }
-        for (int d = ds + tid; d < de; d += nth) {
-            int b = w.dyn_body[d];
-            if (w.info[b].y & BODY_KIN) continue;
-            w.vel[d] = st4(vr.lv(d));
-            w.ang[d] = st4(vr.lw(d));
-        }
-        sy.sync();
-    }
-    // accumulated impulses back into the frame's contacts (inspection only)
-    for (int k = tid; k < ncl; k += nth) {
-        Contact& c = f.contacts[f.corder[ms + k]];
-        const SPt* q = PK(k);
-        for (int i = 0; i < c.np; ++i) { c.p[i].r0xn.w = q[i].a.w; c.p[i].r1xn.w = q[i].e.w; }
+        if (6 * per <= 4 * smem_f4) solve_substeps<false>(w, f, s, sy, sc, 0, 0, ClusterVel{sy.bases, per, sy.lg});
+        else solve_substeps<false>(w, f, s, sy, sc, 0, 0, GlobVel{w.vt_v + ds, w.vt_w + ds});
+    } else {
+        solve_substeps<false>(w, f, s, sy, sc, 0, 0, GlobVel{w.vt_v + ds, w.vt_w + ds});
     }
 }
 
 // one scene per block; NT = 32 or 64, 128 or 256 for scenes up to 1024 dynamic bodies (by size), 512 above
 template <int NT>
 __global__ void __launch_bounds__(NT, 512 / NT) k_solve_block(World w, FrameBuf f, const int* scenes, int smem_f4) {
-    extern __shared__ float4 smem[];
     BlockSync sy;
-    solve_scene(w, f, scenes[blockIdx.x], sy, smem, smem_f4);
+    solve_scene(w, f, scenes[blockIdx.x], sy, smem_f4);
 }
 
 static_assert(kBarrierTimeoutBit == ERR_BARRIER_TIMEOUT, "grid barrier error bit");
@@ -1095,7 +1154,7 @@ static_assert(kBarrierTimeoutBit == ERR_BARRIER_TIMEOUT, "grid barrier error bit
 __global__ void __launch_bounds__(256, 2) k_solve_grid(World w, FrameBuf f, const int* scenes, int n, long long limit) {
     GridSync sy{GridBarrier{f.bar, f.bar + 1, w.err, limit}, (int*)(f.bar + 2)};
     for (int i = 0; i < n; ++i) {
-        solve_scene(w, f, scenes[i], sy, nullptr, 0);
+        solve_scene(w, f, scenes[i], sy, 0);
         sy.sync();
     }
 }
@@ -1103,7 +1162,6 @@ __global__ void __launch_bounds__(256, 2) k_solve_grid(World w, FrameBuf f, cons
 // one cluster of kClusterBlocks blocks per large scene, velocities in distributed shared memory
 template <int NT>
 __global__ void __launch_bounds__(NT, 1) k_solve_cluster(World w, FrameBuf f, const int* scenes, int smem_f4) {
-    extern __shared__ float4 smem[];
     __shared__ float* bases[kClusterBlocks];
     __shared__ int red[kClusterBlocks];
     cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
@@ -1114,7 +1172,7 @@ __global__ void __launch_bounds__(NT, 1) k_solve_cluster(World w, FrameBuf f, co
     while ((1 << lg) < R) ++lg;
     cl.sync();
     ClusterSync sy{rank, R, lg, bases, red0};
-    solve_scene(w, f, scenes[blockIdx.x / R], sy, smem, smem_f4);
+    solve_scene(w, f, scenes[blockIdx.x / R], sy, smem_f4);
     cl.sync();   // no block leaves while the others may still read its shared memory
 }
 
@@ -1184,8 +1242,7 @@ static void launch_block_ranked(int grid, int smem, cudaStream_t st, int rank, c
 }
 
 int launch_solver(const World& w, FrameBuf& f, const SolverLaunch& L, cudaStream_t s) {
-    k_zero_ints<<<(w.n_scenes * (kMaxColors + 1) + 255) / 256, 256, 0, s>>>(f.claim_pos, w.n_scenes * (kMaxColors + 1));
-    int k = 2;
+    int k = 1;
     // large scenes on a second stream, concurrently with the small ones, and first: their
     // chains are the longest (measured with eager launches: solver stage 7.20 -> 6.65 ms
     // on the 4096-scene frame)

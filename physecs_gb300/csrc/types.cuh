@@ -32,6 +32,8 @@ constexpr int kTriManifolds = 16;  // manifolds one body may produce against one
 constexpr int kTriCandidates = 64; // candidate triangles per body-mesh pair
 constexpr int kMaxRowsPerJoint = 8;
 constexpr int kMaxColors = 128;    // contact colours per scene
+constexpr int kPointBins = 4;      // bins of a colour in the solve order: contacts of 4, 3, 2 and 1 points
+constexpr int kColorBins = kPointBins * kMaxColors;
 constexpr int kMeshBoundsChunk = 8192;   // triangle-mesh vertices per block in the collider bounds
 
 struct ConvexMeshDev {   // one ConvexMesh

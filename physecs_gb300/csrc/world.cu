@@ -418,8 +418,8 @@ psx_status psx::rt::build_world(psx_world* W, const psx_scene_desc* scenes, int 
     PSX_TRY(W->alloc(f.color_of, f.man_cap));
     PSX_TRY(W->alloc(f.corder, f.man_cap));
     PSX_TRY(W->alloc(f.scene_ncolor, S));
-    PSX_TRY(W->alloc(f.color_start, (size_t)S * (kMaxColors + 1)));
-    PSX_TRY(W->alloc(f.claim_pos, (size_t)S * (kMaxColors + 1)));
+    PSX_TRY(W->alloc(f.color_start, (size_t)S * kColorBins));
+    PSX_TRY(W->alloc(f.claim_pos, (size_t)S * kColorBins));
     PSX_TRY(W->alloc(f.pt_off, f.man_cap));
     PSX_TRY(W->alloc(f.cbody, f.man_cap));
     PSX_TRY(W->alloc(f.cmask, std::max(1, w.n_dyn)));
@@ -1322,7 +1322,7 @@ PSX_API int32_t psx_world_get_contacts(psx_world* W, int32_t* ids, float* f, int
     if (!W) return -1;
     cudaStreamSynchronize(W->stream);
     int S = W->n_scenes;
-    std::vector<int> scene_man(S + 1), cstart((size_t)S * (kMaxColors + 1)), ncol(S);
+    std::vector<int> scene_man(S + 1);
     cudaMemcpy(scene_man.data(), W->f.scene_man, (S + 1) * sizeof(int), cudaMemcpyDeviceToHost);
     int nm = scene_man[S];
     std::vector<Contact> cs(nm);
