@@ -85,7 +85,8 @@ struct FrameBuf {
     int* color_start;     // [S * kColorBins] contacts per bin of a scene solved by several blocks
     int* claim_pos;       // [S * kColorBins] scatter counters of the same scenes
     // per-substep contact records of scenes whose records do not fit in shared memory
-    int* pt_off;          // [man_cap] first point of each contact, colour order
+    int* pt_off;          // [man_cap] point slots of each contact, solve order: first slot, step - 1 from bit 28
+    int* pt_end;          // [man_cap] end of the slots of each contact's group
     int2* cbody;          // [man_cap] colouring: scene-local dynamic bodies of each contact
     uint4* cmask;         // [n_dyn] colouring: colours each dynamic body carries (128 bits)
     SHdr* s_hdr;          // [man_cap]

@@ -521,67 +521,63 @@ __device__ __forceinline__ M3 world_invI(const World& w, int d) {
 }
 
 
-// update contact rows (src/Physecs.cpp:366-427)
-__device__ void contact_update(const World& w, Contact& c, int ds, SHdr& H, SPt* P) {
-    int4 i0 = w.info[c.body0], i1 = w.info[c.body1];
-    Q4 q0 = ld4(w.quat[c.body0]), q1 = ld4(w.quat[c.body1]);
-    V3 com0 = {0, 0, 0}, v0 = {0, 0, 0}, w0 = {0, 0, 0}, com1 = {0, 0, 0}, v1 = {0, 0, 0}, w1 = {0, 0, 0};
-    if (c.b0 >= 0) { com0 = ld3(w.pos[c.body0]) + qrot(q0, ld3(w.com[i0.z])); v0 = ld3(w.vel[i0.z]); w0 = ld3(w.ang[i0.z]); }
-    if (c.b1 >= 0) { com1 = ld3(w.pos[c.body1]) + qrot(q1, ld3(w.com[i1.z])); v1 = ld3(w.vel[i1.z]); w1 = ld3(w.ang[i1.z]); }
-    V3 n = ld3(c.n);
+// The constants of a contact's solver header.
+__device__ void contact_header(const World& w, const Contact& c, int ds, int slots, SHdr& H) {
     H.n = c.n;
     H.m = make_float4(c.b0 >= 0 ? w.com[c.b0].w : 0.f, c.b1 >= 0 ? w.com[c.b1].w : 0.f, c.frequency, c.damping);
-    H.i.x = c.b0 >= 0 ? c.b0 - ds : -1;
-    H.i.y = c.b1 >= 0 ? c.b1 - ds : -1;
-    H.i.z = c.np | (c.soft << 8);
-    for (int k = 0; k < c.np; ++k) {
-        ContactPt& p = c.p[k];
-        V3 r0 = qrot(q0, ld3(p.r0)), r1 = qrot(q1, ld3(p.r1));
-        V3 cp0 = com0 + r0, cp1 = com1 + r1;
-        float cn = dot(cp1 - cp0, n);
-        V3 rel = v1 + cross(w1, r1) - v0 - cross(w0, r0);
-        float relN = dot(rel, n);
-        V3 t = rel - relN * n;
-        float tl = length(t);
-        if (tl) t = t / tl;
-        p.r1.w = cn;
-        SPt& q = P[k];
-        q.a = st4(cross(r0, n), 0.f);
-        q.b = st4(cross(r1, n), p.r0.w);
-        q.c.w = cn;
-        q.e = st4(t, 0.f);
-        q.f = st4(cross(r0, t), 0.f);
-        q.g = st4(cross(r1, t), 0.f);
-    }
+    H.i = make_int4(c.b0 >= 0 ? c.b0 - ds : -1, c.b1 >= 0 ? c.b1 - ds : -1, c.np | (c.soft << 8) | (((slots >> 28) + 1) << 9), slots & 0xfffffff);
 }
 
-// ContactConstraints::preSolve (src/ContactConstraints.cpp:4-31) and the per-substep
-// constants of solve (:33-101)
-__device__ void contact_presolve(const World& w, int ds, SHdr& H, SPt* P, float h) {
-    const int b0 = H.i.x >= 0 ? ds + H.i.x : -1, b1 = H.i.y >= 0 ? ds + H.i.y : -1, np = H.i.z & 0xff;
-    const bool soft = (H.i.z >> 8) != 0;
+// A contact's rows for one substep: the row update (src/Physecs.cpp:366-427), which reads
+// the velocities the substep started with (w.vel, w.ang), then ContactConstraints::preSolve
+// (src/ContactConstraints.cpp:4-31) and the per-substep constants of solve (:33-101), which
+// read the integrated ones (vr).  `last`: the substep's separations stay with the contact.
+template <class V>
+__device__ void contact_rows(const World& w, Contact& c, const SHdr& H, SPt* __restrict__ P, float h, bool last, const V vr) {
+    const int4 id = *reinterpret_cast<const int4*>(&c.b0);   // b0, b1, body0, body1
+    const int b0 = id.x, b1 = id.y, np = H.i.z & 0xff, step = H.i.z >> 9;
+    const bool soft = (H.i.z & 0x100) != 0;
     const float im0 = H.m.x, im1 = H.m.y;
+    V3 com0 = {0, 0, 0}, v0 = {0, 0, 0}, w0 = {0, 0, 0}, com1 = {0, 0, 0}, v1 = {0, 0, 0}, w1 = {0, 0, 0};
+    V3 nv0 = {0, 0, 0}, nw0 = {0, 0, 0}, nv1 = {0, 0, 0}, nw1 = {0, 0, 0};
     M3 I0 = m3zero(), I1 = m3zero();
-    V3 v0 = {0, 0, 0}, w0 = {0, 0, 0}, v1 = {0, 0, 0}, w1 = {0, 0, 0};
-    if (b0 >= 0) { I0 = world_invI(w, b0); v0 = ld3(w.vel[b0]); w0 = ld3(w.ang[b0]); }
-    if (b1 >= 0) { I1 = world_invI(w, b1); v1 = ld3(w.vel[b1]); w1 = ld3(w.ang[b1]); }
-    V3 n = ld3(H.n);
+    Q4 q0, q1;
+    if (b0 >= 0) {
+        com0 = ld3(w.bq[2 * b0]); q0 = ld4(w.bq[2 * b0 + 1]);
+        v0 = ld3(w.vel[b0]); w0 = ld3(w.ang[b0]);
+        I0 = world_invI(w, b0);
+        vr.ld(H.i.x, nv0, nw0);
+    } else q0 = ld4(w.quat[id.z]);
+    if (b1 >= 0) {
+        com1 = ld3(w.bq[2 * b1]); q1 = ld4(w.bq[2 * b1 + 1]);
+        v1 = ld3(w.vel[b1]); w1 = ld3(w.ang[b1]);
+        I1 = world_invI(w, b1);
+        vr.ld(H.i.y, nv1, nw1);
+    } else q1 = ld4(w.quat[id.w]);
+    const V3 n = ld3(H.n);
     for (int k = 0; k < np; ++k) {
-        SPt& p = P[k];
-        V3 r0xn = ld3(p.a), r1xn = ld3(p.b), r0xt = ld3(p.f), r1xt = ld3(p.g), t = ld3(p.e);
-        V3 r0xnt = mv(I0, r0xn), r1xnt = mv(I1, r1xn), r0xtt = mv(I0, r0xt), r1xtt = mv(I1, r1xt);
-        float invN = dot(n, n) * (im0 + im1) + dot(r0xn, r0xnt) + dot(r1xn, r1xnt);
-        float invT = dot(t, t) * (im0 + im1) + dot(r0xt, r0xtt) + dot(r1xt, r1xtt);
-        float cc = p.c.w;
+        const float4 l0 = c.p[k].r0;
+        const V3 r0 = qrot(q0, ld3(l0)), r1 = qrot(q1, ld3(c.p[k].r1));
+        const V3 cp0 = com0 + r0, cp1 = com1 + r1;
+        const float cc = dot(cp1 - cp0, n);
+        const V3 rel = v1 + cross(w1, r1) - v0 - cross(w0, r0);
+        const float relN = dot(rel, n);
+        V3 t = rel - relN * n;
+        const float tl = length(t);
+        if (tl) t = t / tl;
+        const V3 r0xn = cross(r0, n), r1xn = cross(r1, n), r0xt = cross(r0, t), r1xt = cross(r1, t);
+        const V3 r0xnt = mv(I0, r0xn), r1xnt = mv(I1, r1xn), r0xtt = mv(I0, r0xt), r1xtt = mv(I1, r1xt);
+        const float invN = dot(n, n) * (im0 + im1) + dot(r0xn, r0xnt) + dot(r1xn, r1xnt);
+        const float invT = dot(t, t) * (im0 + im1) + dot(r0xt, r0xtt) + dot(r1xt, r1xtt);
         float t1 = 0.f, t2 = 0.f, lamT = 0.f;
         if (invN) {
-            float eff = 1.f / invN;
+            const float eff = 1.f / invN;
             if (soft) {
-                float af = 2.f * kPi * H.m.z;
-                float stiffness = af * af * eff;
-                float damping = 2.f * af * H.m.w * eff;
-                float gamma = 1.f / (damping + h * stiffness);
-                float beta = h * stiffness / (damping + h * stiffness);
+                const float af = 2.f * kPi * H.m.z;
+                const float stiffness = af * af * eff;
+                const float damping = 2.f * af * H.m.w * eff;
+                const float gamma = 1.f / (damping + h * stiffness);
+                const float beta = h * stiffness / (damping + h * stiffness);
                 t1 = beta * cc / h;
                 t2 = invN + gamma / h;
             } else {
@@ -590,38 +586,73 @@ __device__ void contact_presolve(const World& w, int ds, SHdr& H, SPt* P, float 
             }
         }
         if (invT) {
-            float rv = dot(-t, v0) + dot(-r0xt, w0) + dot(t, v1) + dot(r1xt, w1);
+            const float rv = dot(-t, nv0) + dot(-r0xt, nw0) + dot(t, nv1) + dot(r1xt, nw1);
             lamT = rv / invT;
         }
-        int live = (invN ? 1 : 0) | (invT ? 2 : 0);
-        p.c = st4(r0xnt, t1);
-        p.d = st4(r1xnt, t2);
-        p.f = st4(r0xtt, lamT);
-        p.g = st4(r1xtt, __int_as_float(live));
+        const int live = (invN ? 1 : 0) | (invT ? 2 : 0);
+        SPt& p = P[k * step];
+        p.a = make_float4(-r0xn.x, r1xn.x, -r0xn.y, r1xn.y);
+        p.b = make_float4(-r0xn.z, r1xn.z, r0xnt.x, -r1xnt.x);
+        p.c = make_float4(r0xnt.y, -r1xnt.y, r0xnt.z, -r1xnt.z);
+        p.d = make_float4(0.f, l0.w, t1, t2);
+        p.e = st4(t, 0.f);
+        p.f = make_float4(r0xtt.x, -r1xtt.x, r0xtt.y, -r1xtt.y);
+        p.g = make_float4(r0xtt.z, -r1xtt.z, lamT, __int_as_float(live));
+        if (last) c.p[k].r1.w = cc;
     }
 }
+
+// Two floats in one 64-bit register; the packed operations round each lane as the scalar
+// ones do, at half the instructions.  A packed product is formed as a * b + (-0), which is
+// a * b exactly, with the -0 read from memory: the assembler contracts a packed multiply
+// and the add that follows it into one fused operation, whatever its options.
+struct F2 { unsigned long long u; };
+__constant__ unsigned long long c_minus_zero2 = 0x8000000080000000ull;
+__device__ __forceinline__ F2 f2(float lo, float hi) {
+    F2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.u) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void f2split(F2 a, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(a.u)); }
+__device__ __forceinline__ F2 operator*(F2 a, F2 b) { F2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.u) : "l"(a.u), "l"(b.u), "l"(c_minus_zero2)); return r; }
+__device__ __forceinline__ F2 operator+(F2 a, F2 b) { F2 r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.u) : "l"(a.u), "l"(b.u)); return r; }
+struct F2x3 { F2 x, y, z; };
+__device__ __forceinline__ F2 dot(const F2x3& a, const F2x3& b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
+// (a0, a1) += s * (b0, b1), each component
+__device__ __forceinline__ void axpy(F2x3& a, F2 s, const F2x3& b) { a = {a.x + s * b.x, a.y + s * b.y, a.z + s * b.z}; }
 
 // ContactConstraints::solve (src/ContactConstraints.cpp:33-124) of a contact with at most
 // N points; SOFT: the contact may be soft.  No other thread touches the contact's bodies
 // within its colour, so their velocities stay in registers from the first point to the
 // last; every value equals a reload after each point.
-// The step is one dependent chain of up to 2 N rows, so it is written for latency:
+// The step is one dependent chain of up to 2 N rows, so it is written for latency and
+// few instructions:
+//   * both bodies' sides of a row run as one packed operation (body 0, body 1), on
+//     records that hold the two sides in pairs with the constraint's signs;
 //   * the records are read ahead of the chain (the normal rows' all at once, then the
 //     friction rows') and the accumulated impulses are written after the last row;
-//   * all N rows of each kind are evaluated and a row is kept only when it is live (the
-//     reference skips a row whose inverse effective mass is zero; a contact may have
-//     fewer than N points), so the chain has no branches.  A live row's operations and
-//     their order are the reference's.
+//   * all N rows of each kind are evaluated, with an impulse of zero where a row is not
+//     live (the reference skips a row whose inverse effective mass is zero; a contact may
+//     have fewer than N points) or a side has no simulated body, so the chain has no
+//     branches.  A live row's operations and their order are the reference's (x - l * n
+//     is formed as x + l * (-n), which rounds the same).
 template <int N, bool SOFT, class V>
 __device__ __forceinline__ void contact_solve(const SHdr& H, SPt* __restrict__ P, bool useBias, const V vr) {
-    const V3 n = ld3(H.n);
     const float friction = H.n.w;
-    const float im0 = H.m.x, im1 = H.m.y;
-    const int b0 = H.i.x, b1 = H.i.y, np = H.i.z & 0xff;
-    const bool soft = SOFT && (H.i.z >> 8) != 0;
-    V3 v0 = {0, 0, 0}, w0 = {0, 0, 0}, v1 = {0, 0, 0}, w1 = {0, 0, 0};
-    if (b0 >= 0) vr.ld(b0, v0, w0);
-    if (b1 >= 0) vr.ld(b1, v1, w1);
+    const int b0 = H.i.x, b1 = H.i.y, np = H.i.z & 0xff, step = H.i.z >> 9;
+    const bool soft = SOFT && (H.i.z & 0x100) != 0;
+    const bool sim0 = b0 >= 0, sim1 = b1 >= 0;
+    const F2 im = f2(H.m.x, H.m.y);
+    const F2x3 nm = {f2(-H.n.x, H.n.x), f2(-H.n.y, H.n.y), f2(-H.n.z, H.n.z)};
+    const F2x3 np3 = {f2(H.n.x, -H.n.x), f2(H.n.y, -H.n.y), f2(H.n.z, -H.n.z)};
+    F2x3 v, o;   // linear and angular velocities (body 0, body 1)
+    {
+        V3 v0 = {0, 0, 0}, w0 = {0, 0, 0}, v1 = {0, 0, 0}, w1 = {0, 0, 0};
+        if (sim0) vr.ld(b0, v0, w0);
+        if (sim1) vr.ld(b1, v1, w1);
+        v = {f2(v0.x, v1.x), f2(v0.y, v1.y), f2(v0.z, v1.z)};
+        o = {f2(w0.x, w1.x), f2(w0.y, w1.y), f2(w0.z, w1.z)};
+    }
     // every normal record of the contact is read before the chain; rows past the
     // contact's points read its first point and stay dead
     float4 A[N], B[N], C[N], D[N];
@@ -629,7 +660,7 @@ __device__ __forceinline__ void contact_solve(const SHdr& H, SPt* __restrict__ P
 #pragma unroll
     for (int i = 0; i < N; ++i) {
         const bool has = i < np;
-        const SPt* q = P + (has ? i : 0);
+        const SPt* q = P + (has ? i * step : 0);
         A[i] = q->a; B[i] = q->b; C[i] = q->c; D[i] = q->d;
         live[i] = has ? __float_as_int(q->g.w) : 0;
     }
@@ -638,53 +669,55 @@ __device__ __forceinline__ void contact_solve(const SHdr& H, SPt* __restrict__ P
 #pragma unroll
     for (int i = 0; i < N; ++i) {
         const bool on = (live[i] & 1) != 0;
-        const V3 r0xn = ld3(A[i]), r1xn = ld3(B[i]);
-        float rv = dot(-n, v0) + dot(-r0xn, w0) + dot(n, v1) + dot(r1xn, w1);
+        float lin0, lin1, ang0, ang1;
+        f2split(dot(nm, v), lin0, lin1);
+        f2split(dot(F2x3{f2(A[i].x, A[i].y), f2(A[i].z, A[i].w), f2(B[i].x, B[i].y)}, o), ang0, ang1);
+        const float rv = lin0 + ang0 + lin1 + ang1;
         float lambda;
-        if (soft) lambda = (rv + C[i].w) / D[i].w;
-        else lambda = (rv - B[i].w + (useBias ? C[i].w : 0.f)) * D[i].w;
-        const float prev = A[i].w;
+        if (soft) lambda = (rv + D[i].z) / D[i].w;
+        else lambda = (rv - D[i].y + (useBias ? D[i].z : 0.f)) * D[i].w;
+        const float prev = D[i].x;
         float tot = prev + lambda;
         tot = fminG(tot, 0.f);
         lamN[i] = on ? tot : prev;
         lambda = tot - prev;
-        const V3 nv0 = v0 + lambda * im0 * n, nw0 = w0 + lambda * ld3(C[i]);
-        const V3 nv1 = v1 - lambda * im1 * n, nw1 = w1 - lambda * ld3(D[i]);
-        if (on && b0 >= 0) { v0 = nv0; w0 = nw0; }
-        if (on && b1 >= 0) { v1 = nv1; w1 = nw1; }
+        const F2 l = f2(on && sim0 ? lambda : 0.f, on && sim1 ? lambda : 0.f);
+        axpy(v, l * im, np3);
+        axpy(o, l, F2x3{f2(B[i].z, B[i].w), f2(C[i].x, C[i].y), f2(C[i].z, C[i].w)});
         touched |= on;
     }
     float4 E[N], F[N], G[N];
 #pragma unroll
     for (int i = 0; i < N; ++i) {
-        const int q = i < np ? i : 0;
+        const int q = i < np ? i * step : 0;
         E[i] = P[q].e; F[i] = P[q].f; G[i] = P[q].g;
     }
 #pragma unroll
     for (int i = 0; i < N; ++i) {
         const bool on = (live[i] & 2) != 0;
-        const V3 t = ld3(E[i]);
-        float lambda = F[i].w;
+        float lambda = G[i].z;
         const float limit = friction * lamN[i];
         const float prev = E[i].w;
         float tot = prev + lambda;
         tot = clampG(tot, limit, -limit);
         lamT[i] = tot;
         lambda = tot - prev;
-        const V3 nv0 = v0 + lambda * im0 * t, nw0 = w0 + lambda * ld3(F[i]);
-        const V3 nv1 = v1 - lambda * im1 * t, nw1 = w1 - lambda * ld3(G[i]);
-        if (on && b0 >= 0) { v0 = nv0; w0 = nw0; }
-        if (on && b1 >= 0) { v1 = nv1; w1 = nw1; }
+        const F2 l = f2(on && sim0 ? lambda : 0.f, on && sim1 ? lambda : 0.f);
+        axpy(v, l * im, F2x3{f2(E[i].x, -E[i].x), f2(E[i].y, -E[i].y), f2(E[i].z, -E[i].z)});
+        axpy(o, l, F2x3{f2(F[i].x, F[i].y), f2(F[i].z, F[i].w), f2(G[i].x, G[i].y)});
         touched |= on;
     }
 #pragma unroll
     for (int i = 0; i < N; ++i) {
-        if (live[i] & 1) P[i].a.w = lamN[i];
-        if (live[i] & 2) P[i].e.w = lamT[i];
+        if (live[i] & 1) P[i * step].d.x = lamN[i];
+        if (live[i] & 2) P[i * step].e.w = lamT[i];
     }
     if (touched) {
-        if (b0 >= 0) vr.st(b0, v0, w0);
-        if (b1 >= 0) vr.st(b1, v1, w1);
+        V3 v0, w0, v1, w1;
+        f2split(v.x, v0.x, v1.x); f2split(v.y, v0.y, v1.y); f2split(v.z, v0.z, v1.z);
+        f2split(o.x, w0.x, w1.x); f2split(o.y, w0.y, w1.y); f2split(o.z, w0.z, w1.z);
+        if (sim0) vr.st(b0, v0, w0);
+        if (sim1) vr.st(b1, v1, w1);
     }
 }
 
@@ -696,7 +729,7 @@ template <class V>
 __device__ __forceinline__ void contact_step(const SHdr* __restrict__ Hp, SPt* __restrict__ points, bool useBias, const V vr) {
     const SHdr H = *Hp;
     const int np = H.i.z & 0xff;
-    const bool soft = (H.i.z >> 8) != 0;
+    const bool soft = (H.i.z & 0x100) != 0;
     if (soft && !useBias) return;   // the relaxation skips soft contacts
     SPt* P = points + H.i.w;
     const unsigned lanes = __activemask();
@@ -708,12 +741,17 @@ __device__ __forceinline__ void contact_step(const SHdr* __restrict__ Hp, SPt* _
 
 // ---------------------------------------------------------------- bodies
 
-// integrate velocities (src/Physecs.cpp:441-469)
+// integrate velocities (src/Physecs.cpp:441-469) into the solver's velocities; w.vel and
+// w.ang keep the values the substep started with until its end.  Also stores what the
+// contacts' rows read of the body.
 template <class V>
 __device__ void integrate_velocity(const World& w, int d, int ds, float h, float g, const V vr) {
     int b = w.dyn_body[d];
     if (w.info[b].y & BODY_KIN) return;
-    M3 rot = mat3_cast(ld4(w.quat[b]));
+    const Q4 q = ld4(w.quat[b]);
+    w.bq[2 * d] = st4(ld3(w.pos[b]) + qrot(q, ld3(w.com[d])));
+    w.bq[2 * d + 1] = st4(q);
+    M3 rot = mat3_cast(q);
     M3 invRot = transpose(rot);
     V3 vel = ld3(w.vel[d]) + h * V3{0, -g, 0};
     V3 ang = ld3(w.ang[d]);
@@ -724,8 +762,6 @@ __device__ void integrate_velocity(const World& w, int d, int ds, float h, float
     M3 J = madd(I, mscale(h, msub(mm(matrixCross3(wl), I), matrixCross3(mv(I, wl)))));
     wl = wl - solve33(J, f);
     ang = mv(rot, wl);
-    w.vel[d] = st4(vel);
-    w.ang[d] = st4(ang);
     vr.st(d - ds, vel, ang);
     w.pv_v[d] = make_float4(0, 0, 0, 0);
     w.pv_w[d] = make_float4(0, 0, 0, 0);
@@ -962,8 +998,7 @@ __device__ void solve_substeps(const World& w, FrameBuf& f, int s, const S& sy, 
         } else {
             int fit = 0;
             for (int k = tid; k < ncl; k += nth) {
-                const int end = k + 1 < ncl ? f.pt_off[ms + k + 1] : sc.npts;
-                if (kHdrF4 * (k + 1) + kPtF4 * end <= room) fit = k + 1;
+                if (kHdrF4 * (k + 1) + kPtF4 * f.pt_end[ms + k] <= room) fit = k + 1;
             }
             ks = sy.max_int(fit);
         }
@@ -972,22 +1007,17 @@ __device__ void solve_substeps(const World& w, FrameBuf& f, int s, const S& sy, 
     SPt* const Pg = f.s_pts + 4 * (size_t)ms;
     auto HK = [&](int k) -> SHdr& { return SREC && k < ks ? ((SHdr*)(smem + rec_f4))[k] : Hg[k]; };
     auto PK = [&](int k) -> SPt* { return SREC && k < ks ? (SPt*)(smem + rec_f4 + kHdrF4 * ks) : Pg; };
-    for (int k = tid; k < ncl; k += nth) HK(k).i.w = f.pt_off[ms + k];
+    for (int k = tid; k < ncl; k += nth) contact_header(w, f.contacts[f.corder[ms + k]], ds, f.pt_off[ms + k], HK(k));
     sy.sync();
     const int js0 = w.scene_jsteps[s], js1 = w.scene_jsteps[s + 1];
     const int jb = w.scene_joint[s], je = w.scene_joint[s + 1];
     for (int sub = 0; sub < substeps; ++sub) {
-        for (int k = tid; k < ncl; k += nth) {
-            SHdr& H = HK(k);
-            contact_update(w, f.contacts[f.corder[ms + k]], ds, H, PK(k) + H.i.w);
-        }
         for (int j = jb + tid; j < je; j += nth) make_joint_rows(w, j);
-        sy.sync();
         for (int d = ds + tid; d < de; d += nth) integrate_velocity(w, d, ds, h, g, vr);
         sy.sync();
         for (int k = tid; k < ncl; k += nth) {
-            SHdr& H = HK(k);
-            contact_presolve(w, ds, H, PK(k) + H.i.w, h);
+            const SHdr& H = HK(k);
+            contact_rows(w, f.contacts[f.corder[ms + k]], H, PK(k) + H.i.w, h, sub == substeps - 1, vr);
         }
         for (int st = js0; st < js1; ++st) {
             for (int k = w.jstep_start[st] + tid; k < w.jstep_start[st + 1]; k += nth) joint_presolve(w, w.jsched[k]);
@@ -1034,8 +1064,10 @@ __device__ void solve_substeps(const World& w, FrameBuf& f, int s, const S& sy, 
     // accumulated impulses back into the frame's contacts (inspection only)
     for (int k = tid; k < ncl; k += nth) {
         Contact& c = f.contacts[f.corder[ms + k]];
-        const SPt* q = PK(k) + HK(k).i.w;
-        for (int i = 0; i < c.np; ++i) { c.p[i].r0xn.w = q[i].a.w; c.p[i].r1xn.w = q[i].e.w; }
+        const SHdr& H = HK(k);
+        const SPt* q = PK(k) + H.i.w;
+        const int step = H.i.z >> 9;
+        for (int i = 0; i < c.np; ++i) c.lambda[i] = make_float2(q[i * step].d.x, q[i * step].e.w);
     }
 }
 
@@ -1067,7 +1099,7 @@ __device__ void solve_scene(const World& w, FrameBuf& f, int s, const S& sy, int
     // Counting sort of the scene's contacts by colour and, within a colour, by point count
     // (four points first), one bin each: contacts of one colour touch disjoint bodies and
     // may be solved in any order, and a warp of contacts with the same point count runs no
-    // row it does not need.  A contact's first point follows from its bin, so the records
+    // row it does not need.  A contact's point slots follow from its bin, so the records
     // are packed without a scan over the contacts.  A block keeps the bins in shared
     // memory, a grid or cluster counts in global memory and scans once per block.
     const int nbins = kPointBins * ncol;
@@ -1082,8 +1114,7 @@ __device__ void solve_scene(const World& w, FrameBuf& f, int s, const S& sy, int
     for (int k = tid; k < nc; k += nth) { const int cl = col[k]; if (cl >= 0) atomicAdd(&hist[bin_of(cl, k)], 1); }
     sy.sync();
     if (threadIdx.x < 32) {
-        // bin_a: first contact of the bin; bin_b: its first point less (points per contact)
-        // times that, so that a contact's first point is bin_b + k * points
+        // bin_a: first contact of the bin; bin_b: its first point slot
         int c0 = 0, p0 = 0;
         for (int base = 0; base < nbins; base += 32) {
             const int b = base + (int)threadIdx.x, per = 4 - (b & (kPointBins - 1));
@@ -1095,7 +1126,7 @@ __device__ void solve_scene(const World& w, FrameBuf& f, int s, const S& sy, int
             }
             if (b < nbins) {
                 bin_a[b] = c0 + cs - n;
-                bin_b[b] = p0 + ps - n * per - (c0 + cs - n) * per;
+                bin_b[b] = p0 + ps - n * per;
             }
             c0 += __shfl_sync(~0u, cs, 31);
             p0 += __shfl_sync(~0u, ps, 31);
@@ -1111,20 +1142,31 @@ __device__ void solve_scene(const World& w, FrameBuf& f, int s, const S& sy, int
         const int cl = col[k];
         if (S::kBlock) f.color_of[ms + k] = cl;   // kept for inspection
         if (cl < 0 || (serial_last && cl == ncol - 1)) continue;
-        const int b = bin_of(cl, k), per = 4 - (b & (kPointBins - 1));
+        const int b = bin_of(cl, k);
         const int pos = atomicAdd(&cursor[b], 1) + (S::kBlock ? 0 : bin_a[b]);
         f.corder[ms + pos] = ms + k;
-        f.pt_off[ms + pos] = bin_b[b] + pos * per;
     }
     if (serial_last && tid == 0) {
         // the serial colour keeps contact order
         int pos = colstart[ncol - 1];
         for (int k = 0; k < nc; ++k)
-            if (col[k] == ncol - 1) {
-                f.corder[ms + pos] = ms + k;
-                f.pt_off[ms + pos] = bin_b[kPointBins * (ncol - 1)] + pos * 4;
-                ++pos;
-            }
+            if (col[k] == ncol - 1) f.corder[ms + pos++] = ms + k;
+    }
+    sy.sync();
+    // Point slots: eight contacts of a bin side by side (fewer at its end), point by point,
+    // so that the lanes of a warp read a point of theirs at 112-byte steps, which hit every
+    // bank once; a contact's points in a row (448 bytes a contact) put sixteen lanes on
+    // four banks.  pt_off: the contact's first slot and, above bit 28, the step between its
+    // points less one; pt_end: the end of its eight contacts' slots.
+    for (int k = tid; k < ncl; k += nth) {
+        const int m = f.corder[ms + k] - ms, b = bin_of(f.color_of[ms + m], m), per = 4 - (b & (kPointBins - 1));
+        // in block mode the cursors have moved on to each bin's end
+        const bool serial = serial_last && b == kPointBins * (ncol - 1);
+        const int c0 = serial ? colstart[ncol - 1] : (S::kBlock ? (b ? bin_a[b - 1] : 0) : bin_a[b]);
+        const int c1 = serial ? ncl : (S::kBlock ? bin_a[b] : (b + 1 < nbins ? bin_a[b + 1] : ncl));
+        const int i = k - c0, t8 = i & ~7, step = min(8, c1 - c0 - t8);
+        f.pt_off[ms + k] = (bin_b[b] + t8 * per + (i & 7)) | (step - 1) << 28;
+        f.pt_end[ms + k] = bin_b[b] + (t8 + step) * per;
     }
     sy.sync();
     const SortedContacts sc{ms, ncl, npts, ncol, serial_last, colstart};

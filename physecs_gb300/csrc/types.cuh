@@ -63,12 +63,6 @@ struct Manifold {
 struct ContactPt {
     float4 r0;           // local r0, w = targetVelocity
     float4 r1;           // local r1, w = c
-    float4 r0xn;         // w = lambdaN
-    float4 r1xn;         // w = lambdaT
-    float4 t;            // w = invEffMassN
-    float4 r0xt;         // w = invEffMassT
-    float4 r1xt;
-    float4 r0xnt, r1xnt, r0xtt, r1xtt;
 };
 
 struct Contact {         // ContactConstraints (src/ContactConstraints.h:31-48)
@@ -79,6 +73,7 @@ struct Contact {         // ContactConstraints (src/ContactConstraints.h:31-48)
     int np, soft;
     int color, scene, pair, tri;
     ContactPt p[4];
+    float2 lambda[4];    // accumulated normal and friction impulse of each point after the frame
 };
 
 struct Row {             // Constraint1D / Constraint1DW lane
@@ -107,20 +102,22 @@ struct JointDev {
 // Per-substep solver record of one contact (ContactConstraints, src/ContactConstraints.h:31-48),
 // written in colour order:
 //   n = {normal, friction}   m = {invMass0, invMass1, frequency, damping}
-//   i = {dynamic body 0 or -1, dynamic body 1 or -1, numPoints | soft << 8, first point}
+//   i = {scene-local dynamic body 0 or -1, body 1 or -1, numPoints | soft << 8 | step << 9, first
+//        point slot}; the contact's points lie `step` slots apart
 struct SHdr {
     float4 n, m;
     int4 i;
 };
-// One ContactPointConstraints as the iterations read it:
-//   a = {r0 x n, lambdaN}          b = {r1 x n, targetVelocity}
-//   c = {I0 (r0 x n), bias term}   d = {I1 (r1 x n), effective-mass term}
-//   e = {t, lambdaT}               f = {I0 (r0 x t), friction impulse}
-//   g = {I1 (r1 x t), live rows: 1 normal (invEffMassN != 0), 2 friction (invEffMassT != 0)}
-// Between the row update and preSolve, f/g.xyz hold r0 x t / r1 x t and c.w the separation.
+// One ContactPointConstraints as the iterations read it.  The values of the two bodies lie
+// in pairs (lane 0 for body 0, lane 1 for body 1), negated where the constraint's sign asks
+// for it, so that a packed operation serves both:
+//   a = {(-r0 x n, r1 x n).x, .y}      b = {(...).z, (I0 (r0 x n), -I1 (r1 x n)).x}
+//   c = {(...).y, .z}                  d = {lambdaN, targetVelocity, bias term, effective-mass term}
+//   e = {t, lambdaT}                   f = {(I0 (r0 x t), -I1 (r1 x t)).x, .y}
+//   g = {(...).z, friction impulse, live rows: 1 normal (invEffMassN != 0), 2 friction (invEffMassT != 0)}
 // Friction reads the component velocities, which stay fixed through a substep's
 // iterations (ContactConstraints.cpp:93-101), so its unclamped impulse is formed once
-// per substep in preSolve with the same operations.
+// per substep with the same operations.
 struct SPt {
     float4 a, b, c, d, e, f, g;
 };
@@ -165,6 +162,7 @@ struct World {
     float4* pv_v;        // pseudo velocities, w = constraint count
     float4* pv_w;
     float4* mt;          // 3 per dynamic body, world inverse inertia columns
+    float4* bq;          // 2 per dynamic body: world centre of mass and orientation of the substep
     // colliders
     int4* col_info;      // body, type, mesh, flags
     float4* col_pos;

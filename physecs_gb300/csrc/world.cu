@@ -310,6 +310,7 @@ psx_status psx::rt::build_world(psx_world* W, const psx_scene_desc* scenes, int 
     PSX_TRY(W->alloc(w.pv_v, w.n_dyn));
     PSX_TRY(W->alloc(w.pv_w, w.n_dyn));
     PSX_TRY(W->alloc(w.mt, 3 * (size_t)w.n_dyn));
+    PSX_TRY(W->alloc(w.bq, 2 * (size_t)w.n_dyn));
     PSX_TRY(W->upload(w.col_info, col_info));
     PSX_TRY(W->upload(w.col_pos, col_pos));
     PSX_TRY(W->upload(w.col_quat, col_quat));
@@ -421,6 +422,7 @@ psx_status psx::rt::build_world(psx_world* W, const psx_scene_desc* scenes, int 
     PSX_TRY(W->alloc(f.color_start, (size_t)S * kColorBins));
     PSX_TRY(W->alloc(f.claim_pos, (size_t)S * kColorBins));
     PSX_TRY(W->alloc(f.pt_off, f.man_cap));
+    PSX_TRY(W->alloc(f.pt_end, f.man_cap));
     PSX_TRY(W->alloc(f.cbody, f.man_cap));
     PSX_TRY(W->alloc(f.cmask, std::max(1, w.n_dyn)));
     PSX_TRY(W->alloc(f.s_hdr, f.man_cap));
@@ -1365,7 +1367,7 @@ PSX_API int32_t psx_world_get_contacts(psx_world* W, int32_t* ids, float* f, int
                     const ContactPt& p = c.p[k];
                     float* q = o + 8 + 12 * k;
                     q[0] = p.r0.x; q[1] = p.r0.y; q[2] = p.r0.z; q[3] = p.r1.x; q[4] = p.r1.y; q[5] = p.r1.z;
-                    q[6] = p.r0.w; q[7] = p.r1.w; q[8] = p.r0xn.w; q[9] = p.r1xn.w;
+                    q[6] = p.r0.w; q[7] = p.r1.w; q[8] = c.lambda[k].x; q[9] = c.lambda[k].y;
                 }
                 if (meta) { meta[2 * out] = color_of[m]; meta[2 * out + 1] = c.tri; }
             }
