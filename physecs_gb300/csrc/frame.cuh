@@ -37,6 +37,8 @@ struct BVHNodes {
     int* visits;
 };
 
+constexpr int kBarWords = 8;
+
 struct FrameBuf {
     // broadphase
     float4* scene_lo;     // [S] centroid bounds for Morton quantisation
@@ -78,7 +80,7 @@ struct FrameBuf {
     int* man_scene_cnt;   // [S]
     int* scene_man;       // [S+1]
     // colouring
-    unsigned long long* claim;  // [n_dyn] (hashed priority << 32 | contact index)
+    unsigned long long* claim;  // [2 * n_dyn] (colour << 40 | hashed priority << 24 | contact index), two sets a scene
     int* color_of;        // [man_cap]
     int* corder;          // [man_cap] manifolds sorted by (scene, colour, points)
     int* scene_ncolor;    // [S]
@@ -109,8 +111,8 @@ struct FrameBuf {
     int evt_cap;
     int4* trig_evt;                        // [evt_cap] (frame, 0 enter / 1 exit, collider0, collider1)
     int* n_evt;                            // events since the host last drained them (may pass evt_cap)
-    // grid barrier: count, generation, flag
-    unsigned int* bar;
+    // grid barrier: count, generation, unused, maximum, three vote words
+    unsigned int* bar;    // [kBarWords]
     // per-frame totals: contact points, joint rows (for throughput accounting)
     int* n_points;
     int* n_rows;

@@ -800,11 +800,7 @@ struct BlockSync {
     __device__ __forceinline__ void sync() const { __syncthreads(); }
     __device__ __forceinline__ int tid() const { return threadIdx.x; }
     __device__ __forceinline__ int nth() const { return blockDim.x; }
-    __device__ __forceinline__ bool any(bool v) const { return __syncthreads_or(v) != 0; }
-    // bit 0: a == true somewhere, bit 1: b == true somewhere
-    __device__ __forceinline__ int any2(bool a, bool b) const {
-        return (__syncthreads_or(a) ? 1 : 0) | (__syncthreads_or(b) ? 2 : 0);
-    }
+    __device__ __forceinline__ bool any(bool v, int) const { return __syncthreads_or(v) != 0; }
     // block-wide maximum of v (v >= -1)
     __device__ int max_int(int v) const {
         __shared__ int mx;
@@ -824,22 +820,23 @@ struct GridSync {
     __device__ __forceinline__ void sync() const { bar.sync(); }
     __device__ __forceinline__ int tid() const { return blockIdx.x * blockDim.x + threadIdx.x; }
     __device__ __forceinline__ int nth() const { return gridDim.x * blockDim.x; }
-    __device__ __forceinline__ bool any(bool v) const {
-        if (threadIdx.x == 0 && blockIdx.x == 0) atomicExch(flag, 0);
+    // Whether any thread of the grid holds v; `round` counts the calls, with a barrier between
+    // two of them.  Three words take turns: this round's was cleared a round ago, and the one
+    // that the round after the next uses, which every block has read by now, is cleared here.
+    __device__ __forceinline__ bool any(bool v, int round) const {
+        int* slot = flag + 2;
+        if (threadIdx.x == 0 && blockIdx.x == 0) *(volatile int*)(slot + (round + 2) % 3) = 0;
+        if (__syncthreads_or(v) && threadIdx.x == 0) atomicOr(slot + round % 3, 1);
         bar.sync();
-        if (__syncthreads_or(v) && threadIdx.x == 0) atomicOr(flag, 1);
-        bar.sync();
-        bool r = *(volatile int*)flag != 0;
-        bar.sync();
-        return r;
+        return *(volatile int*)(slot + round % 3) != 0;
     }
-    __device__ __forceinline__ int any2(bool a, bool b) const { return (any(a) ? 1 : 0) | (any(b) ? 2 : 0); }
     // grid-wide maximum of v (v >= -1), through the barrier's spare word
     __device__ int max_int(int v) const {
         int* slot = flag + 1;
         if (threadIdx.x == 0 && blockIdx.x == 0) atomicExch(slot, -1);
         bar.sync();
-        atomicMax(slot, v);
+        v = __reduce_max_sync(~0u, v);
+        if ((threadIdx.x & 31) == 0) atomicMax(slot, v);
         bar.sync();
         int r = *(volatile int*)slot;
         bar.sync();
@@ -858,18 +855,15 @@ struct ClusterSync {
     __device__ __forceinline__ void sync() const { cooperative_groups::this_cluster().sync(); }
     __device__ __forceinline__ int tid() const { return rank * blockDim.x + threadIdx.x; }
     __device__ __forceinline__ int nth() const { return R * blockDim.x; }
-    // cluster-wide bitwise OR of v's two low bits (__syncthreads_or only reports "nonzero")
-    __device__ int reduce_or(int v) const {
-        int b = (__syncthreads_or(v & 1) ? 1 : 0) | (__syncthreads_or(v & 2) ? 2 : 0);
+    __device__ bool any(bool v, int) const {
+        const int b = __syncthreads_or(v);
         if (threadIdx.x == 0) red[rank] = b;
         sync();
         int r = 0;
         for (int i = 0; i < R; ++i) r |= red[i];
         sync();
-        return r;
+        return r != 0;
     }
-    __device__ __forceinline__ bool any(bool v) const { return reduce_or(v ? 1 : 0) != 0; }
-    __device__ __forceinline__ int any2(bool a, bool b) const { return reduce_or((a ? 1 : 0) | (b ? 2 : 0)); }
     __device__ int max_int(int v) const {
         __shared__ int bm;
         if (threadIdx.x == 0) bm = -1;
@@ -891,28 +885,33 @@ struct ClusterSync {
 // going to a hashed priority of the contact's index within the scene; a contact
 // accepted by both bodies takes its colour.  At most one contact per body is coloured
 // per round, so no two contacts of a colour share a dynamic body, and the result does
-// not depend on thread timing.  mask[d - ds], claim[d - ds], cb[k], col[k] are indexed
+// not depend on thread timing.  mask[d - ds], claim[d - ds] (two sets of nd, taken in
+// turn, so that one is reset while the other is in use), cb[k], col[k] are indexed
 // by scene-local dynamic body and contact.  Contacts that find no colour below
-// kMaxColors - 1 form a last colour that one thread solves in contact order; the
-// return value is then negative.
+// kMaxColors - 1 (bodies only gain colours, so such a contact never finds one) form a last
+// colour that one thread solves in contact order; the return value is then negative.
+//
+// A round is two barriers and, but for the last, colours at least one contact: the lowest
+// proposal of a round wins both its bodies.
 template <class S>
 __device__ int colour_contacts(const World& w, FrameBuf& f, int ms, int nc, int ds, int nd, const S& sy,
-                               unsigned long long* claim, uint4* mask, int2* cb, int* col) {
+                               unsigned long long* claims, uint4* mask, int2* cb, int* col) {
     const int tid = sy.tid(), nth = sy.nth();
     const unsigned long long kFree = ~0ull;
-    for (int d = tid; d < nd; d += nth) { claim[d] = kFree; mask[d] = make_uint4(0, 0, 0, 0); }
+    for (int d = tid; d < nd; d += nth) { claims[d] = kFree; mask[d] = make_uint4(0, 0, 0, 0); }
     for (int k = tid; k < nc; k += nth) {
-        const Contact& c = f.contacts[ms + k];
-        cb[k] = make_int2(c.b0 >= 0 ? c.b0 - ds : -1, c.b1 >= 0 ? c.b1 - ds : -1);
-        col[k] = -1;
+        const int2 b = *reinterpret_cast<const int2*>(&f.contacts[ms + k].b0);
+        const int2 l = make_int2(b.x >= 0 ? b.x - ds : -1, b.y >= 0 ? b.y - ds : -1);
+        cb[k] = l;
+        col[k] = l.x < 0 && l.y < 0 ? 0 : -1;
     }
     sy.sync();
-    int ncol = 0;
-    bool overflow = false;
     for (int round = 0;; ++round) {
-        bool left = false, committed = false;
+        unsigned long long* claim = claims + (size_t)(round & 1) * nd;
+        unsigned long long* other = claims + (size_t)(~round & 1) * nd;
+        for (int d = tid; d < nd; d += nth) other[d] = kFree;
         for (int k = tid; k < nc; k += nth) {
-            if (col[k] >= 0) continue;
+            if (col[k] != -1) continue;
             const int2 b = cb[k];
             uint4 m0 = b.x >= 0 ? mask[b.x] : make_uint4(0, 0, 0, 0);
             uint4 m1 = b.y >= 0 ? mask[b.y] : make_uint4(0, 0, 0, 0);
@@ -920,7 +919,7 @@ __device__ int colour_contacts(const World& w, FrameBuf& f, int ms, int nc, int 
             int c = kMaxColors - 1;
             for (int q = 0; q < 4; ++q)
                 if (~u[q]) { c = 32 * q + __ffs(~u[q]) - 1; break; }
-            if (c >= kMaxColors - 1) continue;   // no colour left: the serial colour takes it
+            if (c >= kMaxColors - 1) { col[k] = -2; continue; }   // no colour left: the serial colour takes it
             unsigned long long v = ((unsigned long long)c << 40) |
                                    ((unsigned long long)(cache_hash((unsigned long long)k * 0x9E3779B97F4A7C15ull + round) & 0xffffu) << 24) |
                                    (unsigned)k;
@@ -928,17 +927,16 @@ __device__ int colour_contacts(const World& w, FrameBuf& f, int ms, int nc, int 
             if (b.y >= 0) atomicMin(&claim[b.y], v);
         }
         sy.sync();
+        bool left = false;
         for (int k = tid; k < nc; k += nth) {
-            if (col[k] >= 0) continue;
+            if (col[k] != -1) continue;
             const int2 b = cb[k];
-            unsigned long long v0 = b.x >= 0 ? claim[b.x] : kFree, v1 = b.y >= 0 ? claim[b.y] : kFree;
-            bool mine0 = b.x < 0 || (v0 != kFree && (unsigned)(v0 & 0xffffffu) == (unsigned)k);
-            bool mine1 = b.y < 0 || (v1 != kFree && (unsigned)(v1 & 0xffffffu) == (unsigned)k);
-            if (b.x < 0 && b.y < 0) { col[k] = 0; committed = true; continue; }
+            const unsigned long long v0 = b.x >= 0 ? claim[b.x] : kFree, v1 = b.y >= 0 ? claim[b.y] : kFree;
+            const bool mine0 = b.x < 0 || (unsigned)(v0 & 0xffffffu) == (unsigned)k;
+            const bool mine1 = b.y < 0 || (unsigned)(v1 & 0xffffffu) == (unsigned)k;
             if (mine0 && mine1) {
                 int c = (int)((b.x >= 0 ? v0 : v1) >> 40);
                 col[k] = c;
-                committed = true;
                 // each body accepted only this contact this round: plain updates suffice
                 unsigned bit = 1u << (c & 31);
                 int q = c >> 5;
@@ -948,25 +946,17 @@ __device__ int colour_contacts(const World& w, FrameBuf& f, int ms, int nc, int 
                 left = true;
             }
         }
-        sy.sync();
-        for (int d = tid; d < nd; d += nth) claim[d] = kFree;
-        // the lowest proposal of a round always wins both its bodies, so a round without a
-        // new colour means every open contact is out of colours
-        int flags = sy.any2(left, committed);
-        if (!(flags & 1)) break;
-        if (!(flags & 2)) { overflow = true; break; }
+        if (!sy.any(left, round)) break;
     }
     // colours used; contacts left without one form a last colour, solved serially
     int top = -1;
-    for (int k = tid; k < nc; k += nth) if (col[k] >= 0) top = max(top, col[k]);
+    for (int k = tid; k < nc; k += nth) top = max(top, col[k] < 0 ? kMaxColors : col[k]);
     top = sy.max_int(top);
-    ncol = top + 1;
-    if (overflow) {
-        for (int k = tid; k < nc; k += nth) if (col[k] < 0) col[k] = ncol;
-        sy.sync();
-        return -(ncol + 1);   // negative: the last colour is serial
-    }
-    return ncol;
+    if (top < kMaxColors) return top + 1;
+    // a contact without a colour means a body that carries all of them
+    for (int k = tid; k < nc; k += nth) if (col[k] < 0) col[k] = kMaxColors - 1;
+    sy.sync();
+    return -kMaxColors;
 }
 
 // A scene's contacts in solve order: its first manifold, contacts, point slots, colours,
@@ -1080,18 +1070,15 @@ __device__ void solve_scene(const World& w, FrameBuf& f, int s, const S& sy, int
     // bins of the counting sort: bin_a counts, then cursors; bin_b as written by the scan
     __shared__ int bin_a[kColorBins], bin_b[kColorBins], bin_total[2];
     __shared__ int colstart[kMaxColors + 1];   // first contact of each colour, read by every colour step
-    // ---- graph colouring of the contacts.  Each colour is a maximal set of contacts with
-    // no dynamic body in common, grown in rounds: every uncoloured contact whose bodies
-    // the colour does not hold yet claims them with a hashed priority, and the contacts
-    // that hold all their bodies join the colour.  Priorities use the contact's index
-    // within its scene, so a scene is coloured the same way whatever other scenes
+    // ---- graph colouring of the contacts (colour_contacts).  Priorities use the contact's
+    // index within its scene, so a scene is coloured the same way whatever other scenes
     // share the world.  The working arrays (bodies of each contact, colour of each
-    // contact, one claim word per dynamic body) live in shared memory when they fit.
+    // contact, two claim words per dynamic body) live in shared memory when they fit.
     const int nd = de - ds, nc = me - ms;
-    const bool col_smem = !S::kCluster && 24 * (size_t)nd + 12 * (size_t)nc <= 16 * (size_t)smem_f4;
+    const bool col_smem = !S::kCluster && 32 * (size_t)nd + 12 * (size_t)nc <= 16 * (size_t)smem_f4;
     uint4* cmask = col_smem ? (uint4*)smem : f.cmask + ds;
-    unsigned long long* claim = col_smem ? (unsigned long long*)(cmask + nd) : f.claim + ds;
-    int2* cb = col_smem ? (int2*)(claim + nd) : f.cbody + ms;
+    unsigned long long* claim = col_smem ? (unsigned long long*)(cmask + nd) : f.claim + 2 * (size_t)ds;
+    int2* cb = col_smem ? (int2*)(claim + 2 * nd) : f.cbody + ms;
     int* col = col_smem ? (int*)(cb + nc) : f.color_of + ms;
     int ncol = colour_contacts(w, f, ms, nc, ds, nd, sy, claim, cmask, cb, col);
     const bool serial_last = ncol < 0;
@@ -1365,7 +1352,7 @@ int launch_solver(const World& w, FrameBuf& f, const SolverLaunch& L, cudaStream
         long long limit = L.wait_limit > 0 ? L.wait_limit : kDefaultWaitPolls;
         // the barrier's words start from zero in every launch, whatever an earlier launch
         // that gave up on a wait left in them
-        cudaMemsetAsync(f.bar, 0, 4 * sizeof(unsigned), s);
+        cudaMemsetAsync(f.bar, 0, kBarWords * sizeof(unsigned), s);
         void* args[] = {(void*)&wc, (void*)&fc, (void*)&gs, (void*)&ng, (void*)&limit};
         cudaLaunchCooperativeKernel((void*)k_solve_grid, L.grid_blocks, 256, args, 0, s);
         ++k;

@@ -415,7 +415,7 @@ psx_status psx::rt::build_world(psx_world* W, const psx_scene_desc* scenes, int 
     PSX_TRY(W->alloc(f.contacts, f.man_cap));
     PSX_TRY(W->alloc(f.man_scene_cnt, S + 1));
     PSX_TRY(W->alloc(f.scene_man, S + 1));
-    PSX_TRY(W->alloc(f.claim, std::max(1, w.n_dyn)));
+    PSX_TRY(W->alloc(f.claim, 2 * (size_t)std::max(1, w.n_dyn)));
     PSX_TRY(W->alloc(f.color_of, f.man_cap));
     PSX_TRY(W->alloc(f.corder, f.man_cap));
     PSX_TRY(W->alloc(f.scene_ncolor, S));
@@ -430,12 +430,12 @@ psx_status psx::rt::build_world(psx_world* W, const psx_scene_desc* scenes, int 
     PSX_TRY(W->alloc(f.cache_a, f.cache_cap));
     PSX_TRY(W->alloc(f.cache_b, f.cache_cap));
     PSX_TRY(W->alloc(f.cache_parity, 1));
-    PSX_TRY(W->alloc(f.bar, 4));
+    PSX_TRY(W->alloc(f.bar, kBarWords));
     PSX_TRY(W->alloc(f.n_points, 1));
     PSX_TRY(W->alloc(f.n_rows, 1));
     PSX_CUDA(cudaMemset(f.n_points, 0, sizeof(int)));
     PSX_CUDA(cudaMemset(f.n_rows, 0, sizeof(int)));
-    PSX_CUDA(cudaMemset(f.bar, 0, 4 * sizeof(unsigned)));
+    PSX_CUDA(cudaMemset(f.bar, 0, kBarWords * sizeof(unsigned)));
     PSX_CUDA(cudaMemset(f.cache_parity, 0, sizeof(int)));
     PSX_CUDA(cudaMemset(f.cache_a, 0xff, sizeof(CacheEntry) * (size_t)f.cache_cap));
     PSX_CUDA(cudaMemset(f.cache_b, 0xff, sizeof(CacheEntry) * (size_t)f.cache_cap));
