@@ -173,6 +173,15 @@ __global__ void k_joint_layout(World w, int* n_rows) {
     w.joints[j].makeLower = J.makeLower;
     w.joints[j].nrows = n;
     for (int i = 0; i < kMaxRowsPerJoint; ++i) w.joints[j].rowflags[i] = J.rowflags[i];
+    // preSolve and solve take the rows by kind, in this order of their flags
+    unsigned order = 0;
+    int taken = 0;
+    const int kinds[6] = {RN, RA, RS, RL, RA | RS, RA | RL};
+    for (int kind : kinds)
+        for (int i = 0; i < n; ++i)
+            if (J.rowflags[i] == kind) order |= (unsigned)i << (4 * taken++);
+    w.joints[j].order = order;
+    w.joints[j].norder = taken;
     for (int i = 0; i < n; ++i) {
         Row r;
         r.linear = make_float4(0, 0, 0, 0);
@@ -311,55 +320,63 @@ __device__ void make_joint_rows(const World& w, int j) {
     }
 }
 
-// Constraint1D(W)::preSolve for one row (Constraint1D.cpp:5-52 / Constraint1DW.cpp:5-115)
-__device__ void row_presolve(const World& w, Row& r, bool simd) {
-    int fl = r.flags;
-    bool angf = fl & 2, soft = fl & 1, lim = fl & 4;
+// Constraint1D(W)::preSolve (Constraint1D.cpp:5-52 / Constraint1DW.cpp:5-115) of a joint's
+// rows in solve order.  Every row of a joint has its two bodies, whose inertia is read once
+// and whose pseudo velocities (with the count of rows applied) stay in registers.
+__device__ void joint_presolve(const World& w, int j) {
+    const JointDev& J = w.joints[j];
+    Row* const R = w.rows + (size_t)j * kMaxRowsPerJoint;
+    const int b0 = J.b0, b1 = J.b1, n = J.norder;
+    const bool simd = J.simd != 0, same = b0 >= 0 && b0 == b1;
     float im0 = 0, im1 = 0;
     M3 I0 = m3zero(), I1 = m3zero();
-    if (r.b0 >= 0) { im0 = w.com[r.b0].w; I0 = m3cols(ld3(w.mt[3 * r.b0]), ld3(w.mt[3 * r.b0 + 1]), ld3(w.mt[3 * r.b0 + 2])); }
-    if (r.b1 >= 0) { im1 = w.com[r.b1].w; I1 = m3cols(ld3(w.mt[3 * r.b1]), ld3(w.mt[3 * r.b1 + 1]), ld3(w.mt[3 * r.b1 + 2])); }
-    V3 a0 = ld3(r.angular0), a1 = ld3(r.angular1), l = ld3(r.linear);
-    V3 a0t = mv(I0, a0), a1t = mv(I1, a1);
-    float inv = dot(a0, a0t) + dot(a1, a1t);
-    V3 l0t = ld3(r.linear0t), l1t = ld3(r.linear1t);
-    if (!angf) {
-        inv += dot(l, l) * (im0 + im1);
-        l0t = im0 * l;
-        l1t = im1 * l;
+    float4 pv0 = make_float4(0, 0, 0, 0), pw0 = pv0, pv1 = pv0, pw1 = pv0;
+    if (b0 >= 0) {
+        im0 = w.com[b0].w; I0 = m3cols(ld3(w.mt[3 * b0]), ld3(w.mt[3 * b0 + 1]), ld3(w.mt[3 * b0 + 2]));
+        pv0 = w.pv_v[b0]; pw0 = w.pv_w[b0];
     }
-    r.angular0t = st4(a0t, r.angular0t.w);
-    r.angular1t = st4(a1t, inv);
-    r.linear0t = st4(l0t, r.linear0t.w);
-    r.linear1t = st4(l1t, r.linear1t.w);
-    if (soft) return;
-    float c = r.angular0.w, mn = r.angular1.w, mx = r.linear0t.w;
-    float lambda;
-    if (!simd) {
-        if (!c || !inv) return;
-        lambda = c / inv;
-        if (lim) lambda = clampG(lambda, mn, mx);
-    } else {
-        if (!(inv != 0.f && c != 0.f)) return;
-        lambda = c / inv;
-        if (lim) { lambda = lambda > mn ? lambda : mn; lambda = lambda < mx ? lambda : mx; }
+    if (b1 >= 0) {
+        im1 = w.com[b1].w; I1 = m3cols(ld3(w.mt[3 * b1]), ld3(w.mt[3 * b1 + 1]), ld3(w.mt[3 * b1 + 2]));
+        pv1 = w.pv_v[b1]; pw1 = w.pv_w[b1];
     }
-    if (r.b0 >= 0) {
-        float4 pv = w.pv_v[r.b0], pw = w.pv_w[r.b0];
-        V3 v = ld3(pv), wv = ld3(pw);
-        if (!angf) v += lambda * l0t;
-        wv += lambda * a0t;
-        w.pv_v[r.b0] = st4(v, pv.w + 1.f);
-        w.pv_w[r.b0] = st4(wv, 0.f);
+    unsigned order = J.order;
+    for (int i = 0; i < n; ++i, order >>= 4) {
+        Row& r = R[order & 15u];
+        const int fl = r.flags;
+        const bool angf = fl & 2, soft = fl & 1, lim = fl & 4;
+        const V3 a0 = ld3(r.angular0), a1 = ld3(r.angular1), l = ld3(r.linear);
+        const V3 a0t = mv(I0, a0), a1t = mv(I1, a1);
+        float inv = dot(a0, a0t) + dot(a1, a1t);
+        V3 l0t = ld3(r.linear0t), l1t = ld3(r.linear1t);
+        if (!angf) {
+            inv += dot(l, l) * (im0 + im1);
+            l0t = im0 * l;
+            l1t = im1 * l;
+        }
+        const float c = r.angular0.w, mn = r.angular1.w, mx = r.linear0t.w;
+        r.angular0t = st4(a0t, r.angular0t.w);
+        r.angular1t = st4(a1t, inv);
+        r.linear0t = st4(l0t, mx);
+        r.linear1t = st4(l1t, r.linear1t.w);
+        if (soft || !(inv != 0.f && c != 0.f)) continue;
+        float lambda = c / inv;
+        if (lim) {
+            if (simd) { lambda = lambda > mn ? lambda : mn; lambda = lambda < mx ? lambda : mx; }
+            else lambda = clampG(lambda, mn, mx);
+        }
+        if (b0 >= 0) {
+            pv0 = st4(angf ? ld3(pv0) : ld3(pv0) + lambda * l0t, pv0.w + 1.f);
+            pw0 = st4(ld3(pw0) + lambda * a0t, 0.f);
+        }
+        if (same) { pv1 = pv0; pw1 = pw0; }
+        if (b1 >= 0) {
+            pv1 = st4(angf ? ld3(pv1) : ld3(pv1) - lambda * l1t, pv1.w + 1.f);
+            pw1 = st4(ld3(pw1) - lambda * a1t, 0.f);
+        }
+        if (same) { pv0 = pv1; pw0 = pw1; }
     }
-    if (r.b1 >= 0) {
-        float4 pv = w.pv_v[r.b1], pw = w.pv_w[r.b1];
-        V3 v = ld3(pv), wv = ld3(pw);
-        if (!angf) v -= lambda * l1t;
-        wv -= lambda * a1t;
-        w.pv_v[r.b1] = st4(v, pv.w + 1.f);
-        w.pv_w[r.b1] = st4(wv, 0.f);
-    }
+    if (b0 >= 0) { w.pv_v[b0] = pv0; w.pv_w[b0] = pw0; }
+    if (b1 >= 0) { w.pv_v[b1] = pv1; w.pv_w[b1] = pw1; }
 }
 
 // The dynamic shared memory of the solver kernels: velocities, then contact records.
@@ -407,38 +424,38 @@ struct GlobVel {
     __device__ __forceinline__ void st(int i, V3 v, V3 w) const { v_[i] = st4(v); w_[i] = st4(w); }
 };
 
-// Constraint1D(W)::solve for one row (Constraint1D.cpp:54-127 / Constraint1DW.cpp:117-233)
-template <class V>
-__device__ void row_solve(Row& r, float h, bool warm, bool simd, int ds, const V vr) {
-    int fl = r.flags;
-    bool angf = fl & 2, soft = fl & 1, lim = fl & 4;
-    float inv = r.angular1t.w;
+// Constraint1D(W)::solve for one row (Constraint1D.cpp:54-127 / Constraint1DW.cpp:117-233).
+// V0, W0, V1, W1: the velocities of the joint's bodies (zero, and left so, for a side that
+// is not simulated: s0, s1; `same`: both sides are one body).  total: the row's accumulated
+// impulse.  bias: 0.2 / h, formed once per substep (the device divides f64 slowly).
+__device__ __forceinline__ void row_solve(const Row& r, float& total, float h, float bias, bool warm, bool simd, bool s0,
+                                          bool s1, bool same, V3& V0, V3& W0, V3& V1, V3& W1) {
+    const int fl = r.flags;
+    const bool angf = fl & 2, soft = fl & 1, lim = fl & 4;
+    const float inv = r.angular1t.w;
     if (!simd && !inv) return;
-    // an angular row neither uses nor changes the linear velocities
-    V3 v0 = {0, 0, 0}, w0 = {0, 0, 0}, v1 = {0, 0, 0}, w1 = {0, 0, 0};
-    if (r.b0 >= 0) vr.ld(r.b0 - ds, v0, w0);
-    if (r.b1 >= 0) vr.ld(r.b1 - ds, v1, w1);
-    V3 l0t = ld3(r.linear0t), l1t = ld3(r.linear1t), a0t = ld3(r.angular0t), a1t = ld3(r.angular1t);
-    float c = r.angular0.w;
+    V3 v0 = V0, w0 = W0, v1 = V1, w1 = W1;
+    const V3 l0t = ld3(r.linear0t), l1t = ld3(r.linear1t), a0t = ld3(r.angular0t), a1t = ld3(r.angular1t);
+    const float c = r.angular0.w;
     if (!soft && warm) {
-        bool apply = simd ? (fabsf(c) < (float)1e-4 && fabsf(r.totalLambda) < 10000.f)
-                          : !((double)fabsf(c) > 1e-4 || fabsf(r.totalLambda) > 10000.f);
+        const bool apply = simd ? (fabsf(c) < (float)1e-4 && fabsf(total) < 10000.f)
+                                : !((double)fabsf(c) > 1e-4 || fabsf(total) > 10000.f);
         if (apply) {
-            float lw = r.totalLambda * 0.5f;
-            r.totalLambda = lw;
+            const float lw = total * 0.5f;
+            total = lw;
             if (!angf) { v0 += lw * l0t; v1 -= lw * l1t; }
             w0 += lw * a0t;
             w1 -= lw * a1t;
         }
     }
     if (simd && !inv) return;
-    V3 a0 = ld3(r.angular0), a1 = ld3(r.angular1), l = ld3(r.linear);
+    const V3 a0 = ld3(r.angular0), a1 = ld3(r.angular1), l = ld3(r.linear);
     float rv = dot(a1, w1) - dot(a0, w0);
     if (!angf) rv += dot(l, v1) - dot(l, v0);
-    float tvel = r.linear.w, mn = r.angular1.w, mx = r.linear0t.w, freq = r.linear1t.w, damp = r.angular0t.w;
+    const float tvel = r.linear.w, mn = r.angular1.w, mx = r.linear0t.w, freq = r.linear1t.w, damp = r.angular0t.w;
     float lambda;
     if (simd) {
-        float eff = 1.f / inv;
+        const float eff = 1.f / inv;
         if (soft) {
             float af = (2.f * kPi) * freq;
             float stiffness = af * af * eff;
@@ -447,7 +464,6 @@ __device__ void row_solve(Row& r, float h, bool warm, bool simd, int ds, const V
             float beta = h * stiffness * gamma;
             lambda = (rv + beta * c / h) / (inv + gamma / h);
         } else {
-            float bias = (float)(0.2 / (double)h);
             lambda = (rv - tvel + bias * c) * eff;
         }
     } else {
@@ -463,55 +479,67 @@ __device__ void row_solve(Row& r, float h, bool warm, bool simd, int ds, const V
         }
     }
     if (lim) {
-        float prev = r.totalLambda;
-        r.totalLambda += lambda;
+        const float prev = total;
+        total += lambda;
         if (simd) {
             float lo = mn * h, hi = mx * h;
-            r.totalLambda = r.totalLambda > lo ? r.totalLambda : lo;
-            r.totalLambda = r.totalLambda < hi ? r.totalLambda : hi;
+            total = total > lo ? total : lo;
+            total = total < hi ? total : hi;
         } else {
-            r.totalLambda = clampG(r.totalLambda, mn, mx);
+            total = clampG(total, mn, mx);
         }
-        lambda = r.totalLambda - prev;
+        lambda = total - prev;
     } else {
-        r.totalLambda += lambda;
+        total += lambda;
     }
-    if (!simd) {
-        // the scalar row applies only this iteration's impulse (Constraint1D.cpp:158-168)
-        if (r.b0 >= 0) {
-            vr.ld(r.b0 - ds, v0, w0);
-            vr.st(r.b0 - ds, angf ? v0 : v0 + lambda * l0t, w0 + lambda * a0t);
-        }
-        if (r.b1 >= 0) {
-            vr.ld(r.b1 - ds, v1, w1);
-            vr.st(r.b1 - ds, angf ? v1 : v1 - lambda * l1t, w1 - lambda * a1t);
-        }
-        return;
-    }
-    if (!angf) { v0 += lambda * l0t; v1 -= lambda * l1t; }
+    // the scalar row applies only this iteration's impulse (Constraint1D.cpp:158-168): to
+    // the stored velocities, not to those the warm start changed
+    if (!simd) { v0 = V0; w0 = W0; }
+    if (!angf) v0 += lambda * l0t;
     w0 += lambda * a0t;
+    if (s0) { V0 = v0; W0 = w0; }
+    if (!simd) {
+        if (same) { V1 = V0; W1 = W0; }
+        v1 = V1; w1 = W1;
+    }
+    if (!angf) v1 -= lambda * l1t;
     w1 -= lambda * a1t;
-    if (r.b0 >= 0) vr.st(r.b0 - ds, v0, w0);
-    if (r.b1 >= 0) vr.st(r.b1 - ds, v1, w1);
+    if (s1) { V1 = v1; W1 = w1; }
+    if (same) { V0 = V1; W0 = W1; }
 }
 
-__constant__ int c_flag_order[6] = {0, 2, 1, 4, 3, 6};
-
-__device__ void joint_presolve(const World& w, int j) {
-    JointDev& J = w.joints[j];
-    Row* R = w.rows + j * kMaxRowsPerJoint;
-    for (int fi = 0; fi < 6; ++fi)
-        for (int k = 0; k < J.nrows; ++k)
-            if (J.rowflags[k] == c_flag_order[fi]) row_presolve(w, R[k], J.simd != 0);
+// A joint's rows in solve order, on its bodies' velocities in registers; the next row's
+// record is read while one is solved (a row is a chain of about twenty dependent
+// operations, its record comes from L2).
+__device__ __forceinline__ void joint_rows_solve(const World& w, int j, float h, float bias, bool warm, V3& v0, V3& w0,
+                                                 V3& v1, V3& w1) {
+    const JointDev& J = w.joints[j];
+    Row* const R = w.rows + (size_t)j * kMaxRowsPerJoint;
+    const int b0 = J.b0, b1 = J.b1, n = J.norder;
+    const bool simd = J.simd != 0, same = b0 >= 0 && b0 == b1;
+    unsigned order = J.order;
+    if (!n) return;
+    Row next = R[order & 15u];
+    for (int i = 0; i < n; ++i) {
+        const Row r = next;
+        Row* const at = R + (order & 15u);
+        order >>= 4;
+        if (i + 1 < n) next = R[order & 15u];
+        float total = r.totalLambda;
+        row_solve(r, total, h, bias, warm, simd, b0 >= 0, b1 >= 0, same, v0, w0, v1, w1);
+        at->totalLambda = total;
+    }
 }
 
 template <class V>
-__device__ void joint_solve(const World& w, int j, float h, bool warm, int ds, const V vr) {
-    JointDev& J = w.joints[j];
-    Row* R = w.rows + j * kMaxRowsPerJoint;
-    for (int fi = 0; fi < 6; ++fi)
-        for (int k = 0; k < J.nrows; ++k)
-            if (J.rowflags[k] == c_flag_order[fi]) row_solve(R[k], h, warm, J.simd != 0, ds, vr);
+__device__ void joint_solve(const World& w, int j, float h, float bias, bool warm, int ds, const V vr) {
+    const int b0 = w.joints[j].b0, b1 = w.joints[j].b1;
+    V3 v0 = {0, 0, 0}, w0 = {0, 0, 0}, v1 = {0, 0, 0}, w1 = {0, 0, 0};
+    if (b0 >= 0) vr.ld(b0 - ds, v0, w0);
+    if (b1 >= 0) vr.ld(b1 - ds, v1, w1);
+    joint_rows_solve(w, j, h, bias, warm, v0, w0, v1, w1);
+    if (b0 >= 0) vr.st(b0 - ds, v0, w0);
+    if (b1 >= 0) vr.st(b1 - ds, v1, w1);
 }
 
 // ---------------------------------------------------------------- contacts (ContactConstraints.cpp)
@@ -1001,6 +1029,7 @@ __device__ void solve_substeps(const World& w, FrameBuf& f, int s, const S& sy, 
     sy.sync();
     const int js0 = w.scene_jsteps[s], js1 = w.scene_jsteps[s + 1];
     const int jb = w.scene_joint[s], je = w.scene_joint[s + 1];
+    const float joint_bias = jb < je ? (float)(0.2 / (double)h) : 0.f;
     for (int sub = 0; sub < substeps; ++sub) {
         for (int j = jb + tid; j < je; j += nth) make_joint_rows(w, j);
         for (int d = ds + tid; d < de; d += nth) integrate_velocity(w, d, ds, h, g, vr);
@@ -1037,7 +1066,7 @@ __device__ void solve_substeps(const World& w, FrameBuf& f, int s, const S& sy, 
             if (bias)
                 for (int st = js0; st < js1; ++st) {
                     for (int k = w.jstep_start[st] + tid; k < w.jstep_start[st + 1]; k += nth)
-                        joint_solve(w, w.jsched[k], h, it == 0, ds, vr);
+                        joint_solve(w, w.jsched[k], h, joint_bias, it == 0, ds, vr);
                     sy.sync();
                 }
         }

@@ -94,7 +94,10 @@ struct JointDev {
     float4 a0p, a0q, a1p, a1q;
     float4 r0, r1;                   // anchor relative to COM when dynamic
     float params[8];
-    int makeUpper, makeLower, gearInit, pad;
+    int makeUpper, makeLower, gearInit;
+    int norder;                      // rows solved each iteration, and their indices in solve order,
+    unsigned order;                  // four bits each, the first lowest
+    int pad[3];
     float persistent0, persistent1, virtual0, virtual1;
     int rowflags[kMaxRowsPerJoint];
 };
