@@ -97,7 +97,8 @@ struct JointDev {
     int makeUpper, makeLower, gearInit;
     int norder;                      // rows solved each iteration, and their indices in solve order,
     unsigned order;                  // four bits each, the first lowest
-    int pad[3];
+    int rank0, rank1;                // joints before this one, in solve order, on its two bodies
+    int pad;
     float persistent0, persistent1, virtual0, virtual1;
     int rowflags[kMaxRowsPerJoint];
 };
@@ -160,12 +161,14 @@ struct World {
     float4* ang;
     float4* com;         // xyz com, w invMass
     float4* invI;        // 3 per dynamic body, local inverse inertia columns
-    float4* vt_v;        // solver velocities
-    float4* vt_w;
+    float4* vt;          // 2 per dynamic body: solver velocities; w = solves done this substep (solve_flow)
     float4* pv_v;        // pseudo velocities, w = constraint count
     float4* pv_w;
     float4* mt;          // 3 per dynamic body, world inverse inertia columns
     float4* bq;          // 2 per dynamic body: world centre of mass and orientation of the substep
+    float4* sv;          // 2 per dynamic body: the substep's integrated velocities (solve_flow)
+    int* body_nj;        // joints of each dynamic body
+    int self_joint;      // some joint has one body at both ends
     // colliders
     int4* col_info;      // body, type, mesh, flags
     float4* col_pos;

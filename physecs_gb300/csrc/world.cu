@@ -305,12 +305,12 @@ psx_status psx::rt::build_world(psx_world* W, const psx_scene_desc* scenes, int 
     PSX_TRY(W->upload(w.ang, ang));
     PSX_TRY(W->upload(w.com, com));
     PSX_TRY(W->upload(w.invI, invI));
-    PSX_TRY(W->alloc(w.vt_v, w.n_dyn));
-    PSX_TRY(W->alloc(w.vt_w, w.n_dyn));
+    PSX_TRY(W->alloc(w.vt, 2 * (size_t)w.n_dyn));
     PSX_TRY(W->alloc(w.pv_v, w.n_dyn));
     PSX_TRY(W->alloc(w.pv_w, w.n_dyn));
     PSX_TRY(W->alloc(w.mt, 3 * (size_t)w.n_dyn));
     PSX_TRY(W->alloc(w.bq, 2 * (size_t)w.n_dyn));
+    PSX_TRY(W->alloc(w.sv, 2 * (size_t)w.n_dyn));
     PSX_TRY(W->upload(w.col_info, col_info));
     PSX_TRY(W->upload(w.col_pos, col_pos));
     PSX_TRY(W->upload(w.col_quat, col_quat));
@@ -353,6 +353,17 @@ psx_status psx::rt::build_world(psx_world* W, const psx_scene_desc* scenes, int 
         PSX_TRY(W->upload(w.trimesh_chunks, tch));
         w.n_trimesh_chunks = (int)tch.size();
         PSX_TRY(W->alloc(w.trimesh_keys, 6 * tcols.size()));
+    }
+    {   // each joint's place among its bodies' joints, in solve order
+        std::vector<int> nj(std::max(1, w.n_dyn), 0);
+        for (int j : jsched) {
+            JointDev& J = joints[j];
+            const int d0 = W->h_body_dyn[J.body0], d1 = W->h_body_dyn[J.body1];
+            J.rank0 = d0 >= 0 ? nj[d0]++ : 0;
+            J.rank1 = d1 >= 0 ? nj[d1]++ : 0;
+            if (J.body0 == J.body1) w.self_joint = 1;
+        }
+        PSX_TRY(W->upload(w.body_nj, nj));
     }
     PSX_TRY(W->upload(w.joints, joints));
     PSX_TRY(W->alloc(w.rows, (size_t)kMaxRowsPerJoint * std::max(1, w.n_joints)));
@@ -425,6 +436,7 @@ psx_status psx::rt::build_world(psx_world* W, const psx_scene_desc* scenes, int 
     PSX_TRY(W->alloc(f.pt_end, f.man_cap));
     PSX_TRY(W->alloc(f.cbody, f.man_cap));
     PSX_TRY(W->alloc(f.cmask, std::max(1, w.n_dyn)));
+    PSX_TRY(W->alloc(f.bdeg, std::max(1, w.n_dyn)));
     PSX_TRY(W->alloc(f.s_hdr, f.man_cap));
     PSX_TRY(W->alloc(f.s_pts, 4 * (size_t)f.man_cap));
     PSX_TRY(W->alloc(f.cache_a, f.cache_cap));

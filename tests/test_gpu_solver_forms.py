@@ -56,3 +56,42 @@ def test_contact_forms_match_the_oracle(n, opts, soft, gpu_lib, oracle_lib):
     if n >= 300:
         assert {1, 2, 4} <= seen
     g.close()
+
+
+def _lockstep(s, frames, **opts):
+    from oracle.port_api import OracleScene
+    from physecs_gb300.api import World
+    g, o = World([s], **opts), OracleScene(s)
+    for frame in range(frames):
+        g.step()
+        g.synchronize()
+        ids, _, meta = g.contacts()
+        o.set_contact_order(gpu_keys(ids, meta))
+        o.step()
+        assert o.order_error() == 0
+        assert rel_state_diff(g.read_bodies(), o.state()) <= 1e-5, frame
+    assert g.counts()["error"] == 0
+    g.close()
+
+
+@pytest.mark.parametrize("substeps,iterations", [(1, 0), (1, 1), (3, 5)])
+@pytest.mark.parametrize("name", ["chains", "mechanisms", "free"])
+def test_whole_grid_without_barriers_between_colours(name, substeps, iterations, gpu_lib, oracle_lib):
+    """Joints of every kind, contacts alone and no contacts at all, solved by the whole grid
+    as each body's earlier solves finish; sweeps with no iteration, one and several."""
+    from tests.scene_variants import apart_scene, mechanism_scene
+    if name == "chains":
+        s = scenes.joint_chains(n_chains=9, links=11)
+    elif name == "mechanisms":
+        s = mechanism_scene()
+        s = s[0] if isinstance(s, tuple) else s
+    else:
+        s = apart_scene()
+    s.num_substeps, s.num_iterations = substeps, iterations
+    _lockstep(s, 8, block_scene_max_dyn=1, launch={"large_scene_solver": 2})
+
+
+def test_whole_grid_beyond_the_colour_limit(gpu_lib, oracle_lib):
+    """A serial last colour keeps its contact order on the grid as well."""
+    from tests.test_gpu_parity import _plate_with_spheres
+    _lockstep(_plate_with_spheres(), 3, block_scene_max_dyn=1, launch={"large_scene_solver": 2})
