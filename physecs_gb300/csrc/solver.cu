@@ -135,11 +135,18 @@ __global__ void k_build_contacts(World w, FrameBuf f) {
 
 // ---------------------------------------------------------------- joints
 
+// The rows of schedule entry q (types.cuh): row k, field f at [(k * kRowF4 + f) * 32].
+__device__ __forceinline__ float4* joint_rows(const World& w, int q) {
+    return w.rows + (size_t)(q >> 5) * (kMaxRowsPerJoint * kRowF4 * 32) + (q & 31);
+}
+constexpr int kRowStep = kRowF4 * 32;
+
 // getSolverDesc of each joint type (src/Joints/*.cpp): row flags in creation order,
 // evaluated at frame start; the prismatic limit row exists only while violated.
 __global__ void k_joint_layout(World w, int* n_rows) {
-    int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= w.n_joints) return;
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= w.n_joints) return;
+    const int j = w.jsched[q];
     JointDev J = w.joints[j];
     int f[kMaxRowsPerJoint];
     int n = 0;
@@ -174,27 +181,25 @@ __global__ void k_joint_layout(World w, int* n_rows) {
     w.joints[j].nrows = n;
     for (int i = 0; i < kMaxRowsPerJoint; ++i) w.joints[j].rowflags[i] = J.rowflags[i];
     // preSolve and solve take the rows by kind, in this order of their flags
-    unsigned order = 0;
+    unsigned place = 0;
     int taken = 0;
     const int kinds[6] = {RN, RA, RS, RL, RA | RS, RA | RL};
+    float4* const R = joint_rows(w, q);
     for (int kind : kinds)
-        for (int i = 0; i < n; ++i)
-            if (J.rowflags[i] == kind) order |= (unsigned)i << (4 * taken++);
-    w.joints[j].order = order;
-    w.joints[j].norder = taken;
-    for (int i = 0; i < n; ++i) {
-        Row r;
-        r.linear = make_float4(0, 0, 0, 0);
-        r.angular0 = make_float4(0, 0, 0, 0);
-        r.angular1 = make_float4(0, 0, 0, -FLT_MAX);
-        r.linear0t = make_float4(0, 0, 0, FLT_MAX);
-        r.linear1t = make_float4(0, 0, 0, 0);
-        r.angular0t = make_float4(0, 0, 0, 0);
-        r.angular1t = make_float4(0, 0, 0, 0);
-        r.totalLambda = 0;
-        r.flags = f[i]; r.b0 = J.b0; r.b1 = J.b1;
-        w.rows[j * kMaxRowsPerJoint + i] = r;
-    }
+        for (int i = 0; i < n; ++i) {
+            if (J.rowflags[i] != kind) continue;
+            place |= (unsigned)taken << (4 * i);
+            float4* const r = R + taken++ * kRowStep;
+            r[32 * ROW_LINEAR] = make_float4(0, 0, 0, 0);
+            r[32 * ROW_ANGULAR0] = make_float4(0, 0, 0, 0);
+            r[32 * ROW_ANGULAR1] = make_float4(0, 0, 0, -FLT_MAX);
+            r[32 * ROW_ANGULAR0T] = make_float4(0, 0, 0, __int_as_float(kind));
+            r[32 * ROW_ANGULAR1T] = make_float4(0, 0, 0, 0);
+            r[32 * ROW_MISC] = make_float4(FLT_MAX, 0, 0, 0);
+        }
+    w.joints[j].place = place;
+    w.jruns[q] = JointRun{J.b0, J.b1, n | J.simd << 8, J.b0 >= 0 ? w.com[J.b0].w : 0.f, J.b1 >= 0 ? w.com[J.b1].w : 0.f,
+                          J.rank0, J.rank1, 0};
 }
 
 int launch_joint_layout(const World& w, FrameBuf& f, cudaStream_t s) {
@@ -210,20 +215,25 @@ __device__ __forceinline__ float angleDiffD(float a0, float a1) {  // GearJoint.
     return diff < -pi ? diff + two_pi : diff;
 }
 
-// makeConstraints of each joint type (src/Joints/*.cpp, src/JointsUtil.h:8-28), rows in creation order
-__device__ void make_joint_rows(const World& w, int j) {
-    JointDev& J = w.joints[j];
+// makeConstraints of each joint type (src/Joints/*.cpp, src/JointsUtil.h:8-28) for schedule
+// entry q, rows taken in creation order
+__device__ void make_joint_rows(const World& w, int q) {
+    JointDev& J = w.joints[w.jsched[q]];
     Q4 q0 = ld4(w.quat[J.body0]), q1 = ld4(w.quat[J.body1]);
     M3 u0 = mat3_cast(qmul(q0, ld4(J.a0q))), u1 = mat3_cast(qmul(q1, ld4(J.a1q)));
     V3 r0 = qrot(q0, ld3(J.r0)), r1 = qrot(q1, ld3(J.r1));
     V3 p0 = ld3(w.pos[J.body0]) + qrot(q0, ld3(J.a0p)), p1 = ld3(w.pos[J.body1]) + qrot(q1, ld3(J.a1p));
-    Row* R = w.rows + j * kMaxRowsPerJoint;
+    float4* const R = joint_rows(w, q);
+    const unsigned place = J.place;
     int k = 0;
-    auto lin = [&](V3 l, V3 a0, V3 a1, float c) {
-        R[k].linear = st4(l, R[k].linear.w); R[k].angular0 = st4(a0, c); R[k].angular1 = st4(a1, R[k].angular1.w); ++k;
+    auto row = [&]() { return R + ((place >> (4 * k)) & 15u) * kRowStep; };
+    auto lin = [&](V3 l, V3 a0, V3 a1, float c, float lo = -FLT_MAX) {
+        float4* const r = row();
+        r[32 * ROW_LINEAR] = st4(l, 0.f); r[32 * ROW_ANGULAR0] = st4(a0, c); r[32 * ROW_ANGULAR1] = st4(a1, lo); ++k;
     };
-    auto ang = [&](V3 a, float c) {
-        R[k].angular0 = st4(a, c); R[k].angular1 = st4(a, R[k].angular1.w); ++k;
+    auto ang = [&](V3 a0, V3 a1, float c) {
+        float4* const r = row();
+        r[32 * ROW_ANGULAR0] = st4(a0, c); r[32 * ROW_ANGULAR1] = st4(a1, -FLT_MAX); ++k;
     };
     auto p2p = [&]() {
         V3 d = p1 - p0;
@@ -231,62 +241,61 @@ __device__ void make_joint_rows(const World& w, int j) {
         lin({0, 1, 0}, {-r0.z, 0, r0.x}, {-r1.z, 0, r1.x}, d.y);
         lin({0, 0, 1}, {r0.y, -r0.x, 0}, {r1.y, -r1.x, 0}, d.z);
     };
+    auto angs = [&](V3 a, float c) { ang(a, a, c); };
     switch (J.type) {
         case 0:
             p2p();
-            ang(cross(u1.c[1], u0.c[0]), dot(u0.c[0], u1.c[1]));
-            ang(cross(u1.c[2], u0.c[0]), dot(u0.c[0], u1.c[2]));
-            ang(cross(u1.c[2], u0.c[1]), dot(u0.c[1], u1.c[2]));
+            angs(cross(u1.c[1], u0.c[0]), dot(u0.c[0], u1.c[1]));
+            angs(cross(u1.c[2], u0.c[0]), dot(u0.c[0], u1.c[2]));
+            angs(cross(u1.c[2], u0.c[1]), dot(u0.c[1], u1.c[2]));
             break;
         case 2: p2p(); break;
         case 4:
             p2p();
-            ang(cross(u1.c[2], u0.c[2]), dot(u0.c[2], u1.c[2]));
+            angs(cross(u1.c[2], u0.c[2]), dot(u0.c[2], u1.c[2]));
             break;
         case 1:
             p2p();
-            ang(cross(u1.c[1], u0.c[0]), dot(u0.c[0], u1.c[1]));
-            ang(cross(u1.c[2], u0.c[0]), dot(u0.c[0], u1.c[2]));
+            angs(cross(u1.c[1], u0.c[0]), dot(u0.c[0], u1.c[1]));
+            angs(cross(u1.c[2], u0.c[0]), dot(u0.c[0], u1.c[2]));
             if (J.params[0] != 0.f) {
-                R[k].angular0 = st4(u0.c[0], R[k].angular0.w);
-                R[k].angular1 = st4(u0.c[0], -J.params[2]);
-                R[k].linear.w = J.params[1];
-                R[k].linear0t.w = J.params[2];
+                float4* const r = row();
+                r[32 * ROW_ANGULAR0] = st4(u0.c[0], 0.f);
+                r[32 * ROW_ANGULAR1] = st4(u0.c[0], -J.params[2]);
+                r[32 * ROW_LINEAR].w = J.params[1];
+                r[32 * ROW_MISC].x = J.params[2];
                 ++k;
             }
             break;
         case 6: {
             p2p();
-            ang(cross(u1.c[1], u0.c[0]), dot(u0.c[0], u1.c[1]));
-            ang(cross(u1.c[2], u0.c[0]), dot(u0.c[0], u1.c[2]));
+            angs(cross(u1.c[1], u0.c[0]), dot(u0.c[0], u1.c[1]));
+            angs(cross(u1.c[2], u0.c[0]), dot(u0.c[0], u1.c[2]));
             float a = libm::acosf(clampG(dot(u0.c[2], u1.c[2]), -1.f, 1.f));   // glm::orientedAngle
             if (dot(u0.c[0], cross(u0.c[2], u1.c[2])) < 0.f) a = -a;
-            R[k].angular0 = st4(u0.c[0], a - J.params[0]);
-            R[k].angular1 = st4(u0.c[0], R[k].angular1.w);
-            R[k].linear1t.w = J.params[1];
-            R[k].angular0t.w = J.params[2];
-            ++k;
+            row()[32 * ROW_MISC].y = J.params[1];
+            row()[32 * ROW_MISC].z = J.params[2];
+            angs(u0.c[0], a - J.params[0]);
             break;
         }
         case 3: {
             V3 d = p1 - p0;
             lin(u0.c[1], cross(r0, u0.c[1]), cross(r1, u0.c[1]), dot(d, u0.c[1]));
             lin(u0.c[2], cross(r0, u0.c[2]), cross(r1, u0.c[2]), dot(d, u0.c[2]));
-            ang(cross(u1.c[1], u0.c[0]), dot(u0.c[0], u1.c[1]));
-            ang(cross(u1.c[2], u0.c[0]), dot(u0.c[0], u1.c[2]));
-            ang(cross(u1.c[2], u0.c[1]), dot(u0.c[1], u1.c[2]));
+            angs(cross(u1.c[1], u0.c[0]), dot(u0.c[0], u1.c[1]));
+            angs(cross(u1.c[2], u0.c[0]), dot(u0.c[0], u1.c[2]));
+            angs(cross(u1.c[2], u0.c[1]), dot(u0.c[1], u1.c[2]));
             float dx = dot(d, u0.c[0]);
             V3 r0xx = cross(r0, u0.c[0]), r1xx = cross(r1, u0.c[0]);
             if (J.makeUpper) {
-                R[k].angular1.w = 0.f;  // min = 0
-                lin(u0.c[0], r0xx, r1xx, dx - J.params[0]);
+                lin(u0.c[0], r0xx, r1xx, dx - J.params[0], 0.f);   // min = 0
             } else if (J.makeLower) {
-                R[k].linear0t.w = 0.f;  // max = 0
+                row()[32 * ROW_MISC].x = 0.f;  // max = 0
                 lin(u0.c[0], r0xx, r1xx, dx - J.params[1]);
             }
             if (J.params[2] != 0.f) {
-                R[k].linear1t.w = J.params[4];
-                R[k].angular0t.w = J.params[5];
+                row()[32 * ROW_MISC].y = J.params[4];
+                row()[32 * ROW_MISC].z = J.params[5];
                 lin(u0.c[0], r0xx, r1xx, dx - J.params[3]);
             }
             break;
@@ -312,9 +321,7 @@ __device__ void make_joint_rows(const World& w, int j) {
             J.virtual1 += angleDiffD(a1, J.persistent1);
             J.persistent0 = a0; J.persistent1 = a1;
             float ratio = J.params[0];
-            R[k].angular0 = st4(u0.c[0] * ratio, J.virtual0 * ratio - J.virtual1);
-            R[k].angular1 = st4(-u1.c[0], R[k].angular1.w);
-            ++k;
+            ang(u0.c[0] * ratio, -u1.c[0], J.virtual0 * ratio - J.virtual1);
             break;
         }
     }
@@ -323,34 +330,28 @@ __device__ void make_joint_rows(const World& w, int j) {
 // Constraint1D(W)::preSolve (Constraint1D.cpp:5-52 / Constraint1DW.cpp:5-115) of a joint's
 // rows in solve order.  Every row of a joint has its two bodies, whose inertia is read once
 // and whose pseudo velocities (with the count of rows applied) stay in registers.
-__device__ __forceinline__ void joint_rows_presolve(const World& w, int j, float4& pv0, float4& pw0, float4& pv1, float4& pw1) {
-    const JointDev& J = w.joints[j];
-    Row* const R = w.rows + (size_t)j * kMaxRowsPerJoint;
-    const int b0 = J.b0, b1 = J.b1, n = J.norder;
-    const bool simd = J.simd != 0, same = b0 >= 0 && b0 == b1;
-    float im0 = 0, im1 = 0;
+__device__ __forceinline__ void joint_rows_presolve(const World& w, int q, float4& pv0, float4& pw0, float4& pv1, float4& pw1) {
+    const JointRun J = w.jruns[q];
+    float4* R = joint_rows(w, q);
+    const int b0 = J.b0, b1 = J.b1, n = J.rows & 0xff;
+    const bool simd = (J.rows >> 8) != 0, same = b0 >= 0 && b0 == b1;
+    const float im0 = J.im0, im1 = J.im1;
     M3 I0 = m3zero(), I1 = m3zero();
-    if (b0 >= 0) { im0 = w.com[b0].w; I0 = m3cols(ld3(w.mt[3 * b0]), ld3(w.mt[3 * b0 + 1]), ld3(w.mt[3 * b0 + 2])); }
-    if (b1 >= 0) { im1 = w.com[b1].w; I1 = m3cols(ld3(w.mt[3 * b1]), ld3(w.mt[3 * b1 + 1]), ld3(w.mt[3 * b1 + 2])); }
-    unsigned order = J.order;
-    for (int i = 0; i < n; ++i, order >>= 4) {
-        Row& r = R[order & 15u];
-        const int fl = r.flags;
+    if (b0 >= 0) I0 = m3cols(ld3(w.mt[3 * b0]), ld3(w.mt[3 * b0 + 1]), ld3(w.mt[3 * b0 + 2]));
+    if (b1 >= 0) I1 = m3cols(ld3(w.mt[3 * b1]), ld3(w.mt[3 * b1 + 1]), ld3(w.mt[3 * b1 + 2]));
+    for (int i = 0; i < n; ++i, R += kRowStep) {
+        const float4 rl = R[32 * ROW_LINEAR], r0 = R[32 * ROW_ANGULAR0], r1 = R[32 * ROW_ANGULAR1];
+        const float fw = R[32 * ROW_ANGULAR0T].w, mx = R[32 * ROW_MISC].x;
+        const int fl = __float_as_int(fw);
         const bool angf = fl & 2, soft = fl & 1, lim = fl & 4;
-        const V3 a0 = ld3(r.angular0), a1 = ld3(r.angular1), l = ld3(r.linear);
+        const V3 a0 = ld3(r0), a1 = ld3(r1), l = ld3(rl);
         const V3 a0t = mv(I0, a0), a1t = mv(I1, a1);
         float inv = dot(a0, a0t) + dot(a1, a1t);
-        V3 l0t = ld3(r.linear0t), l1t = ld3(r.linear1t);
-        if (!angf) {
-            inv += dot(l, l) * (im0 + im1);
-            l0t = im0 * l;
-            l1t = im1 * l;
-        }
-        const float c = r.angular0.w, mn = r.angular1.w, mx = r.linear0t.w;
-        r.angular0t = st4(a0t, r.angular0t.w);
-        r.angular1t = st4(a1t, inv);
-        r.linear0t = st4(l0t, mx);
-        r.linear1t = st4(l1t, r.linear1t.w);
+        if (!angf) inv += dot(l, l) * (im0 + im1);
+        const V3 l0t = im0 * l, l1t = im1 * l;
+        const float c = r0.w, mn = r1.w;
+        R[32 * ROW_ANGULAR0T] = st4(a0t, fw);
+        R[32 * ROW_ANGULAR1T] = st4(a1t, inv);
         if (soft || !(inv != 0.f && c != 0.f)) continue;
         float lambda = c / inv;
         if (lim) {
@@ -370,12 +371,12 @@ __device__ __forceinline__ void joint_rows_presolve(const World& w, int j, float
     }
 }
 
-__device__ void joint_presolve(const World& w, int j) {
-    const int b0 = w.joints[j].b0, b1 = w.joints[j].b1;
+__device__ void joint_presolve(const World& w, int q) {
+    const int b0 = w.jruns[q].b0, b1 = w.jruns[q].b1;
     float4 pv0 = make_float4(0, 0, 0, 0), pw0 = pv0, pv1 = pv0, pw1 = pv0;
     if (b0 >= 0) { pv0 = w.pv_v[b0]; pw0 = w.pv_w[b0]; }
     if (b1 >= 0) { pv1 = w.pv_v[b1]; pw1 = w.pv_w[b1]; }
-    joint_rows_presolve(w, j, pv0, pw0, pv1, pw1);
+    joint_rows_presolve(w, q, pv0, pw0, pv1, pw1);
     if (b0 >= 0) { w.pv_v[b0] = pv0; w.pv_w[b0] = pw0; }
     if (b1 >= 0) { w.pv_v[b1] = pv1; w.pv_w[b1] = pw1; }
 }
@@ -425,16 +426,18 @@ struct GlobVel {
 };
 // Constraint1D(W)::solve for one row (Constraint1D.cpp:54-127 / Constraint1DW.cpp:117-233).
 // V0, W0, V1, W1: the velocities of the joint's bodies (zero, and left so, for a side that
-// is not simulated: s0, s1; `same`: both sides are one body).  total: the row's accumulated
+// is not simulated; both sides may be one body).  total: the row's accumulated
 // impulse.  bias: 0.2 / h, formed once per substep (the device divides f64 slowly).
-__device__ __forceinline__ void row_solve(const Row& r, float& total, float h, float bias, bool warm, bool simd, bool s0,
-                                          bool s1, bool same, V3& V0, V3& W0, V3& V1, V3& W1) {
-    const int fl = r.flags;
+struct RowVals { float4 linear, angular0, angular1, angular0t, angular1t, misc; };
+__device__ __forceinline__ void row_solve(const RowVals& r, float& total, float h, float bias, bool warm, const JointRun& J,
+                                          V3& V0, V3& W0, V3& V1, V3& W1) {
+    const bool simd = (J.rows >> 8) != 0, s0 = J.b0 >= 0, s1 = J.b1 >= 0, same = s0 && J.b0 == J.b1;
+    const int fl = __float_as_int(r.angular0t.w);
     const bool angf = fl & 2, soft = fl & 1, lim = fl & 4;
     const float inv = r.angular1t.w;
     if (!simd && !inv) return;
     V3 v0 = V0, w0 = W0, v1 = V1, w1 = W1;
-    const V3 l0t = ld3(r.linear0t), l1t = ld3(r.linear1t), a0t = ld3(r.angular0t), a1t = ld3(r.angular1t);
+    const V3 l = ld3(r.linear), l0t = J.im0 * l, l1t = J.im1 * l, a0t = ld3(r.angular0t), a1t = ld3(r.angular1t);
     const float c = r.angular0.w;
     if (!soft && warm) {
         const bool apply = simd ? (fabsf(c) < (float)1e-4 && fabsf(total) < 10000.f)
@@ -448,10 +451,10 @@ __device__ __forceinline__ void row_solve(const Row& r, float& total, float h, f
         }
     }
     if (simd && !inv) return;
-    const V3 a0 = ld3(r.angular0), a1 = ld3(r.angular1), l = ld3(r.linear);
+    const V3 a0 = ld3(r.angular0), a1 = ld3(r.angular1);
     float rv = dot(a1, w1) - dot(a0, w0);
     if (!angf) rv += dot(l, v1) - dot(l, v0);
-    const float tvel = r.linear.w, mn = r.angular1.w, mx = r.linear0t.w, freq = r.linear1t.w, damp = r.angular0t.w;
+    const float tvel = r.linear.w, mn = r.angular1.w, mx = r.misc.x, freq = r.misc.y, damp = r.misc.z;
     float lambda;
     if (simd) {
         const float eff = 1.f / inv;
@@ -510,35 +513,34 @@ __device__ __forceinline__ void row_solve(const Row& r, float& total, float h, f
 // A joint's rows in solve order, on its bodies' velocities in registers; the next row's
 // record is read while one is solved (a row is a chain of about twenty dependent
 // operations, its record comes from L2).
-__device__ __forceinline__ void joint_rows_solve(const World& w, int j, float h, float bias, bool warm, V3& v0, V3& w0,
-                                                 V3& v1, V3& w1) {
-    const JointDev& J = w.joints[j];
-    Row* const R = w.rows + (size_t)j * kMaxRowsPerJoint;
-    const int b0 = J.b0, b1 = J.b1, n = J.norder;
-    const bool simd = J.simd != 0, same = b0 >= 0 && b0 == b1;
-    unsigned order = J.order;
+__device__ __forceinline__ void joint_rows_solve(const World& w, int q, const JointRun& J, float h, float bias, bool warm,
+                                                 V3& v0, V3& w0, V3& v1, V3& w1) {
+    float4* R = joint_rows(w, q);
+    const int n = J.rows & 0xff;
+    auto read = [](const float4* r) {
+        return RowVals{r[32 * ROW_LINEAR], r[32 * ROW_ANGULAR0], r[32 * ROW_ANGULAR1], r[32 * ROW_ANGULAR0T],
+                       r[32 * ROW_ANGULAR1T], r[32 * ROW_MISC]};
+    };
     if (!n) return;
-    Row next = R[order & 15u];
-    for (int i = 0; i < n; ++i) {
-        const Row r = next;
-        Row* const at = R + (order & 15u);
-        order >>= 4;
-        if (i + 1 < n) next = R[order & 15u];
-        float total = r.totalLambda;
-        row_solve(r, total, h, bias, warm, simd, b0 >= 0, b1 >= 0, same, v0, w0, v1, w1);
-        at->totalLambda = total;
+    RowVals next = read(R);
+    for (int i = 0; i < n; ++i, R += kRowStep) {
+        const RowVals r = next;
+        if (i + 1 < n) next = read(R + kRowStep);
+        float total = r.misc.w;
+        row_solve(r, total, h, bias, warm, J, v0, w0, v1, w1);
+        R[32 * ROW_MISC].w = total;
     }
 }
 
 template <class V>
-__device__ void joint_solve(const World& w, int j, float h, float bias, bool warm, int ds, const V vr) {
-    const int b0 = w.joints[j].b0, b1 = w.joints[j].b1;
+__device__ void joint_solve(const World& w, int q, float h, float bias, bool warm, int ds, const V vr) {
+    const JointRun J = w.jruns[q];
     V3 v0 = {0, 0, 0}, w0 = {0, 0, 0}, v1 = {0, 0, 0}, w1 = {0, 0, 0};
-    if (b0 >= 0) vr.ld(b0 - ds, v0, w0);
-    if (b1 >= 0) vr.ld(b1 - ds, v1, w1);
-    joint_rows_solve(w, j, h, bias, warm, v0, w0, v1, w1);
-    if (b0 >= 0) vr.st(b0 - ds, v0, w0);
-    if (b1 >= 0) vr.st(b1 - ds, v1, w1);
+    if (J.b0 >= 0) vr.ld(J.b0 - ds, v0, w0);
+    if (J.b1 >= 0) vr.ld(J.b1 - ds, v1, w1);
+    joint_rows_solve(w, q, J, h, bias, warm, v0, w0, v1, w1);
+    if (J.b0 >= 0) vr.st(J.b0 - ds, v0, w0);
+    if (J.b1 >= 0) vr.st(J.b1 - ds, v1, w1);
 }
 
 // ---------------------------------------------------------------- contacts (ContactConstraints.cpp)
@@ -1034,10 +1036,10 @@ __device__ void solve_substeps(const World& w, FrameBuf& f, int s, const S& sy, 
     for (int k = tid; k < ncl; k += nth) contact_header(w, f.contacts[f.corder[ms + k]], ds, f.pt_off[ms + k], HK(k));
     sy.sync();
     const int js0 = w.scene_jsteps[s], js1 = w.scene_jsteps[s + 1];
-    const int jb = w.scene_joint[s], je = w.scene_joint[s + 1];
+    const int jb = w.scene_joint[s], je = w.scene_joint[s + 1];   // schedule entries: every joint of the scene once
     const float joint_bias = jb < je ? (float)(0.2 / (double)h) : 0.f;
     for (int sub = 0; sub < substeps; ++sub) {
-        for (int j = jb + tid; j < je; j += nth) make_joint_rows(w, j);
+        for (int q = jb + tid; q < je; q += nth) make_joint_rows(w, q);
         for (int d = ds + tid; d < de; d += nth) integrate_velocity<false>(w, d, ds, h, g, vr);
         sy.sync();
         for (int k = tid; k < ncl; k += nth) {
@@ -1045,7 +1047,7 @@ __device__ void solve_substeps(const World& w, FrameBuf& f, int s, const S& sy, 
             contact_rows(w, f.contacts[f.corder[ms + k]], H, PK(k) + H.i.w, h, sub == substeps - 1, vr);
         }
         for (int st = js0; st < js1; ++st) {
-            for (int k = w.jstep_start[st] + tid; k < w.jstep_start[st + 1]; k += nth) joint_presolve(w, w.jsched[k]);
+            for (int k = w.jstep_start[st] + tid; k < w.jstep_start[st + 1]; k += nth) joint_presolve(w, k);
             sy.sync();
         }
         sy.sync();
@@ -1072,7 +1074,7 @@ __device__ void solve_substeps(const World& w, FrameBuf& f, int s, const S& sy, 
             if (bias)
                 for (int st = js0; st < js1; ++st) {
                     for (int k = w.jstep_start[st] + tid; k < w.jstep_start[st + 1]; k += nth)
-                        joint_solve(w, w.jsched[k], h, joint_bias, it == 0, ds, vr);
+                        joint_solve(w, k, h, joint_bias, it == 0, ds, vr);
                     sy.sync();
                 }
         }
@@ -1148,9 +1150,8 @@ __device__ void solve_flow(const World& w, FrameBuf& f, int s, const GridSync& s
     const float4 kn = w.knobs[s];
     const int substeps = (int)kn.x, iterations = (int)kn.y;
     const float g = kn.z, h = kn.w / substeps;
-    const int jb = w.scene_joint[s], je = w.scene_joint[s + 1];
-    const int jq0 = w.jstep_start[w.scene_jsteps[s]], jq1 = w.jstep_start[w.scene_jsteps[s + 1]];
-    const float joint_bias = jb < je ? (float)(0.2 / (double)h) : 0.f;
+    const int jq0 = w.scene_joint[s], jq1 = w.scene_joint[s + 1];   // schedule entries: every joint of the scene once
+    const float joint_bias = jq0 < jq1 ? (float)(0.2 / (double)h) : 0.f;
     SHdr* const Hg = f.s_hdr + ms;
     SPt* const Pg = f.s_pts + 4 * (size_t)ms;
     float4* const vt = w.vt + 2 * (size_t)ds;
@@ -1179,7 +1180,7 @@ __device__ void solve_flow(const World& w, FrameBuf& f, int s, const GridSync& s
     }
     const long long limit = max(1ll, sy.bar.limit >> 3);   // a poll here takes some eight of the barrier's
     for (int sub = 0; sub < substeps; ++sub) {
-        for (int j = jb + slot; j < je; j += nth) make_joint_rows(w, j);
+        for (int q = jq0 + slot; q < jq1; q += nth) make_joint_rows(w, q);
         for (int d = slot; d < nd; d += nth) integrate_velocity<true>(w, ds + d, ds, h, g, GlobVel{vt});
         sy.sync();
         for (int k = slot; k < ncl; k += nth)
@@ -1218,7 +1219,7 @@ __device__ void solve_flow(const World& w, FrameBuf& f, int s, const GridSync& s
                 e0 = (place.x & 0xff) + it * (place.x >> 8) + relax;
                 e1 = (place.y & 0xff) + it * (place.y >> 8) + relax;
             } else if (kind == FLOW_JOINT) {
-                const JointDev& J = w.joints[w.jsched[idx]];
+                const JointRun J = w.jruns[idx];
                 b0 = J.b0 >= 0 ? J.b0 - ds : -1;
                 b1 = J.b1 >= 0 ? J.b1 - ds : -1;
                 const int d0 = b0 >= 0 && it >= 0 ? f.bdeg[J.b0] : 0, d1 = b1 >= 0 && it >= 0 ? f.bdeg[J.b1] : 0;
@@ -1269,9 +1270,8 @@ __device__ void solve_flow(const World& w, FrameBuf& f, int s, const GridSync& s
                     const bool bias = it < iterations;
                     if (bias || !(hi.z & 0x100)) contact_forms(Hg[idx], Pg + hi.w, bias, pv);
                 } else if (kind == FLOW_JOINT) {
-                    const int j = w.jsched[idx];
-                    if (it < 0) joint_rows_presolve(w, j, ps0, pw0, ps1, pw1);
-                    else joint_rows_solve(w, j, h, joint_bias, it == 0, pv.v0, pv.w0, pv.v1, pv.w1);
+                    if (it < 0) joint_rows_presolve(w, idx, ps0, pw0, ps1, pw1);
+                    else joint_rows_solve(w, idx, w.jruns[idx], h, joint_bias, it == 0, pv.v0, pv.w0, pv.v1, pv.w1);
                 } else if (kind == FLOW_POS) {
                     integrate_position(w, ds + b0, w.dyn_body[ds + b0], h, pv.v0, pv.w0, ld3(ps0), ld3(pw0), ps0.w);
                 } else {

@@ -76,16 +76,21 @@ struct Contact {         // ContactConstraints (src/ContactConstraints.h:31-48)
     float2 lambda[4];    // accumulated normal and friction impulse of each point after the frame
 };
 
-struct Row {             // Constraint1D / Constraint1DW lane
-    float4 linear;       // w = targetVelocity
-    float4 angular0;     // w = c
-    float4 angular1;     // w = min
-    float4 linear0t;     // w = max
-    float4 linear1t;     // w = frequency
-    float4 angular0t;    // w = dampingRatio
-    float4 angular1t;    // w = invEffMass
-    float totalLambda;
-    int flags, b0, b1;
+// One joint row (Constraint1D / a Constraint1DW lane) is six float4 fields:
+//   ROW_LINEAR {linear, targetVelocity}       ROW_ANGULAR0 {angular0, c}
+//   ROW_ANGULAR1 {angular1, min}              ROW_ANGULAR0T {I0 angular0, flags}
+//   ROW_ANGULAR1T {I1 angular1, invEffMass}   ROW_MISC {max, frequency, dampingRatio, totalLambda}
+// The rows of a joint lie in solve order, and the joints in schedule order, 32 side by side
+// field by field: a warp that solves a step's joints reads 512 bytes in a row for each field.
+enum : int { ROW_LINEAR, ROW_ANGULAR0, ROW_ANGULAR1, ROW_ANGULAR0T, ROW_ANGULAR1T, ROW_MISC, kRowF4 };
+
+// what the solver reads of a joint, in schedule order
+struct JointRun {
+    int b0, b1;          // global dynamic index or -1
+    int rows;            // rows | simd << 8
+    float im0, im1;      // inverse masses, 0 on a side that is not simulated
+    int rank0, rank1;    // joints before this one, in solve order, on its two bodies
+    int pad;
 };
 
 struct JointDev {
@@ -95,10 +100,9 @@ struct JointDev {
     float4 r0, r1;                   // anchor relative to COM when dynamic
     float params[8];
     int makeUpper, makeLower, gearInit;
-    int norder;                      // rows solved each iteration, and their indices in solve order,
-    unsigned order;                  // four bits each, the first lowest
+    unsigned place;                  // each row's place in solve order, four bits each, the first lowest
     int rank0, rank1;                // joints before this one, in solve order, on its two bodies
-    int pad;
+    int pad[2];
     float persistent0, persistent1, virtual0, virtual1;
     int rowflags[kMaxRowsPerJoint];
 };
@@ -196,7 +200,8 @@ struct World {
     unsigned long long* trimesh_keys;   // [6][n_trimesh_cols] bounds reduction keys
     // joints
     JointDev* joints;
-    Row* rows;             // kMaxRowsPerJoint per joint
+    float4* rows;          // kMaxRowsPerJoint rows per joint (ROW_*)
+    JointRun* jruns;       // per schedule entry
     int* jsched;           // joint indices in solve order (colour, sub-colour)
     int* jsched_step;      // step id per schedule entry
     int* scene_jsteps;     // [S+1] step boundaries into jstep_start

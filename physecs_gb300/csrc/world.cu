@@ -366,7 +366,8 @@ psx_status psx::rt::build_world(psx_world* W, const psx_scene_desc* scenes, int 
         PSX_TRY(W->upload(w.body_nj, nj));
     }
     PSX_TRY(W->upload(w.joints, joints));
-    PSX_TRY(W->alloc(w.rows, (size_t)kMaxRowsPerJoint * std::max(1, w.n_joints)));
+    PSX_TRY(W->alloc(w.rows, (size_t)kMaxRowsPerJoint * kRowF4 * ((w.n_joints + 31) / 32 * 32)));
+    PSX_TRY(W->alloc(w.jruns, w.n_joints));
     PSX_TRY(W->upload(w.jsched, jsched));
     PSX_TRY(W->upload(w.jstep_start, jstep_start));
     PSX_TRY(W->upload(w.scene_jsteps, scene_jsteps));
