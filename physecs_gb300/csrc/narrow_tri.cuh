@@ -476,6 +476,51 @@ __device__ __forceinline__ bool inSet(const uint32_t* s, int n, uint32_t v) {
     return false;
 }
 
+// one triangle of the midphase against the body, in the mesh's frame
+__device__ __forceinline__ bool triTest(const World& w, const TriView& mesh, int ti, V3 lp, Q4 lo, const GeomD& g0, TCI& ci,
+                                        Polytope& epaPoly, int* err) {
+    const TriDev tri = mesh.tris[ti];
+    V3 a = tv(mesh, tri.idx.x), b = tv(mesh, tri.idx.y), c = tv(mesh, tri.idx.z);
+    ci.boxFeature = BF_FACE; ci.boxAxis = 0; ci.featureIndex = 0; ci.feature = TF_FACE;
+    ci.tri = ti;
+    switch (g0.type) {
+        case G_SPHERE: return sphereTri(lp, g0.p[0], a, b, c, ld3(tri.normal), ci);
+        case G_CAPSULE: return capsuleTri(lp, lo, g0.p[0], g0.p[1], a, b, c, ld3(tri.normal), ci);
+        case G_BOX: return boxTri(lp, lo, gv(g0), a, b, c, ld3(tri.normal), ci);
+        case G_CONVEX: return convexTri(w, lp, lo, g0.mesh, gv(g0), a, b, c, ld3(tri.centroid), ci, epaPoly, err);
+        default: return false;
+    }
+}
+
+// the manifold (at most one) of a candidate by the triangle's feature
+__device__ __forceinline__ void triFaceContact(const World& w, const TriView& mesh, const TCI& c, V3 lp, Q4 lo, const GeomD& g0,
+                                               V3 pos1, Q4 or1, ManOut& out) {
+    switch (g0.type) {
+        case G_SPHERE: sphereTriContacts(pos1, or1, c, out); break;
+        case G_CAPSULE: capsuleTriFace(lp, lo, g0.p[0], g0.p[1], pos1, or1, mesh, c, out); break;
+        case G_BOX: boxTriFace(lp, lo, gv(g0), pos1, or1, mesh, c, out); break;
+        case G_CONVEX: convexTriFace(w, lp, lo, g0.mesh, gv(g0), pos1, or1, mesh, c, out); break;
+    }
+}
+__device__ __forceinline__ void triRimContact(const World& w, const TriView& mesh, const TCI& c, V3 lp, Q4 lo, const GeomD& g0,
+                                              V3 pos1, Q4 or1, ManOut& out) {
+    switch (g0.type) {
+        case G_SPHERE: case G_CAPSULE: sphereTriContacts(pos1, or1, c, out); break;
+        case G_BOX:
+            if (c.feature == TF_VERTEX || c.boxFeature == BF_FACE) boxFaceTri(lp, lo, gv(g0), pos1, or1, mesh, c, out);
+            else boxEdgeTriEdge(lp, lo, gv(g0), pos1, or1, mesh, c, out);
+            break;
+        case G_CONVEX: convexFaceTri(w, lp, lo, g0.mesh, gv(g0), pos1, or1, mesh, c, out); break;
+    }
+}
+
+// an edge or vertex candidate whose vertices an earlier contact covers makes none
+template <class F>
+__device__ __forceinline__ bool triVoided(const TCI& c, const uint32_t* id, F&& covered) {
+    if (c.feature == TF_EDGE) return covered(id[(c.featureIndex + 1) % 3]) && covered(id[(c.featureIndex + 2) % 3]);
+    return c.feature == TF_VERTEX && covered(id[c.featureIndex]);
+}
+
 // collisionTriangleMesh (CollisionTriangleMesh.cpp:882-956): body (g0 at pos0/or0) against mesh at pos1/or1.
 // Writes manifolds in the reference's emission order; returns whether any triangle was hit.
 __device__ inline bool collideTriMesh(const World& w, V3 pos0, Q4 or0, const GeomD& g0, V3 pos1, Q4 or1, int meshId,
@@ -499,20 +544,10 @@ __device__ inline bool collideTriMesh(const World& w, V3 pos0, Q4 or0, const Geo
         if (triCount) {
             for (int i = 0; i < triCount; ++i) {
                 int ti = index + i;
-                const TriDev tri = mesh.tris[ti];
-                V3 a = tv(mesh, tri.idx.x), b = tv(mesh, tri.idx.y), c = tv(mesh, tri.idx.z);
                 TCI ci;
-                ci.boxFeature = BF_FACE; ci.boxAxis = 0; ci.featureIndex = 0; ci.feature = TF_FACE;
-                bool hit = false;
-                switch (g0.type) {
-                    case G_SPHERE: hit = sphereTri(lp, g0.p[0], a, b, c, ld3(tri.normal), ci); break;
-                    case G_CAPSULE: hit = capsuleTri(lp, lo, g0.p[0], g0.p[1], a, b, c, ld3(tri.normal), ci); break;
-                    case G_BOX: hit = boxTri(lp, lo, gv(g0), a, b, c, ld3(tri.normal), ci); break;
-                    case G_CONVEX: hit = convexTri(w, lp, lo, g0.mesh, gv(g0), a, b, c, ld3(tri.centroid), ci, epaPoly, out.err); break;
-                    default: break;
-                }
+                const bool hit = triTest(w, mesh, ti, lp, lo, g0, ci, epaPoly, out.err);
                 if (hit) {
-                    if (nc < kTriCandidates) { ci.tri = ti; contacts[nc++] = ci; }
+                    if (nc < kTriCandidates) contacts[nc++] = ci;
                     else raise_err(out.err, ERR_TRI_CAPACITY);
                 }
             }
@@ -525,19 +560,13 @@ __device__ inline bool collideTriMesh(const World& w, V3 pos0, Q4 or0, const Geo
     if (nc == 0) return false;
     uint32_t voided[3 * kTriCandidates];
     int nvoid = 0;
-    V3 he = gv(g0);
     for (int i = nc - 1; i >= 0; i--) {
         TCI c = contacts[i];
         if (c.feature == TF_FACE) {
             const TriDev tri = mesh.tris[c.tri];
             uint32_t id[3] = {(uint32_t)tri.idx.x, (uint32_t)tri.idx.y, (uint32_t)tri.idx.z};
             for (int k = 0; k < 3; ++k) if (!inSet(voided, nvoid, id[k])) voided[nvoid++] = id[k];
-            switch (g0.type) {
-                case G_SPHERE: sphereTriContacts(pos1, or1, c, out); break;
-                case G_CAPSULE: capsuleTriFace(lp, lo, g0.p[0], g0.p[1], pos1, or1, mesh, c, out); break;
-                case G_BOX: boxTriFace(lp, lo, he, pos1, or1, mesh, c, out); break;
-                case G_CONVEX: convexTriFace(w, lp, lo, g0.mesh, he, pos1, or1, mesh, c, out); break;
-            }
+            triFaceContact(w, mesh, c, lp, lo, g0, pos1, or1, out);
             contacts[i] = contacts[nc - 1];
             contacts[nc - 1] = c;
             --nc;
@@ -554,27 +583,208 @@ __device__ inline bool collideTriMesh(const World& w, V3 pos0, Q4 or0, const Geo
         const TCI c = contacts[i];
         const TriDev tri = mesh.tris[c.tri];
         uint32_t id[3] = {(uint32_t)tri.idx.x, (uint32_t)tri.idx.y, (uint32_t)tri.idx.z};
-        if (c.feature == TF_EDGE) {
-            if (inSet(voided, nvoid, id[(c.featureIndex + 1) % 3]) && inSet(voided, nvoid, id[(c.featureIndex + 2) % 3])) continue;
-            switch (g0.type) {
-                case G_SPHERE: case G_CAPSULE: sphereTriContacts(pos1, or1, c, out); break;
-                case G_BOX:
-                    if (c.boxFeature == BF_FACE) boxFaceTri(lp, lo, he, pos1, or1, mesh, c, out);
-                    else boxEdgeTriEdge(lp, lo, he, pos1, or1, mesh, c, out);
-                    break;
-                case G_CONVEX: convexFaceTri(w, lp, lo, g0.mesh, he, pos1, or1, mesh, c, out); break;
-            }
-        } else if (c.feature == TF_VERTEX) {
-            if (inSet(voided, nvoid, id[c.featureIndex])) continue;
-            switch (g0.type) {
-                case G_SPHERE: case G_CAPSULE: sphereTriContacts(pos1, or1, c, out); break;
-                case G_BOX: boxFaceTri(lp, lo, he, pos1, or1, mesh, c, out); break;
-                case G_CONVEX: convexFaceTri(w, lp, lo, g0.mesh, he, pos1, or1, mesh, c, out); break;
-            }
-        }
+        if (triVoided(c, id, [&](uint32_t v) { return inSet(voided, nvoid, v); })) continue;
+        if (c.feature == TF_EDGE || c.feature == TF_VERTEX) triRimContact(w, mesh, c, lp, lo, g0, pos1, or1, out);
         for (int k = 0; k < 3; ++k) if (!inSet(voided, nvoid, id[k])) voided[nvoid++] = id[k];
     }
     return true;
+}
+
+// ---------------------------------------------------------------- a warp per pair
+
+// What a warp keeps in shared memory: the midphase lists of the pairs it walks together,
+// and one pair's candidates.
+constexpr int kTriGroup = 8;      // pairs whose midphase a warp walks together, a lane each
+constexpr int kTriKept = 48;      // triangles a lane keeps; a pair with more is walked again by the whole warp
+struct TriWarpMem {
+    int kept[kTriGroup][kTriKept];
+    TCI cand[kTriCandidates];
+    uint32_t voided[3 * kTriCandidates];
+    int pending[64];
+    unsigned char order[kTriCandidates], surv[kTriCandidates];
+};
+
+// the body of a pair in its mesh's frame
+struct TriPair {
+    V3 pos1, lp;
+    Q4 or1, lo;
+    GeomD g0;
+    TriView mesh;
+    Bounds lb;
+    bool flip;     // the mesh is the pair's first collider
+};
+__device__ inline TriPair triPair(const World& w, int2 pr) {
+    TriPair t;
+    V3 pos0, pos1;
+    Q4 or0, or1;
+    GeomD g0, g1;
+    collider_pose(w, pr.x, pos0, or0, g0);
+    collider_pose(w, pr.y, pos1, or1, g1);
+    t.flip = g0.type == G_TRIMESH;
+    if (t.flip) {
+        V3 p = pos0; pos0 = pos1; pos1 = p;
+        Q4 q = or0; or0 = or1; or1 = q;
+        GeomD g = g0; g0 = g1; g1 = g;
+    }
+    const TriMeshDev tm = w.trimesh[g1.mesh];
+    t.mesh = TriView{w.tri_verts + tm.vert_start, w.tris + tm.tri_start, w.tri_nodes + tm.node_start};
+    const Q4 inv1 = qinverse(or1);
+    t.pos1 = pos1;
+    t.or1 = or1;
+    t.lp = qrot(inv1, pos0 - pos1);
+    t.lo = qmul(inv1, or0);
+    t.g0 = g0;
+    t.lb = getBounds(w, t.lp, t.lo, g0);
+    return t;
+}
+
+// The midphase of collideTriMesh: leaf(first triangle, triangles) for the leaves the body's
+// bounds meet, in its depth-first order.
+template <class F>
+__device__ __forceinline__ void triWalk(const TriPair& t, int* err, F&& leaf) {
+    int stack[64];
+    int sp = 0;
+    stack[sp++] = 0;
+    while (sp) {
+        const TriNodeDev node = t.mesh.nodes[stack[--sp]];
+        if (!intersectsB(t.lb, ld3(node.bmin), ld3(node.bmax))) continue;
+        const int triCount = __float_as_int(node.bmin.w), index = __float_as_int(node.bmax.w);
+        if (triCount) {
+            leaf(index, triCount);
+        } else {
+            if (sp + 2 > 64) { raise_err(err, ERR_STACK_CAPACITY); break; }
+            stack[sp++] = index + 1;
+            stack[sp++] = index;
+        }
+    }
+}
+
+// collideTriMesh by a whole warp, with the same candidates, manifolds and order: a lane tests
+// one triangle of the midphase at a time, then builds the manifold of one contact at a time;
+// which contacts there are (the vertices earlier ones cover) is decided by the vertex indices
+// alone, before the manifolds.  kept, n: the midphase's triangles, or n < 0 to walk for them.
+// store(manifold, k): the k-th manifold that has points.  Returns their number.
+template <class F>
+__device__ int collideTriMeshWarp(const World& w, const TriPair& t, const int* kept, int n, TriWarpMem& sm, Polytope& poly,
+                                  int* err, F&& store) {
+    const int lane = threadIdx.x & 31;
+    const unsigned below = (1u << lane) - 1u;
+    int nc = 0;
+    auto test = [&](const int* list, int m) {   // m <= 32 triangles
+        TCI ci;
+        const bool hit = lane < m && triTest(w, t.mesh, list[lane], t.lp, t.lo, t.g0, ci, poly, err);
+        const unsigned hits = __ballot_sync(~0u, hit);
+        const int at = nc + __popc(hits & below);
+        if (hit) {
+            if (at < kTriCandidates) sm.cand[at] = ci;
+            else raise_err(err, ERR_TRI_CAPACITY);
+        }
+        nc = min(kTriCandidates, nc + __popc(hits));
+        __syncwarp();
+    };
+    if (n >= 0) {
+        for (int i = 0; i < n; i += 32) test(kept + i, min(32, n - i));
+    } else {
+        int np = 0;
+        triWalk(t, err, [&](int first, int count) {
+            for (int i = 0; i < count; i += 32) {
+                const int m = min(32, count - i);
+                if (lane < m) sm.pending[np + lane] = first + i + lane;
+                np += m;
+                __syncwarp();
+                if (np >= 32) {
+                    test(sm.pending, 32);
+                    const int rest = np - 32, v = lane < rest ? sm.pending[32 + lane] : 0;
+                    __syncwarp();
+                    if (lane < rest) sm.pending[lane] = v;
+                    np = rest;
+                    __syncwarp();
+                }
+            }
+        });
+        test(sm.pending, np);
+    }
+    if (nc == 0) return 0;
+    int pushed = 0, stored = 0;
+    auto emit = [&](bool mine, const TCI& c, bool face) {   // the lanes' manifolds, in lane order
+        ManifoldL m;
+        ManOut out{&m, 0, 1, err};
+        if (mine) {
+            if (face) triFaceContact(w, t.mesh, c, t.lp, t.lo, t.g0, t.pos1, t.or1, out);
+            else triRimContact(w, t.mesh, c, t.lp, t.lo, t.g0, t.pos1, t.or1, out);
+        }
+        const unsigned made = __ballot_sync(~0u, out.n != 0);
+        const bool fits = out.n && pushed + __popc(made & below) < kTriManifolds;
+        const bool keep = fits && m.numPoints;
+        const unsigned kept_lanes = __ballot_sync(~0u, keep);
+        if (out.n && !fits) raise_err(err, ERR_TRI_CAPACITY);
+        if (keep) {
+            if (t.flip) flipM(m);
+            store(m, stored + __popc(kept_lanes & below));
+        }
+        pushed += __popc(made);
+        stored += __popc(kept_lanes);
+    };
+    // face contacts, the last candidate first; their triangles' vertices are covered
+    int nf = 0, nvoid = 0;
+    for (int top = nc; top > 0; top -= 32) {
+        const int i = top - 1 - lane;
+        const bool face = i >= 0 && sm.cand[max(i, 0)].feature == TF_FACE;
+        const unsigned faces = __ballot_sync(~0u, face);
+        if (face) {
+            const int4 id = t.mesh.tris[sm.cand[i].tri].idx;
+            uint32_t* v = sm.voided + nvoid + 3 * __popc(faces & below);
+            v[0] = id.x; v[1] = id.y; v[2] = id.z;
+        }
+        emit(face, sm.cand[max(i, 0)], true);
+        nf += __popc(faces);
+        nvoid += 3 * __popc(faces);
+    }
+    __syncwarp();
+    const int rest = nc - nf;
+    if (rest == 0) return stored;
+    if (lane == 0) {
+        // the others in the order that taking the faces out by swaps leaves, then sorted by distance, stably
+        for (int i = 0; i < nc; ++i) sm.order[i] = (unsigned char)i;
+        int left = nc;
+        for (int i = nc - 1; i >= 0; --i) {
+            const unsigned char c = sm.order[i];
+            if (sm.cand[c].feature != TF_FACE) continue;
+            sm.order[i] = sm.order[left - 1];
+            sm.order[left - 1] = c;
+            --left;
+        }
+        for (int i = 1; i < left; ++i) {
+            const unsigned char v = sm.order[i];
+            const float d = sm.cand[v].distance;
+            int j = i;
+            while (j > 0 && d < sm.cand[sm.order[j - 1]].distance) { sm.order[j] = sm.order[j - 1]; --j; }
+            sm.order[j] = v;
+        }
+    }
+    __syncwarp();
+    int ns = 0;
+    for (int i = 0; i < rest; ++i) {
+        const int ci = sm.order[i];
+        const int4 id4 = t.mesh.tris[sm.cand[ci].tri].idx;
+        const uint32_t id[3] = {(uint32_t)id4.x, (uint32_t)id4.y, (uint32_t)id4.z};
+        auto covered = [&](uint32_t v) {
+            bool in = false;
+            for (int k = lane; k < nvoid; k += 32) in |= sm.voided[k] == v;
+            return __any_sync(~0u, in) != 0;
+        };
+        if (triVoided(sm.cand[ci], id, covered)) continue;
+        if (lane < 3) sm.voided[nvoid + lane] = id[lane];
+        nvoid += 3;
+        if (lane == 0) sm.surv[ns] = (unsigned char)ci;
+        ++ns;
+        __syncwarp();
+    }
+    for (int i = 0; i < ns; i += 32) {
+        const TCI& c = sm.cand[sm.surv[min(i + lane, ns - 1)]];
+        emit(i + lane < ns && (c.feature == TF_EDGE || c.feature == TF_VERTEX), c, false);
+    }
+    return stored;
 }
 
 }  // namespace psx

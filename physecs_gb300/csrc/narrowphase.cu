@@ -416,35 +416,49 @@ __global__ void __launch_bounds__(256) k_convex_contacts(World w, FrameBuf f) {
     }
 }
 
-// triangle-mesh pairs (src/Collision.cpp:897-907): the mesh may be either collider
-__global__ void __launch_bounds__(64) k_narrow_tri(World w, FrameBuf f) {
-    int n = f.cat_count[2];
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
-        int p = f.cat_list[2 * f.pair_cap + t];
-        if (t >= f.tri_cap) { atomicOr(w.err, ERR_TRI_CAPACITY); f.pair_nman[p] = 0; continue; }
-        f.pair_tslot[p] = t;
-        int2 pr = f.pairs[p];
-        V3 pos0, pos1;
-        Q4 or0, or1;
-        GeomD g0, g1;
-        collider_pose(w, pr.x, pos0, or0, g0);
-        collider_pose(w, pr.y, pos1, or1, g1);
-        ManifoldL ms[kTriManifolds];
-        TCI cand[kTriCandidates];
-        Polytope poly;
-        ManOut out{ms, 0, kTriManifolds, w.err};
-        bool flip = g0.type == G_TRIMESH;
-        if (flip) collideTriMesh(w, pos1, or1, g1, pos0, or0, g0.mesh, out, cand, poly);
-        else collideTriMesh(w, pos0, or0, g0, pos1, or1, g1.mesh, out, cand, poly);
-        int cnt = 0;
-        for (int k = 0; k < out.n; ++k) {
-            ManifoldL& m = ms[k];
-            if (flip) flipM(m);
-            if (!m.numPoints) continue;
-            store_manifold(f.man_tri[t * kTriManifolds + cnt], m, p);
-            ++cnt;
+// Triangle-mesh pairs (src/Collision.cpp:897-907): the mesh may be either collider.  A body's
+// work against a mesh is a chain of dependent tests and clips, most bodies near a mesh touch
+// none of it and some a dozen triangles, so a thread per pair left a warp with its slowest
+// lane.  Here a warp walks the midphase of kTriGroup pairs together, a lane each (a lane's
+// walk is bound by the latency of its nodes), then takes the pairs that met triangles one
+// by one, a lane per triangle and then a lane per contact.
+constexpr int kTriWarps = 2;
+__global__ void __launch_bounds__(32 * kTriWarps) k_narrow_tri(World w, FrameBuf f) {
+    __shared__ TriWarpMem mem[kTriWarps];
+    TriWarpMem& sm = mem[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31;
+    const int n = f.cat_count[2];
+    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, warps = (gridDim.x * blockDim.x) >> 5;
+    Polytope poly;
+    for (int base = warp * kTriGroup; base < n; base += warps * kTriGroup) {
+        const int t = base + lane;
+        int met = 0;
+        if (lane < kTriGroup && t < n) {
+            const int p = f.cat_list[2 * f.pair_cap + t];
+            if (t >= f.tri_cap) {
+                atomicOr(w.err, ERR_TRI_CAPACITY);
+            } else {
+                f.pair_tslot[p] = t;
+                const TriPair tp = triPair(w, f.pairs[p]);
+                triWalk(tp, w.err, [&](int first, int count) {
+                    for (int i = 0; i < count; ++i, ++met)
+                        if (met < kTriKept) sm.kept[lane][met] = first + i;
+                });
+            }
+            if (!met) f.pair_nman[p] = 0;
         }
-        f.pair_nman[p] = cnt;
+        unsigned todo = __ballot_sync(~0u, met > 0);
+        __syncwarp();
+        while (todo) {
+            const int l = __ffs(todo) - 1;
+            todo &= todo - 1;
+            const int tt = base + l, p = f.cat_list[2 * f.pair_cap + tt], m = __shfl_sync(~0u, met, l);
+            const TriPair tp = triPair(w, f.pairs[p]);
+            const int cnt = collideTriMeshWarp(w, tp, sm.kept[l], m <= kTriKept ? m : -1, sm, poly, w.err,
+                                               [&](const ManifoldL& r, int k) { store_manifold(f.man_tri[tt * kTriManifolds + k], r, p); });
+            if (lane == 0) f.pair_nman[p] = cnt;
+            __syncwarp();
+        }
     }
 }
 
@@ -511,7 +525,7 @@ int launch_narrowphase(const World& w, FrameBuf& f, const StreamPair& sp, const 
     k_narrow_analytic<2><<<152 * ns.analytic_blocks_per_sm, ns.analytic_threads, 0, s>>>(w, f);
     k_narrow_analytic<1><<<152 * ns.analytic_blocks_per_sm, ns.analytic_threads, 0, s>>>(w, f);
     k_narrow_analytic<0><<<152 * ns.analytic_blocks_per_sm, ns.analytic_threads, 0, s>>>(w, f);
-    k_narrow_tri<<<1216, 64, 0, s>>>(w, f);
+    k_narrow_tri<<<152 * 16, 32 * kTriWarps, 0, s>>>(w, f);
     const int kt = launch_triggers(w, f, s);
     cudaStreamWaitEvent(s, sp.join, 0);
     scan_exclusive_dev(f.pair_nman, f.pair_moff, f.n_pairs, f.pair_cap, f.n_man, f.scan_scratch, s);
