@@ -96,17 +96,21 @@ void scan_exclusive_dev(const int* in, int* out, const int* n_dev, int n_max, in
 
 // ---------------------------------------------------------------- radix sort
 //
-// One 8-bit digit per pass.  A tile of kTile keys is split into 8 contiguous
+// One 8-bit digit per pass.  A tile of keys is split into 8 contiguous
 // warp chunks; per-warp digit counters make the ranking stable: a key's rank is
 // (keys of the same digit in earlier tiles) + (in earlier warps of this tile) +
 // (earlier in this warp's chunk), the last counted 32 keys at a time with
 // __match_any_sync.
 namespace {
-constexpr int kTile = 4096;
 constexpr int kRadixThreads = 256;
 constexpr int kWarps = kRadixThreads / 32;
-constexpr int kPerWarp = kTile / kWarps;  // 512 keys per warp
+// A warp ranks its chunk 32 keys at a time, one round after another, so the tile sets the
+// chain's length.  4096 keys a tile leave 65,537 keys to 17 blocks (25.6 us a scatter); up
+// to 2^18 keys, 1024 a tile fill the chip's SMs (65 blocks).  Above, larger tiles keep
+// the histogram small.
+int radix_tile(int n) { return n <= (1 << 18) ? 1024 : 4096; }
 
+template <int kTile>
 __global__ void k_radix_hist(const uint32_t* keys, int n, int shift, int* hist, int ntiles) {
     __shared__ int h[256];
     for (int i = threadIdx.x; i < 256; i += blockDim.x) h[i] = 0;
@@ -120,8 +124,10 @@ __global__ void k_radix_hist(const uint32_t* keys, int n, int shift, int* hist, 
     for (int d = threadIdx.x; d < 256; d += blockDim.x) hist[d * ntiles + blockIdx.x] = h[d];
 }
 
+template <int kTile>
 __global__ void k_radix_scatter(const uint32_t* keys, const int* vals, uint32_t* ok, int* ov, int n, int shift,
                                 const int* offs, int ntiles) {
+    constexpr int kPerWarp = kTile / kWarps;
     __shared__ int wc[kWarps][256];   // per-warp running counters, then per-warp base offsets
     int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (int i = lane; i < 256; i += 32) wc[wid][i] = 0;
@@ -165,7 +171,7 @@ __global__ void k_radix_scatter(const uint32_t* keys, const int* vals, uint32_t*
 }  // namespace
 
 size_t radix_hist_ints(int n) {
-    int ntiles = (n + kTile - 1) / kTile;
+    int ntiles = (n + radix_tile(n) - 1) / radix_tile(n);
     if (ntiles == 0) ntiles = 1;
     size_t h = (size_t)256 * ntiles;
     return 2 * h + scan_scratch_ints((int)h) + 1;
@@ -173,7 +179,7 @@ size_t radix_hist_ints(int n) {
 
 int radix_sort_pairs(uint32_t* keys, int* vals, uint32_t* tmpk, int* tmpv, int n, int bits, int* hist, cudaStream_t s) {
     if (n <= 0) return 0;
-    int ntiles = (n + kTile - 1) / kTile;
+    const int tile = radix_tile(n), ntiles = (n + tile - 1) / tile;
     int h = 256 * ntiles;
     int* offs = hist + h;
     int* scratch = offs + h;
@@ -182,9 +188,11 @@ int radix_sort_pairs(uint32_t* keys, int* vals, uint32_t* tmpk, int* tmpv, int n
     int passes = (bits + 7) / 8;
     for (int p = 0; p < passes; ++p) {
         int shift = 8 * p;
-        k_radix_hist<<<ntiles, kRadixThreads, 0, s>>>(ka, n, shift, hist, ntiles);
+        if (tile == 1024) k_radix_hist<1024><<<ntiles, kRadixThreads, 0, s>>>(ka, n, shift, hist, ntiles);
+        else k_radix_hist<4096><<<ntiles, kRadixThreads, 0, s>>>(ka, n, shift, hist, ntiles);
         scan_exclusive(hist, offs, h, nullptr, scratch, s);
-        k_radix_scatter<<<ntiles, kRadixThreads, 0, s>>>(ka, va, kb, vb, n, shift, offs, ntiles);
+        if (tile == 1024) k_radix_scatter<1024><<<ntiles, kRadixThreads, 0, s>>>(ka, va, kb, vb, n, shift, offs, ntiles);
+        else k_radix_scatter<4096><<<ntiles, kRadixThreads, 0, s>>>(ka, va, kb, vb, n, shift, offs, ntiles);
         uint32_t* tk = ka; ka = kb; kb = tk;
         int* tv = va; va = vb; vb = tv;
     }
