@@ -238,26 +238,29 @@ int launch_trimesh_bounds(const World& w, int c0, int c1, bool margin, cudaStrea
 
 // ---------------------------------------------------------------- Morton keys
 
-__global__ void k_scene_bounds(World w, FrameBuf f) {
-    int s = blockIdx.x;
+// Bounds of the enabled colliders' centres of scene s, and (w of the upper corner) the
+// mean longest side of their bounds, by the first 256 threads of a block; valid in thread 0.
+constexpr int kBoundsThreads = 256;
+template <int kRound>
+__device__ __forceinline__ void scene_bounds(const World& w, int s, float4& out_lo, float4& out_hi) {
     int cs = w.scene_col[s], ce = w.scene_col[s + 1];
+    if (threadIdx.x >= kBoundsThreads) ce = cs;
     float lo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, hi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
     float size_sum = 0.f;   // longest side of the colliders' bounds, summed
     int count = 0;
     // Latency-bound: one block reads the whole scene, and each round of loads is a trip to
-    // L2 or beyond.  Twelve colliders a thread are read in one round and folded in the same
+    // L2 or beyond.  kRound colliders a thread are read in one round and folded in the same
     // order as one by one (the sum's rounding decides which colliders count as large):
     // 65,537 colliders took 257 us one at a time.
-    constexpr int kRound = 12;
-    for (int base = cs + threadIdx.x; base < ce; base += kRound * blockDim.x) {
+    for (int base = cs + threadIdx.x; base < ce; base += kRound * kBoundsThreads) {
         float4 a[kRound], b[kRound];
         bool on[kRound];
 #pragma unroll
         for (int u = 0; u < kRound; ++u) {
-            const int c = min(base + u * (int)blockDim.x, ce - 1);
+            const int c = min(base + u * kBoundsThreads, ce - 1);
             a[u] = w.aabb_min[c];
             b[u] = w.aabb_max[c];
-            on[u] = base + u * (int)blockDim.x < ce && (w.col_info[c].w & COL_ENABLE);   // disabled colliders never pair
+            on[u] = base + u * kBoundsThreads < ce && (w.col_info[c].w & COL_ENABLE);   // disabled colliders never pair
         }
 #pragma unroll
         for (int u = 0; u < kRound; ++u) {
@@ -281,22 +284,27 @@ __global__ void k_scene_bounds(World w, FrameBuf f) {
         count += __shfl_xor_sync(0xffffffffu, count, o);
     }
     int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    if (lane == 0) {
+    if (lane == 0 && wid < kBoundsThreads / 32) {
         for (int k = 0; k < 3; ++k) { sh[k][wid] = lo[k]; sh[3 + k][wid] = hi[k]; }
         sh[6][wid] = size_sum;
         shn[wid] = count;
     }
     __syncthreads();
     if (threadIdx.x == 0) {
-        for (int q = 1; q < (int)(blockDim.x >> 5); ++q) {
+        for (int q = 1; q < kBoundsThreads / 32; ++q) {
             for (int k = 0; k < 3; ++k) { sh[k][0] = fminf(sh[k][0], sh[k][q]); sh[3 + k][0] = fmaxf(sh[3 + k][0], sh[3 + k][q]); }
             sh[6][0] += sh[6][q];
             shn[0] += shn[q];
         }
-        // .w of the upper corner: the colliders' mean longest side
-        f.scene_lo[s] = make_float4(sh[0][0], sh[1][0], sh[2][0], 0.f);
-        f.scene_hi[s] = make_float4(sh[3][0], sh[4][0], sh[5][0], shn[0] ? sh[6][0] / (float)shn[0] : 0.f);
+        out_lo = make_float4(sh[0][0], sh[1][0], sh[2][0], 0.f);
+        out_hi = make_float4(sh[3][0], sh[4][0], sh[5][0], shn[0] ? sh[6][0] / (float)shn[0] : 0.f);
     }
+}
+
+__global__ void __launch_bounds__(kBoundsThreads) k_scene_bounds(World w, FrameBuf f) {
+    float4 lo, hi;
+    scene_bounds<12>(w, blockIdx.x, lo, hi);
+    if (threadIdx.x == 0) { f.scene_lo[blockIdx.x] = lo; f.scene_hi[blockIdx.x] = hi; }
 }
 
 __device__ __forceinline__ uint32_t expand_bits(uint32_t v, int bits) {
@@ -315,30 +323,31 @@ __device__ __forceinline__ uint32_t expand_bits(uint32_t v, int bits) {
 // ones' leaves instead of walking the whole tree itself.  The code depends only on the
 // collider's own scene, never on how many scenes share the world, so a scene gets the
 // same order alone or in any batch.
+__device__ __forceinline__ uint32_t morton_code(const World& w, int c, float4 lo, float4 hi) {
+    if (!(w.col_info[c].w & COL_ENABLE)) return 1u << 31;
+    float4 a = w.aabb_min[c], b = w.aabb_max[c];
+    const float scale = 1024.f;
+    float m[3] = {(a.x + b.x) * 0.5f, (a.y + b.y) * 0.5f, (a.z + b.z) * 0.5f};
+    float l[3] = {lo.x, lo.y, lo.z}, h[3] = {hi.x, hi.y, hi.z};
+    uint32_t code = 0;
+    for (int k = 0; k < 3; ++k) {
+        float ext = h[k] - l[k];
+        float u = ext > 0.f ? (m[k] - l[k]) / ext : 0.f;
+        u = fminf(fmaxf(u, 0.f), 1.f);
+        uint32_t q = (uint32_t)fminf(u * scale, scale - 1.f);
+        code |= expand_bits(q, 10) << (2 - k);
+    }
+    float spread = fmaxf(fmaxf(h[0] - l[0], h[1] - l[1]), h[2] - l[2]);
+    float size = fmaxf(fmaxf(b.x - a.x, b.y - a.y), b.z - a.z);
+    if ((spread > 0.f && size >= 0.25f * spread) || (hi.w > 0.f && size >= 16.f * hi.w)) code |= 1u << 30;
+    return code;
+}
+
 __global__ void k_morton(World w, FrameBuf f) {
     int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= w.n_colliders) return;
-    int4 ci = w.col_info[c];
-    uint32_t code = 1u << 31;
-    if (ci.w & COL_ENABLE) {
-        int s = w.info[ci.x].w;
-        float4 lo = f.scene_lo[s], hi = f.scene_hi[s];
-        float4 a = w.aabb_min[c], b = w.aabb_max[c];
-        const float scale = 1024.f;
-        float m[3] = {(a.x + b.x) * 0.5f, (a.y + b.y) * 0.5f, (a.z + b.z) * 0.5f};
-        float l[3] = {lo.x, lo.y, lo.z}, h[3] = {hi.x, hi.y, hi.z};
-        code = 0;
-        for (int k = 0; k < 3; ++k) {
-            float ext = h[k] - l[k];
-            float u = ext > 0.f ? (m[k] - l[k]) / ext : 0.f;
-            u = fminf(fmaxf(u, 0.f), 1.f);
-            uint32_t q = (uint32_t)fminf(u * scale, scale - 1.f);
-            code |= expand_bits(q, 10) << (2 - k);
-        }
-        float spread = fmaxf(fmaxf(h[0] - l[0], h[1] - l[1]), h[2] - l[2]);
-        float size = fmaxf(fmaxf(b.x - a.x, b.y - a.y), b.z - a.z);
-        if ((spread > 0.f && size >= 0.25f * spread) || (hi.w > 0.f && size >= 16.f * hi.w)) code |= 1u << 30;
-    }
+    const int s = w.info[w.col_info[c].x].w;
+    const uint32_t code = morton_code(w, c, f.scene_lo[s], f.scene_hi[s]);
     f.mkey[c] = code;
     f.keys[c] = code;
     f.order[c] = c;
@@ -360,11 +369,35 @@ __global__ void k_gather_keys(World w, FrameBuf f) {
 
 // ---------------------------------------------------------------- Karras radix tree
 
-__device__ __forceinline__ int kdelta(const uint32_t* keys, int n, int i, int j) {
+// length of the common prefix of the keys of sorted leaves i and j (equal keys: of their positions)
+template <class K>
+__device__ __forceinline__ int kdelta(const K& keys, int n, int i, int j) {
     if (j < 0 || j >= n) return -1;
-    uint32_t a = keys[i], b = keys[j];
+    uint32_t a = keys(i), b = keys(j);
     if (a == b) return 32 + __clz((uint32_t)(i ^ j));
     return __clz(a ^ b);
+}
+
+// internal node i of a tree over n sorted leaves: the leaves [lo, hi] it covers, split after gamma
+template <class K>
+__device__ __forceinline__ void karras_node(const K& keys, int n, int i, int& lo, int& hi, int& gamma) {
+    int d = (kdelta(keys, n, i, i + 1) - kdelta(keys, n, i, i - 1)) >= 0 ? 1 : -1;
+    int dmin = kdelta(keys, n, i, i - d);
+    int lmax = 2;
+    while (kdelta(keys, n, i, i + lmax * d) > dmin) lmax <<= 1;
+    int l = 0;
+    for (int t = lmax >> 1; t >= 1; t >>= 1)
+        if (kdelta(keys, n, i, i + (l + t) * d) > dmin) l += t;
+    int j = i + l * d;
+    int dnode = kdelta(keys, n, i, j);
+    int sp = 0, t = l;
+    do {
+        t = (t + 1) >> 1;
+        if (kdelta(keys, n, i, i + (sp + t) * d) > dnode) sp += t;
+    } while (t > 1);
+    gamma = i + sp * d + min(d, 0);
+    lo = min(i, j);
+    hi = max(i, j);
 }
 
 __device__ __forceinline__ int scene_of_position(const World& w, int p) {
@@ -385,24 +418,10 @@ __global__ void k_karras(World w, FrameBuf f) {
     int n = ce - cs;
     int i = p - cs;
     if (n < 2 || i >= n - 1) return;
-    const uint32_t* keys = f.keys + cs;
+    const uint32_t* sorted = f.keys + cs;
     int ibase = cs - s;
-    int d = (kdelta(keys, n, i, i + 1) - kdelta(keys, n, i, i - 1)) >= 0 ? 1 : -1;
-    int dmin = kdelta(keys, n, i, i - d);
-    int lmax = 2;
-    while (kdelta(keys, n, i, i + lmax * d) > dmin) lmax <<= 1;
-    int l = 0;
-    for (int t = lmax >> 1; t >= 1; t >>= 1)
-        if (kdelta(keys, n, i, i + (l + t) * d) > dmin) l += t;
-    int j = i + l * d;
-    int dnode = kdelta(keys, n, i, j);
-    int sp = 0, t = l;
-    do {
-        t = (t + 1) >> 1;
-        if (kdelta(keys, n, i, i + (sp + t) * d) > dnode) sp += t;
-    } while (t > 1);
-    int gamma = i + sp * d + min(d, 0);
-    int lo = min(i, j), hi = max(i, j);
+    int lo, hi, gamma;
+    karras_node([&](int q) { return sorted[q]; }, n, i, lo, hi, gamma);
     int node = ibase + i;
     int left = (lo == gamma) ? ~(cs + gamma) : ibase + gamma;
     int right = (hi == gamma + 1) ? ~(cs + gamma + 1) : ibase + gamma + 1;
@@ -650,42 +669,107 @@ __global__ void k_pairs_check(FrameBuf f, int* err) {
     if (*f.n_pairs > f.pair_cap) { atomicOr(err, ERR_PAIR_CAPACITY); *f.n_pairs = f.pair_cap; }
 }
 
-// One block per scene sorts the scene's (Morton code, collider) pairs in shared memory
-// with a bitonic network over 64-bit keys (code << 32 | collider), which orders equal
-// codes by collider exactly like the stable radix sort.  A scene that is not running
-// gets a constant code instead: its tree is never walked, only built and refitted.
-__global__ void __launch_bounds__(256) k_scene_sort(World w, FrameBuf f, int pmax) {
-    extern __shared__ unsigned long long sk[];
-    const int s = blockIdx.x;
+// The whole tree of a scene of at most 4096 colliders by one block: centre bounds, Morton
+// codes, the sort, Karras' construction and the bottom-up refit.  The sort is a bitonic
+// network over 64-bit keys (code << 32 | collider) in shared memory, which orders equal
+// codes by collider exactly like the stable radix sort.  Five launches of separate kernels
+// took 91 us on a scene of 2001 colliders and 37 us on one of 17, most of it the refit's
+// device-wide fences (two a level) and the launches; within a block a level is a
+// shared-memory count and a block fence.  Broadphase stage with the five and with the one:
+// 85 and 57 us (17 colliders), 243 and 207 (2001), 1569 and 1370 (4096 scenes).  A scene that is not running keeps its colliders'
+// order and gets no tree (nothing walks it), except for queries (ALL), which see it in
+// that order.
+__host__ __device__ constexpr size_t scene_tree_bytes(int pmax) { return (size_t)pmax * (8 + 4 + 2 + 4); }
+template <bool ALL>
+__global__ void __launch_bounds__(1024) k_scene_tree(World w, FrameBuf f, int pmax) {
+    extern __shared__ unsigned long long sk[];                                    // [pmax] sort keys
+    unsigned* const up = reinterpret_cast<unsigned*>(sk + pmax);                  // [pmax] node: parent | children done << 16
+    unsigned short* const leaf_up = reinterpret_cast<unsigned short*>(up + pmax); // [pmax] leaf: parent
+    short2* const kids = reinterpret_cast<short2*>(leaf_up + pmax);               // [pmax] node: children, leaves as ~position
+    const int s = blockIdx.x, tid = threadIdx.x, nth = blockDim.x;
     const int cs = w.scene_col[s], n = w.scene_col[s + 1] - cs;
     if (n <= 0) return;
-    if (w.scene_active && !w.scene_active[s]) {
-        for (int i = threadIdx.x; i < n; i += blockDim.x) { f.order[cs + i] = cs + i; f.keys[cs + i] = 0u; }
+    const bool idle = w.scene_active && !w.scene_active[s];
+    if (idle && !ALL) {
+        for (int i = tid; i < n; i += nth) f.order[cs + i] = cs + i;
         return;
     }
+    __shared__ float4 lo_hi[2];
+    {
+        float4 lo, hi;
+        scene_bounds<4>(w, s, lo, hi);
+        if (tid == 0) { lo_hi[0] = lo; lo_hi[1] = hi; }
+    }
+    __syncthreads();
     int P = 1;
     while (P < n) P <<= 1;
     if (P > pmax) return;   // the launch sizes pmax for the largest scene
-    for (int i = threadIdx.x; i < P; i += blockDim.x)
-        sk[i] = i < n ? ((unsigned long long)f.mkey[cs + i] << 32) | (unsigned)(cs + i) : ~0ull;
+    for (int i = tid; i < P; i += nth)
+        sk[i] = i < n ? ((unsigned long long)(idle ? 0u : morton_code(w, cs + i, lo_hi[0], lo_hi[1])) << 32) | (unsigned)(cs + i) : ~0ull;
     __syncthreads();
     for (int size = 2; size <= P; size <<= 1) {
         for (int stride = size >> 1; stride > 0; stride >>= 1) {
-            for (int t = threadIdx.x; t < P / 2; t += blockDim.x) {
+            for (int t = tid; t < P / 2; t += nth) {
                 int i = 2 * t - (t & (stride - 1));   // first of the pair
                 int j = i + stride;
-                bool up = (i & size) == 0;
+                bool asc = (i & size) == 0;
                 unsigned long long a = sk[i], b = sk[j];
-                if ((a > b) == up) { sk[i] = b; sk[j] = a; }
+                if ((a > b) == asc) { sk[i] = b; sk[j] = a; }
             }
             __syncthreads();
         }
     }
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        unsigned long long v = sk[i];
-        f.order[cs + i] = (int)(unsigned)v;
-        f.keys[cs + i] = (uint32_t)(v >> 32);
+    for (int i = tid; i < n; i += nth) f.order[cs + i] = (int)(unsigned)sk[i];
+    if (n < 2) return;
+    const int ibase = cs - s;
+    if (tid == 0) up[0] = 0xffffu;
+    for (int i = tid; i < n - 1; i += nth) {
+        int lo, hi, gamma;
+        karras_node([&](int q) { return (uint32_t)(sk[q] >> 32); }, n, i, lo, hi, gamma);
+        const bool lleaf = lo == gamma, rleaf = hi == gamma + 1;
+        const int node = ibase + i;
+        f.bvh.left[node] = lleaf ? ~(cs + gamma) : ibase + gamma;
+        f.bvh.right[node] = rleaf ? ~(cs + gamma + 1) : ibase + gamma + 1;
+        f.bvh.last[node] = cs + hi;
+        kids[i] = make_short2((short)(lleaf ? ~gamma : gamma), (short)(rleaf ? ~(gamma + 1) : gamma + 1));
+        if (lleaf) leaf_up[gamma] = (unsigned short)i; else up[gamma] = (unsigned)i;
+        if (rleaf) leaf_up[gamma + 1] = (unsigned short)i; else up[gamma + 1] = (unsigned)i;
     }
+    __syncthreads();
+    for (int p = tid; p < n; p += nth) {
+        unsigned node = leaf_up[p];
+        while (node != 0xffffu) {
+            __threadfence_block();
+            const unsigned before = atomicAdd(&up[node], 0x10000u);
+            if (before < 0x10000u) break;   // the other child's thread goes on
+            __threadfence_block();
+            const short2 k = kids[node];
+            float4 lmin, lmax, rmin, rmax;
+            if (k.x < 0) leaf_bounds<ALL>(w, (int)(unsigned)sk[~k.x], lmin, lmax);
+            else { lmin = f.bvh.bmin[ibase + k.x]; lmax = f.bvh.bmax[ibase + k.x]; }
+            if (k.y < 0) leaf_bounds<ALL>(w, (int)(unsigned)sk[~k.y], rmin, rmax);
+            else { rmin = f.bvh.bmin[ibase + k.y]; rmax = f.bvh.bmax[ibase + k.y]; }
+            f.bvh.bmin[ibase + node] = make_float4(fminf(lmin.x, rmin.x), fminf(lmin.y, rmin.y), fminf(lmin.z, rmin.z), 0.f);
+            f.bvh.bmax[ibase + node] = make_float4(fmaxf(lmax.x, rmax.x), fmaxf(lmax.y, rmax.y), fmaxf(lmax.z, rmax.z), 0.f);
+            node = before & 0xffffu;
+        }
+    }
+}
+
+template <bool ALL>
+static void launch_scene_tree(const World& w, FrameBuf& f, int pmax, cudaStream_t s) {
+    constexpr int kMaxDevices = 64;
+    static int done[kMaxDevices] = {};
+    const int bytes = (int)scene_tree_bytes(pmax);
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev >= 0 && dev < kMaxDevices && done[dev] < bytes) {
+        cudaFuncSetAttribute(k_scene_tree<ALL>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+        done[dev] = bytes;
+    }
+    // few scenes: a block as wide as its sort has pairs, for latency
+    const int threads = w.n_scenes <= 152 ? std::max(kBoundsThreads, std::min(1024, pmax / 2)) : kBoundsThreads;
+    k_scene_tree<ALL><<<w.n_scenes, threads, bytes, s>>>(w, f, pmax);
 }
 
 // Each scene's LBVH over the colliders' current bounds: scene bounds, Morton codes, the
@@ -693,14 +777,16 @@ __global__ void __launch_bounds__(256) k_scene_sort(World w, FrameBuf f, int pma
 int launch_bvh_build(const World& w, FrameBuf& f, int scene_bits, int scene_sort_pmax, bool all_leaves, cudaStream_t s) {
     int n = w.n_colliders;
     if (n == 0) return 0;
+    if (scene_sort_pmax > 0) {
+        if (all_leaves) launch_scene_tree<true>(w, f, scene_sort_pmax, s);
+        else launch_scene_tree<false>(w, f, scene_sort_pmax, s);
+        return 1;
+    }
     int nb = (n + 255) / 256;
-    k_scene_bounds<<<w.n_scenes, 256, 0, s>>>(w, f);
+    k_scene_bounds<<<w.n_scenes, kBoundsThreads, 0, s>>>(w, f);
     k_morton<<<nb, 256, 0, s>>>(w, f);
     int k = 2;
-    if (scene_sort_pmax > 0) {
-        k_scene_sort<<<w.n_scenes, 256, scene_sort_pmax * sizeof(unsigned long long), s>>>(w, f, scene_sort_pmax);
-        ++k;
-    } else {
+    {
         // (scene, Morton) order as two stable LSD sorts: Morton first, then scene
         k += radix_sort_pairs(f.keys, f.order, f.keys_tmp, f.order_tmp, n, 32, f.radix_hist, s);
         if (scene_bits > 0) {
@@ -720,7 +806,7 @@ int launch_broadphase(const World& w, FrameBuf& f, int scene_bits, int scene_sor
     int n = w.n_colliders;
     if (n == 0) return 0;
     int nb = (n + 255) / 256;
-    int k = launch_bvh_build(w, f, scene_bits, scene_sort_pmax, false, s) - 2;
+    int k = launch_bvh_build(w, f, scene_bits, scene_sort_pmax, false, s);
     if (f.trav_k > 0) {   // one walk, the kept pairs placed after the scan, a second walk only for long lists
         k_traverse<kCollect><<<nb, 256, 0, s>>>(w, f);
         scan_exclusive(f.leaf_cnt, f.leaf_off, n, f.n_pairs, f.scan_scratch, s);
@@ -733,7 +819,7 @@ int launch_broadphase(const World& w, FrameBuf& f, int scene_bits, int scene_sor
         k_traverse<kEmit><<<nb, 256, 0, s>>>(w, f);
     }
     k_pairs_check<<<1, 1, 0, s>>>(f, w.err);
-    return k + 4 + 3 + 1;
+    return k + 2 + 3 + 1;
 }
 
 }  // namespace psx

@@ -134,7 +134,7 @@ int launch_apply_deltas(const World& w, const DeltaRec* d, int n, const int* joi
 int launch_unpack_bodies(const World& w, const float* pos, const float* vel, const float* ang, cudaStream_t s);
 int launch_pack_bodies(const World& w, float* pos, float* vel, float* ang, cudaStream_t s);
 // scene_sort_pmax > 0: every scene has at most that many colliders (a power of two) and
-// is sorted by its own block in shared memory; 0: one radix sort over the whole world
+// its own block builds its tree; 0: one radix sort over the whole world
 int launch_broadphase(const World& w, FrameBuf& f, int scene_bits, int scene_sort_pmax, cudaStream_t s);
 // each scene's LBVH over the current bounds (all_leaves: every collider reachable, for queries)
 int launch_bvh_build(const World& w, FrameBuf& f, int scene_bits, int scene_sort_pmax, bool all_leaves, cudaStream_t s);
