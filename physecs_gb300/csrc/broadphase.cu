@@ -20,8 +20,9 @@ namespace psx {
 // getBounds (src/BoundsUtil.cpp:23-85) at the collider's world pose (src/Physecs.cpp:79-90).
 // margin_mode 0: every collider, no margin (onRigidBodyCreate, src/Physecs.cpp:25-37);
 // margin_mode 1: colliders of simulated dynamic bodies, +0.01 m (src/Physecs.cpp:555-559).
-__global__ void k_aabb(World w, int c0, int c1, int margin_mode) {
+__global__ void k_aabb(World w, int c0, int c1, int margin_mode, int* flip) {
     int c = c0 + blockIdx.x * blockDim.x + threadIdx.x;
+    if (flip && c == c0) *flip ^= 1;
     if (c >= c1) return;
     int4 ci = w.col_info[c];
     int4 bi = w.info[ci.x];
@@ -215,13 +216,13 @@ int launch_apply_deltas(const World& w, const DeltaRec* d, int n, const int* joi
     return k;
 }
 
-int launch_aabb(const World& w, int margin_mode, cudaStream_t s) {
-    return launch_aabb_range(w, 0, w.n_colliders, margin_mode, s);
+int launch_aabb(const World& w, int margin_mode, cudaStream_t s, int* flip) {
+    return launch_aabb_range(w, 0, w.n_colliders, margin_mode, s, flip);
 }
 
-int launch_aabb_range(const World& w, int c0, int c1, int margin_mode, cudaStream_t s) {
+int launch_aabb_range(const World& w, int c0, int c1, int margin_mode, cudaStream_t s, int* flip) {
     if (c1 <= c0) return 0;
-    k_aabb<<<(c1 - c0 + 255) / 256, 256, 0, s>>>(w, c0, c1, margin_mode);
+    k_aabb<<<(c1 - c0 + 255) / 256, 256, 0, s>>>(w, c0, c1, margin_mode, flip);
     if (margin_mode == 1) return 1;
     return 1 + launch_trimesh_bounds(w, c0, c1, false, s);
 }
@@ -528,9 +529,15 @@ __device__ __forceinline__ void place_pair(const World& w, const FrameBuf& f, in
     }
 }
 
+// the pair count kept within the list's room
+__device__ __forceinline__ void check_pairs(const World& w, const FrameBuf& f) {
+    if (*f.n_pairs > f.pair_cap) { atomicOr(w.err, ERR_PAIR_CAPACITY); *f.n_pairs = f.pair_cap; }
+}
+
 template <int MODE>
 __global__ void __launch_bounds__(256) k_traverse(World w, FrameBuf f) {
     constexpr bool EMIT = MODE == kEmit || MODE == kTail;
+    if (MODE == kEmit && blockIdx.x == 0 && threadIdx.x == 0) check_pairs(w, f);
     if (MODE == kTail && *f.trav_tail == 0) return;
     if (MODE == kCollect && blockIdx.x == 0 && threadIdx.x == 0) *f.trav_tail = 0;
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
@@ -644,6 +651,7 @@ __global__ void __launch_bounds__(256) k_traverse(World w, FrameBuf f) {
 // warp per 32 leaves so that the copies of one leaf are consecutive lanes' stores.
 __global__ void __launch_bounds__(256) k_pairs_place(World w, FrameBuf f) {
     const int K = f.trav_k;
+    if (blockIdx.x == 0 && threadIdx.x == 0) check_pairs(w, f);
     const int lane = threadIdx.x & 31;
     const int warps = (gridDim.x * blockDim.x) >> 5;
     const int2* scratch = trav_scratch(f);
@@ -663,10 +671,6 @@ __global__ void __launch_bounds__(256) k_pairs_place(World w, FrameBuf f) {
         }
     }
     if (tail) *f.trav_tail = 1;
-}
-
-__global__ void k_pairs_check(FrameBuf f, int* err) {
-    if (*f.n_pairs > f.pair_cap) { atomicOr(err, ERR_PAIR_CAPACITY); *f.n_pairs = f.pair_cap; }
 }
 
 // The whole tree of a scene of at most 4096 colliders by one block: centre bounds, Morton
@@ -809,17 +813,15 @@ int launch_broadphase(const World& w, FrameBuf& f, int scene_bits, int scene_sor
     int k = launch_bvh_build(w, f, scene_bits, scene_sort_pmax, false, s);
     if (f.trav_k > 0) {   // one walk, the kept pairs placed after the scan, a second walk only for long lists
         k_traverse<kCollect><<<nb, 256, 0, s>>>(w, f);
-        scan_exclusive(f.leaf_cnt, f.leaf_off, n, f.n_pairs, f.scan_scratch, s);
+        k += scan_exclusive(f.leaf_cnt, f.leaf_off, n, f.n_pairs, f.scan_scratch, s);
         k_pairs_place<<<std::min(nb, 152 * 8), 256, 0, s>>>(w, f);
         k_traverse<kTail><<<nb, 256, 0, s>>>(w, f);
-        ++k;
-    } else {
-        k_traverse<kCount><<<nb, 256, 0, s>>>(w, f);
-        scan_exclusive(f.leaf_cnt, f.leaf_off, n, f.n_pairs, f.scan_scratch, s);
-        k_traverse<kEmit><<<nb, 256, 0, s>>>(w, f);
+        return k + 3;
     }
-    k_pairs_check<<<1, 1, 0, s>>>(f, w.err);
-    return k + 2 + 3 + 1;
+    k_traverse<kCount><<<nb, 256, 0, s>>>(w, f);
+    k += scan_exclusive(f.leaf_cnt, f.leaf_off, n, f.n_pairs, f.scan_scratch, s);
+    k_traverse<kEmit><<<nb, 256, 0, s>>>(w, f);
+    return k + 2;
 }
 
 }  // namespace psx

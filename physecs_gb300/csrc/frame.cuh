@@ -122,8 +122,9 @@ struct FrameBuf {
 
 // kernel launch helpers (definitions in the .cu files); each returns the number of
 // kernels it queued
-int launch_aabb(const World& w, int margin_mode, cudaStream_t s);
-int launch_aabb_range(const World& w, int c0, int c1, int margin_mode, cudaStream_t s);
+// flip (the frame's last kernel): the restitution cache's parity, toggled
+int launch_aabb(const World& w, int margin_mode, cudaStream_t s, int* flip = nullptr);
+int launch_aabb_range(const World& w, int c0, int c1, int margin_mode, cudaStream_t s, int* flip = nullptr);
 // getBoundsTriangleMesh for the triangle-mesh colliders in [c0, c1), with the 0.01 m
 // margin of updateBounds or without it
 int launch_trimesh_bounds(const World& w, int c0, int c1, bool margin, cudaStream_t s);

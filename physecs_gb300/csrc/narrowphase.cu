@@ -500,44 +500,50 @@ static void launch_convex_epa_flat(const World& w, FrameBuf& f, cudaStream_t s) 
 
 // The convex kernels (bound by the FP64 pipe) run on the aux stream beside the analytic
 // and triangle-mesh kernels (FP32, latency-bound); the categories write disjoint slots.
+// The kernels of kinds of pairs that the world cannot have are not launched: an empty
+// convex chain costs a fork, five launches and a join, an empty k_narrow_tri 20 us (its
+// blocks' shared memory).
 int launch_narrowphase(const World& w, FrameBuf& f, const StreamPair& sp, const NarrowShape& ns, cudaStream_t s) {
     cudaMemsetAsync(f.cat_count, 0, 10 * sizeof(int), s);
     k_classify<<<1216, 256, 0, s>>>(w, f);
-    cudaEventRecord(sp.fork, s);
-    cudaStreamWaitEvent(sp.aux, sp.fork, 0);
-    k_convex_gjk<<<152 * ns.gjk_blocks_per_sm, 128, 0, sp.aux>>>(w, f);
-    // epa_lanes 1: a lane per pair first; the pairs that outgrow it go to the grouped
-    // kernel (16 lanes), or with epa_full_only straight to the full polytope.
-    // (Generating the finished pairs' contacts on another stream beside the longer passes
-    // was measured slower: it takes SMs from them.)
-    const bool flat = ns.epa_lanes == 1;
-    if (flat) launch_convex_epa_flat(w, f, sp.aux);
-    if (!ns.epa_full_only) {
-        const int src = flat ? 8 : 3;
-        if (ns.epa_lanes == 8) launch_convex_epa<8, 1>(w, f, ns.convex_blocks_per_sm, src, sp.aux);
-        else if (ns.epa_lanes == 16 || ns.epa_lanes == 1) launch_convex_epa<16, 1>(w, f, ns.convex_blocks_per_sm, src, sp.aux);
-        else if (ns.convex_warps == 1) launch_convex_epa<32, 1>(w, f, ns.convex_blocks_per_sm, src, sp.aux);
-        else if (ns.convex_warps == 2) launch_convex_epa<32, 2>(w, f, ns.convex_blocks_per_sm, src, sp.aux);
-        else launch_convex_epa<32, 3>(w, f, ns.convex_blocks_per_sm, src, sp.aux);
-    }
-    {
+    int k = 1;
+    if (w.may_convex) {
+        cudaEventRecord(sp.fork, s);
+        cudaStreamWaitEvent(sp.aux, sp.fork, 0);
+        k_convex_gjk<<<152 * ns.gjk_blocks_per_sm, 128, 0, sp.aux>>>(w, f);
+        // epa_lanes 1: a lane per pair first; the pairs that outgrow it go to the grouped
+        // kernel (16 lanes), or with epa_full_only straight to the full polytope.
+        // (Generating the finished pairs' contacts on another stream beside the longer passes
+        // was measured slower: it takes SMs from them.)
+        const bool flat = ns.epa_lanes == 1;
+        if (flat) { launch_convex_epa_flat(w, f, sp.aux); ++k; }
+        if (!ns.epa_full_only) {
+            const int src = flat ? 8 : 3;
+            if (ns.epa_lanes == 8) launch_convex_epa<8, 1>(w, f, ns.convex_blocks_per_sm, src, sp.aux);
+            else if (ns.epa_lanes == 16 || ns.epa_lanes == 1) launch_convex_epa<16, 1>(w, f, ns.convex_blocks_per_sm, src, sp.aux);
+            else if (ns.convex_warps == 1) launch_convex_epa<32, 1>(w, f, ns.convex_blocks_per_sm, src, sp.aux);
+            else if (ns.convex_warps == 2) launch_convex_epa<32, 2>(w, f, ns.convex_blocks_per_sm, src, sp.aux);
+            else launch_convex_epa<32, 3>(w, f, ns.convex_blocks_per_sm, src, sp.aux);
+            ++k;
+        }
         static bool done[kMaxDevices] = {};
         set_smem_attrs((const void*)k_convex_epa_full, done, (int)sizeof(WarpPoly));
         // the full pass alone: as many blocks as shared memory lets reside
         const int lst = ns.epa_full_only ? (flat ? 8 : 3) : 6;
         k_convex_epa_full<<<ns.epa_full_only && !flat ? 152 * 16 : 152 * 8, 32, sizeof(WarpPoly), sp.aux>>>(w, f, lst, flat);
+        k_convex_contacts<<<1216 * 128 / ns.contacts_threads, ns.contacts_threads, 0, sp.aux>>>(w, f);
+        cudaEventRecord(sp.join, sp.aux);
+        k += 3;
     }
-    k_convex_contacts<<<1216 * 128 / ns.contacts_threads, ns.contacts_threads, 0, sp.aux>>>(w, f);
-    cudaEventRecord(sp.join, sp.aux);
     // box-box pairs first: the longest
     k_narrow_analytic<2><<<152 * ns.analytic_blocks_per_sm, ns.analytic_threads, 0, s>>>(w, f);
     k_narrow_analytic<1><<<152 * ns.analytic_blocks_per_sm, ns.analytic_threads, 0, s>>>(w, f);
     k_narrow_analytic<0><<<152 * ns.analytic_blocks_per_sm, ns.analytic_threads, 0, s>>>(w, f);
-    k_narrow_tri<<<152 * 16, 32 * kTriWarps, 0, s>>>(w, f);
-    const int kt = launch_triggers(w, f, s);
-    cudaStreamWaitEvent(s, sp.join, 0);
-    scan_exclusive_dev(f.pair_nman, f.pair_moff, f.n_pairs, f.pair_cap, f.n_man, f.scan_scratch, s);
-    return 2 + 8 + 3 + kt + (flat ? 1 : 0) - (ns.epa_full_only ? 1 : 0);
+    k += 3;
+    if (w.n_trimesh_cols) { k_narrow_tri<<<152 * 16, 32 * kTriWarps, 0, s>>>(w, f); ++k; }
+    k += launch_triggers(w, f, s);
+    if (w.may_convex) cudaStreamWaitEvent(s, sp.join, 0);
+    return k + scan_exclusive_dev(f.pair_nman, f.pair_moff, f.n_pairs, f.pair_cap, f.n_man, f.scan_scratch, s);
 }
 
 }  // namespace psx

@@ -77,21 +77,59 @@ __global__ void k_scan_add(int* out, int n, const int* n_dev, const int* sums) {
 }
 }  // namespace
 
+namespace {
+// The whole scan in one block: below kSmallScan elements three launches cost more than
+// their work (about 2.5 us each in a frame's chain; up to eight rounds of 4096 here).
+constexpr int kSmallScan = 32768;
+__global__ void __launch_bounds__(1024) k_scan_small(const int* in, int* out, int n, const int* n_dev, int* total) {
+    __shared__ int sums[33];
+    if (n_dev) n = min(n, *n_dev);
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    int carry = 0;
+    for (int c = 0; c < n; c += 4096) {
+        const int base = c + threadIdx.x * 4;
+        int v[4], t = 0;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) { v[k] = base + k < n ? in[base + k] : 0; t += v[k]; }
+        const int inc = warp_incl_scan(t);
+        if (lane == 31) sums[wid] = inc;
+        __syncthreads();
+        if (wid == 0) {
+            const int w = sums[lane], wi = warp_incl_scan(w);
+            sums[lane] = wi - w;
+            if (lane == 31) sums[32] = wi;
+        }
+        __syncthreads();
+        int ex = carry + sums[wid] + inc - t;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) { if (base + k < n) out[base + k] = ex; ex += v[k]; }
+        carry += sums[32];
+        __syncthreads();
+    }
+    if (threadIdx.x == 0 && total) *total = carry;
+}
+}  // namespace
+
 size_t scan_scratch_ints(int n) { return (size_t)(n + kScanBlock - 1) / kScanBlock + 1; }
 
-static void scan_impl(const int* in, int* out, int n, const int* n_dev, int* total, int* scratch, cudaStream_t s) {
+static int scan_impl(const int* in, int* out, int n, const int* n_dev, int* total, int* scratch, cudaStream_t s) {
+    if (n <= kSmallScan) {
+        k_scan_small<<<1, 1024, 0, s>>>(in, out, n, n_dev, total);
+        return 1;
+    }
     int nb = (n + kScanBlock - 1) / kScanBlock;
     if (nb == 0) nb = 1;
     k_scan_blocks<<<nb, 256, 0, s>>>(in, out, n, n_dev, scratch);
     k_scan_sums<<<1, 256, 0, s>>>(scratch, nb, total);
     k_scan_add<<<nb, 256, 0, s>>>(out, n, n_dev, scratch);
+    return 3;
 }
 
-void scan_exclusive(const int* in, int* out, int n, int* total, int* scratch, cudaStream_t s) {
-    scan_impl(in, out, n, nullptr, total, scratch, s);
+int scan_exclusive(const int* in, int* out, int n, int* total, int* scratch, cudaStream_t s) {
+    return scan_impl(in, out, n, nullptr, total, scratch, s);
 }
-void scan_exclusive_dev(const int* in, int* out, const int* n_dev, int n_max, int* total, int* scratch, cudaStream_t s) {
-    scan_impl(in, out, n_max, n_dev, total, scratch, s);
+int scan_exclusive_dev(const int* in, int* out, const int* n_dev, int n_max, int* total, int* scratch, cudaStream_t s) {
+    return scan_impl(in, out, n_max, n_dev, total, scratch, s);
 }
 
 // ---------------------------------------------------------------- radix sort
@@ -185,12 +223,12 @@ int radix_sort_pairs(uint32_t* keys, int* vals, uint32_t* tmpk, int* tmpv, int n
     int* scratch = offs + h;
     uint32_t* ka = keys; int* va = vals;
     uint32_t* kb = tmpk; int* vb = tmpv;
-    int passes = (bits + 7) / 8;
+    int passes = (bits + 7) / 8, launches = 0;
     for (int p = 0; p < passes; ++p) {
         int shift = 8 * p;
         if (tile == 1024) k_radix_hist<1024><<<ntiles, kRadixThreads, 0, s>>>(ka, n, shift, hist, ntiles);
         else k_radix_hist<4096><<<ntiles, kRadixThreads, 0, s>>>(ka, n, shift, hist, ntiles);
-        scan_exclusive(hist, offs, h, nullptr, scratch, s);
+        launches += 2 + scan_exclusive(hist, offs, h, nullptr, scratch, s);
         if (tile == 1024) k_radix_scatter<1024><<<ntiles, kRadixThreads, 0, s>>>(ka, va, kb, vb, n, shift, offs, ntiles);
         else k_radix_scatter<4096><<<ntiles, kRadixThreads, 0, s>>>(ka, va, kb, vb, n, shift, offs, ntiles);
         uint32_t* tk = ka; ka = kb; kb = tk;
@@ -200,7 +238,7 @@ int radix_sort_pairs(uint32_t* keys, int* vals, uint32_t* tmpk, int* tmpv, int n
         cudaMemcpyAsync(keys, ka, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, s);
         cudaMemcpyAsync(vals, va, sizeof(int) * n, cudaMemcpyDeviceToDevice, s);
     }
-    return passes * 5;
+    return launches;
 }
 
 }  // namespace psx

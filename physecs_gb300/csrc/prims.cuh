@@ -7,11 +7,11 @@
 namespace psx {
 
 // Exclusive prefix sum of n ints; writes the grand total to *total (device pointer).
-// scratch must hold scan_scratch_ints(n) ints.
+// scratch must hold scan_scratch_ints(n) ints.  Returns the number of kernels queued.
 size_t scan_scratch_ints(int n);
-void scan_exclusive(const int* in, int* out, int n, int* total, int* scratch, cudaStream_t s);
+int scan_exclusive(const int* in, int* out, int n, int* total, int* scratch, cudaStream_t s);
 // Variant whose element count is read on the device from *n_dev (at most n_max elements).
-void scan_exclusive_dev(const int* in, int* out, const int* n_dev, int n_max, int* total, int* scratch, cudaStream_t s);
+int scan_exclusive_dev(const int* in, int* out, const int* n_dev, int n_max, int* total, int* scratch, cudaStream_t s);
 
 // Stable LSD radix sort of (key, value) pairs over bits [0, bits).  The result ends
 // up in (keys, vals); tmp buffers hold n elements each; hist needs radix_hist_ints(n).

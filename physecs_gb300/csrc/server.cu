@@ -260,6 +260,7 @@ PSX_API psx_status psx_server_create(const psx_server_opts* o, psx_server** out)
         return fail(PSX_ERR_OUT_OF_MEMORY, buf);
     }
     S->h_active.assign(n_slots, 0);
+    if (o->mesh_pool) W->w.may_convex = 1;   // requests bring convex colliders
     W->w.scene_active = S->d_active;
     W->w.scene_fresh = S->d_fresh;
     if (cudaMallocHost(&S->pin_active, sizeof(int) * n_slots) != cudaSuccess ||

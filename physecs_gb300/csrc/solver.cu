@@ -25,14 +25,15 @@ constexpr float kPi = 3.14159265358979323846f;
 // ---------------------------------------------------------------- restitution cache
 
 
-__global__ void k_cache_clear(FrameBuf f) {
+// before the contacts: this frame's cache table empty, the counters zero
+__global__ void k_contacts_begin(FrameBuf f, int n_scenes) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i == 0) *f.n_points = 0;
+    if (i <= n_scenes) f.man_scene_cnt[i] = 0;
     if (i >= f.cache_cap) return;
     CacheEntry* cur = f.cache_parity[0] ? f.cache_b : f.cache_a;
     cur[i].key = kEmpty;
 }
-
-__global__ void k_cache_flip(FrameBuf f) { f.cache_parity[0] ^= 1; }
 
 // ---------------------------------------------------------------- contact rows (src/Physecs.cpp:215-314)
 
@@ -1459,18 +1460,11 @@ __global__ void __launch_bounds__(NT, 1) k_solve_cluster(World w, FrameBuf f, co
     cl.sync();   // no block leaves while the others may still read its shared memory
 }
 
-__global__ void k_zero_ints(int* p, int n) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) p[i] = 0;
-}
-
 int launch_contacts(const World& w, FrameBuf& f, cudaStream_t s) {
-    k_cache_clear<<<(f.cache_cap + 255) / 256, 256, 0, s>>>(f);
-    k_zero_ints<<<(w.n_scenes + 256) / 256, 256, 0, s>>>(f.man_scene_cnt, w.n_scenes + 1);
-    k_zero_ints<<<1, 32, 0, s>>>(f.n_points, 1);
+    const int cells = std::max(f.cache_cap, w.n_scenes + 1);
+    k_contacts_begin<<<(cells + 255) / 256, 256, 0, s>>>(f, w.n_scenes);
     k_build_contacts<<<1216, 128, 0, s>>>(w, f);
-    scan_exclusive(f.man_scene_cnt, f.scene_man, w.n_scenes + 1, nullptr, f.scan_scratch, s);
-    return 4 + 3;
+    return 2 + scan_exclusive(f.man_scene_cnt, f.scene_man, w.n_scenes + 1, nullptr, f.scan_scratch, s);
 }
 
 int solver_grid_blocks() {
@@ -1525,7 +1519,7 @@ static void launch_block_ranked(int grid, int smem, cudaStream_t st, int rank, c
 }
 
 int launch_solver(const World& w, FrameBuf& f, const SolverLaunch& L, cudaStream_t s) {
-    int k = 1;
+    int k = 0;
     // large scenes on a second stream, concurrently with the small ones, and first: their
     // chains are the longest (measured with eager launches: solver stage 7.20 -> 6.65 ms
     // on the 4096-scene frame)
@@ -1611,7 +1605,6 @@ int launch_solver(const World& w, FrameBuf& f, const SolverLaunch& L, cudaStream
         cudaLaunchCooperativeKernel((void*)k_solve_grid, L.grid_blocks, 256, args, 0, s);
         ++k;
     }
-    k_cache_flip<<<1, 1, 0, s>>>(f);
     return k;
 }
 

@@ -195,6 +195,7 @@ struct World {
     int4* tri_src;         // per triangle, index order: mesh-local vertex indices, w = mesh's first vertex
     int* trimesh_cols;     // colliders whose shape is a triangle mesh
     int n_trimesh_cols;
+    int may_convex;        // some collider is, or in a serving slot may become, a convex mesh
     int2* trimesh_chunks;  // (trimesh_cols slot, chunk of kMeshBoundsChunk vertices) for their bounds
     int n_trimesh_chunks;
     unsigned long long* trimesh_keys;   // [6][n_trimesh_cols] bounds reduction keys

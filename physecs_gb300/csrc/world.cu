@@ -323,6 +323,8 @@ psx_status psx::rt::build_world(psx_world* W, const psx_scene_desc* scenes, int 
     PSX_TRY(W->alloc(w.bq, 2 * (size_t)w.n_dyn));
     PSX_TRY(W->alloc(w.sv, 2 * (size_t)w.n_dyn));
     PSX_TRY(W->upload(w.col_info, col_info));
+    w.may_convex = 0;
+    for (const int4& ci : col_info) w.may_convex |= ci.y == PSX_CONVEX_MESH;
     PSX_TRY(W->upload(w.col_pos, col_pos));
     PSX_TRY(W->upload(w.col_quat, col_quat));
     PSX_TRY(W->upload(w.col_params, col_params));
@@ -546,7 +548,7 @@ int psx::rt::queue_frame(psx_world* W, cudaEvent_t* ev) {
                    W->aux_stream, W->ev_fork, W->ev_join, W->wait_limit, W->large_nt};
     k += launch_solver(W->w, W->f, L, s);
     if (ev) cudaEventRecord(ev[4], s);
-    k += launch_aabb(W->w, 1, s);
+    k += launch_aabb(W->w, 1, s, W->f.cache_parity);
     if (ev) cudaEventRecord(ev[5], s);
     W->launches += k;
     return k;
