@@ -88,7 +88,7 @@ struct FrameBuf {
     int* claim_pos;       // [S * kColorBins] scatter counters of the same scenes
     // per-substep contact records of scenes whose records do not fit in shared memory
     int* pt_off;          // [man_cap] point slots of each contact, solve order: first slot, step - 1 from bit 28
-    int* pt_end;          // [man_cap] end of the slots of each contact's group
+    int* pt_group;        // [man_cap] first of the slots of each contact's group
     int2* cbody;          // [man_cap] colouring: scene-local dynamic bodies of each contact; then
                           // (solve_flow, solve order) its places among its bodies' solves
     int* bdeg;            // [n_dyn] solve_flow: a body's contacts | its solves per iteration << 16

@@ -447,7 +447,7 @@ psx_status psx::rt::build_world(psx_world* W, const psx_scene_desc* scenes, int 
     PSX_TRY(W->alloc(f.color_start, (size_t)S * kColorBins));
     PSX_TRY(W->alloc(f.claim_pos, (size_t)S * kColorBins));
     PSX_TRY(W->alloc(f.pt_off, f.man_cap));
-    PSX_TRY(W->alloc(f.pt_end, f.man_cap));
+    PSX_TRY(W->alloc(f.pt_group, f.man_cap));
     PSX_TRY(W->alloc(f.cbody, f.man_cap));
     PSX_TRY(W->alloc(f.cmask, std::max(1, w.n_dyn)));
     PSX_TRY(W->alloc(f.bdeg, std::max(1, w.n_dyn)));
