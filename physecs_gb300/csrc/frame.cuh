@@ -168,7 +168,7 @@ int launch_overlap_mtd(const World& w, FrameBuf& f, const ShapeIn* qs, int n, in
 // a second stream with a fork / join event pair, for kernels that may overlap
 struct StreamPair {
     cudaStream_t aux;
-    cudaEvent_t fork, join;
+    cudaEvent_t fork, join, mid;
 };
 struct NarrowShape {
     int convex_warps, convex_blocks_per_sm;   // EPA: warps per block, blocks per SM

@@ -95,7 +95,7 @@ struct psx_world {
     cudaEvent_t ev_tfork = nullptr, ev_tjoin[2] = {nullptr, nullptr};
     cudaStream_t aux_stream = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;     // solver: large scenes on the aux stream
-    cudaEvent_t ev_fork2 = nullptr, ev_join2 = nullptr;   // narrowphase: convex pairs on the aux stream
+    cudaEvent_t ev_fork2 = nullptr, ev_mid2 = nullptr, ev_join2 = nullptr;   // narrowphase: convex pairs on the aux stream
     std::vector<float4> h_knobs;
     bool use_graph = false;
     cudaGraphExec_t graph = nullptr;
@@ -150,6 +150,7 @@ struct psx_world {
         if (ev_fork) cudaEventDestroy(ev_fork);
         if (ev_fork2) cudaEventDestroy(ev_fork2);
         if (ev_join2) cudaEventDestroy(ev_join2);
+        if (ev_mid2) cudaEventDestroy(ev_mid2);
         if (ev_join) cudaEventDestroy(ev_join);
         if (aux_stream) cudaStreamDestroy(aux_stream);
         for (cudaStream_t t : tier_stream) if (t) cudaStreamDestroy(t);
