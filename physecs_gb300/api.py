@@ -304,12 +304,14 @@ class World:
         distance}; accept: one value per world body (nonzero: the filter accepts its
         entity) or None for every entity.  Returns {body, collider, entity, distance, pos}
         arrays; body -1 where a ray hits nothing."""
-        rays = np.asarray(rays, np.float64).reshape(-1, 8)
+        rays = np.asarray(rays)
+        if rays.dtype != np.float32:     # other types keep their scene indices exact
+            rays = np.asarray(rays, np.float64)
+        rays = rays.reshape(-1, 8)
         n = len(rays)
-        buf = np.zeros((n, 8), np.float32)
-        buf[:, 1:] = rays[:, 1:]
+        buf = rays.astype(np.float32, order="C")   # a copy: the scene index goes in as an integer
         buf.view(np.int32)[:, 0] = rays[:, 0].astype(np.int32)
-        out = np.zeros((max(n, 1), 7), np.float32)   # psx_ray_hit: 7 words
+        out = np.empty((max(n, 1), 7), np.float32)   # psx_ray_hit: 7 words
         acc = None if accept is None else np.ascontiguousarray(accept, np.uint8)
         _check(load().psx_world_raycast(self.h, n, _p(buf), _p(acc) if acc is not None else None, _p(out)))
         out = out[:n]

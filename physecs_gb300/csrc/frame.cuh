@@ -140,9 +140,9 @@ int launch_broadphase(const World& w, FrameBuf& f, int scene_bits, int scene_sor
 // each scene's LBVH over the current bounds (all_leaves: every collider reachable, for queries)
 int launch_bvh_build(const World& w, FrameBuf& f, int scene_bits, int scene_sort_pmax, bool all_leaves, cudaStream_t s);
 
-// scene queries (query.cu); the layouts are psx_ray and psx_overlap_query of include/psx.h
+// scene queries (query.cu); the layouts are psx_ray, psx_ray_hit and psx_overlap_query of include/psx.h
 struct RayIn { int scene; float ox, oy, oz, dx, dy, dz, maxd; };
-struct RayOut { int collider; float dist; };   // world collider index or -1
+struct RayOut { int body, collider; unsigned entity; float dist, x, y, z; };   // psx_ray_hit; body -1: no hit
 struct ShapeIn {
     int scene;
     float px, py, pz, qx, qy, qz, qw;
@@ -151,8 +151,8 @@ struct ShapeIn {
     int mesh;     // world convex mesh index
     int filter;   // collider data bits (0: any)
 };
-int launch_raycast(const World& w, FrameBuf& f, const RayIn* rays, int n, const unsigned char* accept, RayOut* out,
-                   cudaStream_t s);
+int launch_raycast(const World& w, FrameBuf& f, const RayIn* rays, int n, const unsigned char* accept,
+                   const int4* hit_ids, RayOut* out, cudaStream_t s);
 int launch_overlap(const World& w, FrameBuf& f, const ShapeIn* qs, int n, int cap, int* counts, int* hits, cudaStream_t s);
 // one CharacterController::move per record (psx_character layout; body is the world index)
 struct CharIn {

@@ -62,6 +62,7 @@ struct psx_world {
     size_t ddev_bytes = 0;
     cudaEvent_t ev_delta = nullptr;        // the last batch's upload is done
     void* qbuf = nullptr;                  // scene-query staging on the device
+    int4* hit_ids = nullptr;               // per collider: scene-local body, index within it, entity (from the first ray query on)
     std::vector<psx_trigger_event> trig_pending;   // drained from the device, not yet delivered
     long long trig_lost = 0;               // events past the device log's capacity
     // exits of last-frame trigger pairs whose collider a topology change removed: due at
