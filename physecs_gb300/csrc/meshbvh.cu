@@ -8,10 +8,10 @@
 // node ids, bounds (bit for bit) and leaf ranges.
 //
 //   * Top levels (nodes above kSmall triangles): level by level over chunks of kChunk
-//     triangles.  Bucket bounds are reduced with 64-bit keys (value, position) so that,
-//     among equal values (+0 / -0), the first triangle in the node's order wins, as in
-//     the reference's left fold.  One thread per node picks the split by the
-//     reference's own sequence of comparisons.
+//     triangles.  Bucket bounds are reduced as 32-bit keys; where one is zero, the first
+//     triangle in the node's order that has it decides between +0 and -0, as in the
+//     reference's left fold.  One warp per node picks the split by the reference's own
+//     sequence of comparisons.
 //   * The partition uses a closed form of the reference's two-pointer loop.  With k
 //     triangles going left, the loop keeps left triangles of [0, k) in place, pairs
 //     the t-th right triangle of [0, k) with the t-th left triangle of [k, n) counted
@@ -27,6 +27,7 @@
 //     starts once the tree is complete.
 #include <algorithm>
 #include <cfloat>
+#include <utility>
 #include <vector>
 #include "meshbvh.cuh"
 #include "ordkey.cuh"
@@ -83,13 +84,13 @@ struct Build {
 struct Level {
     Slot* slots;
     int* n_slots;
-    unsigned long long* keys;   // [slot][kKeys]
+    unsigned* keys;             // [slot][kKeys] bounds of the bins, as order-preserving keys
+    unsigned* zpos;             // [slot][kKeys] first position whose value is zero
     int* cnt;                   // [slot][kBins]
     int* chunk_slot;
     int* chunk_k;
     int* n_chunks;
     int2* chunk_cnt;            // (front-right, back-left) per chunk
-    int2* chunk_off;
     int slot_cap, chunk_cap;
 };
 
@@ -97,6 +98,9 @@ __device__ __forceinline__ unsigned long long kmin(float v, int pos) { return ke
 __device__ __forceinline__ unsigned long long kmax(float v, int pos) { return key_max(v, pos); }
 __device__ __forceinline__ int kpos_min(unsigned long long k) { return key_min_index(k); }
 __device__ __forceinline__ int kpos_max(unsigned long long k) { return key_max_index(k); }
+
+// the float of an order-preserving key (ordkey.cuh); zero comes back as +0
+__device__ __forceinline__ float key_float(unsigned k) { return __uint_as_float((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k); }
 
 __device__ __forceinline__ float comp(const TriDev& t, int c) {
     switch (c) {
@@ -181,34 +185,43 @@ __device__ int new_node(const Build& B, int start, int count, int mesh, int dept
     return id;
 }
 
-// a node above kSmall triangles joins the level: a slot, empty bins, its chunks
+// a node above kSmall triangles joins the level (by a whole warp): a slot, empty bins, its chunks
 __device__ void add_slot(const Level& Lv, int node, int count, const Build& B) {
-    const int s = atomicAdd(Lv.n_slots, 1);
-    const int nch = (count + kChunk - 1) / kChunk;
-    const int cb = atomicAdd(Lv.n_chunks, nch);
+    const int lane = threadIdx.x & 31, nch = (count + kChunk - 1) / kChunk;
+    int s = 0, cb = 0;
+    if (lane == 0) {
+        s = atomicAdd(Lv.n_slots, 1);
+        cb = atomicAdd(Lv.n_chunks, nch);
+    }
+    s = __shfl_sync(~0u, s, 0);
+    cb = __shfl_sync(~0u, cb, 0);
     if (s >= Lv.slot_cap || cb + nch > Lv.chunk_cap) {
-        atomicOr(B.err, 2);
-        for (int i = 0; i < nch && cb + i < Lv.chunk_cap; ++i) Lv.chunk_slot[cb + i] = -1;
+        if (lane == 0) atomicOr(B.err, 2);
+        for (int i = lane; i < nch && cb + i < Lv.chunk_cap; i += 32) Lv.chunk_slot[cb + i] = -1;
         return;
     }
-    Slot sl;
-    sl.node = node; sl.chunk_base = cb; sl.nchunks = nch; sl.ok = 0;
-    sl.axis = sl.split = sl.k = sl.r = 0;
-    Lv.slots[s] = sl;
-    for (int i = 0; i < kKeys; ++i) Lv.keys[(size_t)s * kKeys + i] = (i % 6) < 3 ? kMinInit : kMaxInit;
-    for (int i = 0; i < kBins; ++i) Lv.cnt[(size_t)s * kBins + i] = 0;
-    for (int i = 0; i < nch; ++i) { Lv.chunk_slot[cb + i] = s; Lv.chunk_k[cb + i] = i; }
+    if (lane == 0) {
+        Slot sl;
+        sl.node = node; sl.chunk_base = cb; sl.nchunks = nch; sl.ok = 0;
+        sl.axis = sl.split = sl.k = sl.r = 0;
+        Lv.slots[s] = sl;
+    }
+    for (int i = lane; i < kKeys; i += 32) {
+        Lv.keys[(size_t)s * kKeys + i] = (i % 6) < 3 ? ~0u : 0u;
+        Lv.zpos[(size_t)s * kKeys + i] = ~0u;
+    }
+    for (int i = lane; i < kBins; i += 32) Lv.cnt[(size_t)s * kBins + i] = 0;
+    for (int i = lane; i < nch; i += 32) { Lv.chunk_slot[cb + i] = s; Lv.chunk_k[cb + i] = i; }
 }
 
-__device__ void route_child(const Build& B, const Level& next, int id) {
-    if (id < 0) return;
-    const int count = B.nodes[id].count;
-    if (count <= 1) return;
-    if (count <= kSmall) {
+// a new child (by a whole warp): the next level, the small list, or nothing for a leaf
+__device__ void route_child(const Build& B, const Level& next, int id, int count) {
+    if (id < 0 || count <= 1) return;
+    if (count > kSmall) {
+        add_slot(next, id, count, B);
+    } else if ((threadIdx.x & 31) == 0) {
         const int i = atomicAdd(B.n_small, 1);
         B.small[i] = id;   // at most one entry per node: n_small < node_cap
-    } else {
-        add_slot(next, id, count, B);
     }
 }
 
@@ -265,7 +278,7 @@ __global__ void __launch_bounds__(kThreads) k_root_keys(Build B, const int2* chu
 
 // root nodes: ids 0 .. n_meshes-1
 __global__ void k_roots(Build B, int n_meshes, const unsigned long long* root_keys, Level L0) {
-    for (int m = blockIdx.x * blockDim.x + threadIdx.x; m < n_meshes; m += gridDim.x * blockDim.x) {
+    for (int m = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; m < n_meshes; m += (gridDim.x * blockDim.x) >> 5) {   // a warp each
         const BuildMesh M = B.meshes[m];
         float b[6];
         for (int i = 0; i < 6; ++i) {
@@ -276,10 +289,8 @@ __global__ void k_roots(Build B, int n_meshes, const unsigned long long* root_ke
         n.start = M.tri_start; n.count = M.tri_count; n.mesh = m; n.depth = 0; n.rturns = 0; n.parent = -1;
         n.side = 0; n.leaf = M.tri_count <= 1; n.rank = -1; n.pad = 0;
         for (int c = 0; c < 3; ++c) { n.bmin[c] = b[c]; n.bmax[c] = b[3 + c]; }
-        B.nodes[m] = n;
-        if (M.tri_count <= 1) continue;
-        if (M.tri_count <= kSmall) B.small[atomicAdd(B.n_small, 1)] = m;
-        else add_slot(L0, m, M.tri_count, B);
+        if ((threadIdx.x & 31) == 0) B.nodes[m] = n;
+        route_child(B, L0, m, M.tri_count);
     }
 }
 
@@ -287,9 +298,12 @@ __global__ void k_roots(Build B, int n_meshes, const unsigned long long* root_ke
 
 // fillBuckets for every axis (src/TriangleMesh.cpp:16-40), one chunk a block.  A thread
 // takes kPer consecutive triangles and folds runs that share a bucket before it
-// touches shared memory.
-__global__ void __launch_bounds__(kThreads) k_level_bins(Build B, Level Lv) {
-    __shared__ unsigned long long sk[kKeys];
+// touches shared memory.  Equal values have equal bits except for zero, so a bin keeps its
+// bounds as 32-bit keys (native minima; 64-bit keys with the position took 19 us a level on
+// 131,072 triangles) and beside them the first position with a zero.
+__global__ void __launch_bounds__(kThreads) k_level_bins(Build B, Level Lv, Level next) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) { *next.n_slots = 0; *next.n_chunks = 0; }   // the level before it is done
+    __shared__ unsigned sk[kKeys], sz[kKeys];
     __shared__ int sc[kBins];
     const int nc = min(*Lv.n_chunks, Lv.chunk_cap), ns = min(*Lv.n_slots, Lv.slot_cap);
     for (int c = blockIdx.x; c < nc; c += gridDim.x) {
@@ -297,17 +311,17 @@ __global__ void __launch_bounds__(kThreads) k_level_bins(Build B, Level Lv) {
         if (si < 0 || si >= ns) continue;
         const Slot sl = Lv.slots[si];
         const BNode nd = B.nodes[sl.node];
-        for (int i = threadIdx.x; i < kKeys; i += blockDim.x) sk[i] = (i % 6) < 3 ? kMinInit : kMaxInit;
+        for (int i = threadIdx.x; i < kKeys; i += blockDim.x) { sk[i] = (i % 6) < 3 ? ~0u : 0u; sz[i] = ~0u; }
         for (int i = threadIdx.x; i < kBins; i += blockDim.x) sc[i] = 0;
         __syncthreads();
         float s[3], len[3];
         for (int a = 0; a < 3; ++a) { s[a] = nd.bmin[a]; len[a] = nd.bmax[a] - nd.bmin[a]; }
         const int base = nd.start + Lv.chunk_k[c] * kChunk, end = nd.start + nd.count;
         int cur[3] = {-1, -1, -1}, n[3] = {0, 0, 0};
-        unsigned long long k[3][6];
+        unsigned k[3][6];
         auto flush = [&](int a) {
             if (!n[a]) return;
-            unsigned long long* d = sk + (a * kBk + cur[a]) * 6;
+            unsigned* d = sk + (a * kBk + cur[a]) * 6;
             for (int i = 0; i < 3; ++i) atomicMin(&d[i], k[a][i]);
             for (int i = 3; i < 6; ++i) atomicMax(&d[i], k[a][i]);
             atomicAdd(&sc[a * kBk + cur[a]], n[a]);
@@ -316,16 +330,18 @@ __global__ void __launch_bounds__(kThreads) k_level_bins(Build B, Level Lv) {
             const int p = base + threadIdx.x * kPer + j;
             if (p >= end) break;
             const TriDev t = B.tri[B.perm[p]];
-            unsigned long long kv[6];
-            for (int i = 0; i < 3; ++i) kv[i] = kmin(comp(t, i), p);
-            for (int i = 3; i < 6; ++i) kv[i] = kmax(comp(t, i), p);
+            unsigned kv[6];
+            bool zero = false;
+            for (int i = 0; i < 6; ++i) { kv[i] = ord_fkey(comp(t, i)); zero |= comp(t, i) == 0.f; }
             for (int a = 0; a < 3; ++a) {
                 if (!len[a]) continue;
                 const int bi = bucket_of(cen(t, a), s[a], len[a]);
+                if (zero)
+                    for (int i = 0; i < 6; ++i) if (comp(t, i) == 0.f) atomicMin(&sz[(a * kBk + bi) * 6 + i], (unsigned)p);
                 if (bi != cur[a]) {
                     flush(a);
                     cur[a] = bi; n[a] = 0;
-                    for (int i = 0; i < 6; ++i) k[a][i] = i < 3 ? kMinInit : kMaxInit;
+                    for (int i = 0; i < 6; ++i) k[a][i] = i < 3 ? ~0u : 0u;
                 }
                 for (int i = 0; i < 3; ++i) k[a][i] = min(k[a][i], kv[i]);
                 for (int i = 3; i < 6; ++i) k[a][i] = max(k[a][i], kv[i]);
@@ -336,9 +352,10 @@ __global__ void __launch_bounds__(kThreads) k_level_bins(Build B, Level Lv) {
         __syncthreads();
         const size_t so = (size_t)si;
         for (int i = threadIdx.x; i < kKeys; i += blockDim.x) {
-            const unsigned long long v = sk[i];
-            if ((i % 6) < 3) { if (v != kMinInit) atomicMin(&Lv.keys[so * kKeys + i], v); }
-            else if (v != kMaxInit) atomicMax(&Lv.keys[so * kKeys + i], v);
+            const unsigned v = sk[i];
+            if ((i % 6) < 3) { if (v != ~0u) atomicMin(&Lv.keys[so * kKeys + i], v); }
+            else if (v) atomicMax(&Lv.keys[so * kKeys + i], v);
+            if (sz[i] != ~0u) atomicMin(&Lv.zpos[so * kKeys + i], sz[i]);
         }
         for (int i = threadIdx.x; i < kBins; i += blockDim.x)
             if (sc[i]) atomicAdd(&Lv.cnt[so * kBins + i], sc[i]);
@@ -362,8 +379,9 @@ __global__ void __launch_bounds__(32 * kChooseWarps) k_level_choose(Build B, Lev
         for (int i = lane; i < kKeys; i += 32) {
             const int c = i % 6;
             if (!scnt[wi][i / 6]) { sval[wi][i] = c < 3 ? FLT_MAX : -FLT_MAX; continue; }
-            const unsigned long long k = Lv.keys[(size_t)s * kKeys + i];
-            sval[wi][i] = comp(B.tri[B.perm[c < 3 ? kpos_min(k) : kpos_max(k)]], c);
+            float v = key_float(Lv.keys[(size_t)s * kKeys + i]);
+            if (v == 0.f) v = comp(B.tri[B.perm[Lv.zpos[(size_t)s * kKeys + i]]], c);   // +0 or -0, whichever came first
+            sval[wi][i] = v;
         }
         __syncwarp();
         const float nb[6] = {nd.bmin[0], nd.bmin[1], nd.bmin[2], nd.bmax[0], nd.bmax[1], nd.bmax[2]};
@@ -372,13 +390,16 @@ __global__ void __launch_bounds__(32 * kChooseWarps) k_level_choose(Build B, Lev
         const int pick = warp_choose(sval[wi], scnt[wi], nb, L, R, cl, cr);
         if (pick < 0) {
             if (lane == 0) B.nodes[sl.node].leaf = 1;
-        } else if (lane == pick) {
-            sl.ok = 1; sl.axis = pick / (kBk - 1); sl.split = pick % (kBk - 1) + 1; sl.k = cl;
-            Lv.slots[s] = sl;
-            const int l = new_node(B, nd.start, cl, nd.mesh, nd.depth + 1, nd.rturns, sl.node, 0, L);
-            const int r = new_node(B, nd.start + cl, cr, nd.mesh, nd.depth + 1, nd.rturns + 1, sl.node, 1, R);
-            route_child(B, next, l);
-            route_child(B, next, r);
+        } else {
+            int l = -1, r = -1;
+            if (lane == pick) {
+                sl.ok = 1; sl.axis = pick / (kBk - 1); sl.split = pick % (kBk - 1) + 1; sl.k = cl;
+                Lv.slots[s] = sl;
+                l = new_node(B, nd.start, cl, nd.mesh, nd.depth + 1, nd.rturns, sl.node, 0, L);
+                r = new_node(B, nd.start + cl, cr, nd.mesh, nd.depth + 1, nd.rturns + 1, sl.node, 1, R);
+            }
+            route_child(B, next, __shfl_sync(~0u, l, pick), __shfl_sync(~0u, cl, pick));
+            route_child(B, next, __shfl_sync(~0u, r, pick), __shfl_sync(~0u, cr, pick));
         }
         __syncwarp();
     }
@@ -414,24 +435,6 @@ __global__ void __launch_bounds__(kThreads) k_level_count(Build B, Level Lv) {
     }
 }
 
-// per split node: chunk offsets in position order, and r
-__global__ void k_level_scan(Level Lv, int* err) {
-    const int ns = min(*Lv.n_slots, Lv.slot_cap);
-    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < ns; s += gridDim.x * blockDim.x) {
-        Slot sl = Lv.slots[s];
-        if (!sl.ok) continue;
-        int a = 0, b = 0;
-        for (int i = 0; i < sl.nchunks; ++i) {
-            const int2 v = Lv.chunk_cnt[sl.chunk_base + i];
-            Lv.chunk_off[sl.chunk_base + i] = make_int2(a, b);
-            a += v.x; b += v.y;
-        }
-        sl.r = a;
-        if (a != b) { sl.ok = 0; atomicOr(err, 16); }   // cannot happen: both count the misplaced pairs
-        Lv.slots[s] = sl;
-    }
-}
-
 // block-wide exclusive scan of one int per thread
 __device__ __forceinline__ int block_excl(int v, int* sh, int& total) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -457,9 +460,12 @@ __device__ __forceinline__ int block_excl(int v, int* sh, int& total) {
     return r;
 }
 
-// ranks: fr / bl hold positions (relative to the node) by rank
+// ranks: fr / bl hold positions (relative to the node) by rank.  A chunk's offset is the sum
+// of the node's counts before it, formed by its block; the first chunk's block also leaves
+// the node's r.
 __global__ void __launch_bounds__(kThreads) k_level_rank(Build B, Level Lv) {
     __shared__ int sh[kThreads / 32];
+    __shared__ int2 s_off, s_all;
     const int nc = min(*Lv.n_chunks, Lv.chunk_cap), ns = min(*Lv.n_slots, Lv.slot_cap);
     for (int c = blockIdx.x; c < nc; c += gridDim.x) {
         const int si = Lv.chunk_slot[c];
@@ -467,8 +473,28 @@ __global__ void __launch_bounds__(kThreads) k_level_rank(Build B, Level Lv) {
         const Slot sl = Lv.slots[si];
         if (!sl.ok) continue;
         const BNode nd = B.nodes[sl.node];
-        const int2 off = Lv.chunk_off[c];
-        const int base = nd.start + Lv.chunk_k[c] * kChunk, end = min(base + kChunk, nd.start + nd.count);
+        if (threadIdx.x == 0) { s_off = make_int2(0, 0); s_all = make_int2(0, 0); }
+        __syncthreads();
+        const int ck = Lv.chunk_k[c];
+        {
+            int2 o = make_int2(0, 0), all = o;
+            for (int i = threadIdx.x; i < sl.nchunks; i += blockDim.x) {
+                const int2 v = Lv.chunk_cnt[sl.chunk_base + i];
+                all.x += v.x; all.y += v.y;
+                if (i < ck) { o.x += v.x; o.y += v.y; }
+            }
+            if (all.x | all.y) {
+                atomicAdd(&s_off.x, o.x); atomicAdd(&s_off.y, o.y);
+                atomicAdd(&s_all.x, all.x); atomicAdd(&s_all.y, all.y);
+            }
+        }
+        __syncthreads();
+        const int2 off = s_off;
+        if (ck == 0 && threadIdx.x == 0) {
+            Lv.slots[si].r = s_all.x;
+            if (s_all.x != s_all.y) atomicOr(B.err, 16);   // cannot happen: both count the misplaced pairs
+        }
+        const int base = nd.start + ck * kChunk, end = min(base + kChunk, nd.start + nd.count);
         const int p0 = base + threadIdx.x * kPer;
         int nfr = 0, nbl = 0;
         for (int j = 0; j < kPer; ++j) {
@@ -537,58 +563,105 @@ __global__ void k_level_copy(Build B, Level Lv) {
 
 // ---------------------------------------------------------------- small subtrees
 
+constexpr int kNodeWords = sizeof(BNode) / 4;
 struct WarpSmem {
-    unsigned long long key[kKeys];
-    int cnt[kBins];
+    float tri[9][kSmall];        // the subtree's triangles (bounds, centroid) in their order at its root
+    int orig[kSmall];            // their indices
+    BNode stack[kSmall];         // nodes to split
+    int stack_id[kSmall];
+    unsigned key[kKeys];
     float val[kKeys];
-    int fr[kSmall], bl[kSmall], stage[kSmall], stack[kSmall];
-    int choice[6];   // ok, axis, split, cl, left id, right id
+    int cnt[kBins];
+    unsigned char ord[kSmall], stage[kSmall], fr[kSmall], bl[kSmall];   // position -> triangle; partition
+    int choice[4];               // ok, axis, split, cl
     float lr[12];
 };
 
-// One warp builds the subtree of a node of at most kSmall triangles (two per lane),
-// depth first with a stack in shared memory.
+// One warp builds the subtree of a node of at most kSmall triangles (two per lane), depth
+// first.  A split is a chain of dependent steps, so everything it reads lies in shared
+// memory: the triangles are loaded once, nodes wait on a stack with their bounds, and node
+// ids come from one reservation per subtree (those left over are marked by mesh -1).  The
+// bins are 32-bit minima of the values; which of +0 and -0 came first in the node's order
+// is looked up only where a bin's bound is zero.  With 64-bit (value, position) minima in
+// shared memory, which are compare-and-swap loops, and triangles and nodes in global
+// memory, 131,072 triangles took 455 us here.
 __global__ void __launch_bounds__(32 * kWarpsSmall) k_small_subtrees(Build B) {
     __shared__ WarpSmem smem[kWarpsSmall];
     WarpSmem& S = smem[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
+    const unsigned below = (1u << lane) - 1u;
     const int warps = gridDim.x * kWarpsSmall;
     const int n_small = *B.n_small;
     for (int w = blockIdx.x * kWarpsSmall + (threadIdx.x >> 5); w < n_small; w += warps) {
-        if (lane == 0) S.stack[0] = B.small[w];
-        int top = 1;
+        const int root = B.small[w];
+        const int start0 = B.nodes[root].start, n0 = B.nodes[root].count;
+        if (lane < kNodeWords) reinterpret_cast<int*>(&S.stack[0])[lane] = reinterpret_cast<const int*>(&B.nodes[root])[lane];
+        int base = 0;
+        if (lane == 0) {
+            S.stack_id[0] = root;
+            base = atomicAdd(B.n_nodes, 2 * (n0 - 1));
+            if (base + 2 * (n0 - 1) > B.node_cap) { atomicOr(B.err, 1); base = -1; }
+        }
+        base = __shfl_sync(~0u, base, 0);
+        for (int x = lane; x < n0; x += 32) {
+            const int o = B.perm[start0 + x];
+            const TriDev t = B.tri[o];
+            for (int c = 0; c < 6; ++c) S.tri[c][x] = comp(t, c);
+            for (int c = 0; c < 3; ++c) S.tri[6 + c][x] = cen(t, c);
+            S.orig[x] = o;
+            S.ord[x] = (unsigned char)x;
+        }
         __syncwarp();
+        if (base < 0) continue;
+        int top = 1, used = 0;
         while (top > 0) {
-            const int id = S.stack[--top];
-            __syncwarp();
-            const BNode nd = B.nodes[id];
-            for (int i = lane; i < kKeys; i += 32) S.key[i] = (i % 6) < 3 ? kMinInit : kMaxInit;
+            --top;
+            const BNode nd = S.stack[top];
+            const int id = S.stack_id[top], ls = nd.start - start0, n = nd.count;
+            for (int i = lane; i < kKeys; i += 32) S.key[i] = (i % 6) < 3 ? ~0u : 0u;
             if (lane < kBins) S.cnt[lane] = 0;
             __syncwarp();
             float s[3], len[3];
             for (int a = 0; a < 3; ++a) { s[a] = nd.bmin[a]; len[a] = nd.bmax[a] - nd.bmin[a]; }
-            int pos[2], orig[2];
+            int tr[2], bin[2][3];
+#pragma unroll
             for (int j = 0; j < 2; ++j) {
                 const int x = lane + 32 * j;
-                pos[j] = nd.start + x;
-                orig[j] = x < nd.count ? B.perm[pos[j]] : -1;
-                if (orig[j] < 0) continue;
-                const TriDev t = B.tri[orig[j]];
+                tr[j] = x < n ? S.ord[ls + x] : -1;
+#pragma unroll
+                for (int a = 0; a < 3; ++a) bin[j][a] = -1;
+                if (tr[j] < 0) continue;
+                unsigned key[6];
+#pragma unroll
+                for (int c = 0; c < 6; ++c) key[c] = ord_fkey(S.tri[c][tr[j]]);
+#pragma unroll
                 for (int a = 0; a < 3; ++a) {
                     if (!len[a]) continue;
-                    const int bi = bucket_of(cen(t, a), s[a], len[a]);
-                    unsigned long long* k = S.key + (a * kBk + bi) * 6;
-                    for (int i = 0; i < 3; ++i) atomicMin(&k[i], kmin(comp(t, i), pos[j]));
-                    for (int i = 3; i < 6; ++i) atomicMax(&k[i], kmax(comp(t, i), pos[j]));
-                    atomicAdd(&S.cnt[a * kBk + bi], 1);
+                    const int bi = a * kBk + bucket_of(S.tri[6 + a][tr[j]], s[a], len[a]);
+                    bin[j][a] = bi;
+                    for (int c = 0; c < 3; ++c) atomicMin(&S.key[bi * 6 + c], key[c]);
+                    for (int c = 3; c < 6; ++c) atomicMax(&S.key[bi * 6 + c], key[c]);
+                    atomicAdd(&S.cnt[bi], 1);
                 }
             }
             __syncwarp();
-            for (int i = lane; i < kKeys; i += 32) {
-                const int c = i % 6;
-                if (!S.cnt[i / 6]) { S.val[i] = c < 3 ? FLT_MAX : -FLT_MAX; continue; }
-                const unsigned long long k = S.key[i];
-                S.val[i] = comp(B.tri[B.perm[c < 3 ? kpos_min(k) : kpos_max(k)]], c);
+            for (int i0 = 0; i0 < kKeys; i0 += 32) {
+                const int i = i0 + lane, c = i % 6;
+                const bool in = i < kKeys;
+                float v = c < 3 ? FLT_MAX : -FLT_MAX;
+                if (in && S.cnt[i / 6]) v = key_float(S.key[i]);
+                if (in) S.val[i] = v;
+                // a bound of zero: the sign of the first triangle, in the node's order, that has it
+                for (unsigned zeros = __ballot_sync(~0u, in && v == 0.f); zeros; zeros &= zeros - 1) {
+                    const int zi = i0 + __ffs(zeros) - 1, zb = zi / 6, za = zb / kBk, zc = zi % 6;
+                    for (int j = 0; j < 2; ++j) {
+                        const bool at = bin[j][za] == zb && S.tri[zc][max(tr[j], 0)] == 0.f;
+                        const unsigned who = __ballot_sync(~0u, at);
+                        if (!who) continue;
+                        if (lane == __ffs(who) - 1) S.val[zi] = S.tri[zc][tr[j]];
+                        break;
+                    }
+                }
             }
             __syncwarp();
             {
@@ -609,11 +682,10 @@ __global__ void __launch_bounds__(32 * kWarpsSmall) k_small_subtrees(Build B) {
             bool left[2], fr[2], bl[2];
             for (int j = 0; j < 2; ++j) {
                 const int x = lane + 32 * j;
-                left[j] = orig[j] >= 0 && goes_left(cen(B.tri[orig[j]], axis), s[axis], len[axis], split);
-                fr[j] = orig[j] >= 0 && x < k && !left[j];
-                bl[j] = orig[j] >= 0 && x >= k && left[j];
+                left[j] = tr[j] >= 0 && goes_left(S.tri[6 + axis][max(tr[j], 0)], s[axis], len[axis], split);
+                fr[j] = tr[j] >= 0 && x < k && !left[j];
+                bl[j] = tr[j] >= 0 && x >= k && left[j];
             }
-            const unsigned below = (1u << lane) - 1u;
             const unsigned mfr0 = __ballot_sync(0xffffffffu, fr[0]), mfr1 = __ballot_sync(0xffffffffu, fr[1]);
             const unsigned mbl0 = __ballot_sync(0xffffffffu, bl[0]), mbl1 = __ballot_sync(0xffffffffu, bl[1]);
             int rk[2];
@@ -621,38 +693,47 @@ __global__ void __launch_bounds__(32 * kWarpsSmall) k_small_subtrees(Build B) {
             rk[1] = fr[1] ? __popc(mfr0) + __popc(mfr1 & below) : __popc(mbl0) + __popc(mbl1 & below);
             const int r = __popc(mfr0) + __popc(mfr1);
             for (int j = 0; j < 2; ++j) {
-                if (fr[j]) S.fr[rk[j]] = lane + 32 * j;
-                if (bl[j]) S.bl[rk[j]] = lane + 32 * j;
+                if (fr[j]) S.fr[rk[j]] = (unsigned char)(lane + 32 * j);
+                if (bl[j]) S.bl[rk[j]] = (unsigned char)(lane + 32 * j);
             }
             __syncwarp();
-            const int n = nd.count;
             for (int j = 0; j < 2; ++j) {
-                if (orig[j] < 0) continue;
+                if (tr[j] < 0) continue;
                 const int x = lane + 32 * j;
                 int dest;
                 if (x < k) dest = left[j] ? x : (rk[j] == 0 ? n : S.bl[r - rk[j]]) - 1;
                 else if (left[j]) dest = S.fr[r - 1 - rk[j]];
                 else dest = x == k ? (r ? S.bl[0] : n) - 1 : x - 1;
                 if (dest < 0 || dest >= n) { atomicOr(B.err, 32); continue; }
-                S.stage[dest] = orig[j];
+                S.stage[dest] = (unsigned char)tr[j];
             }
             __syncwarp();
-            for (int j = 0; j < 2; ++j) {
-                const int x = lane + 32 * j;
-                if (x < n) B.perm[nd.start + x] = S.stage[x];
+            for (int x = lane; x < n; x += 32) S.ord[ls + x] = S.stage[x];
+            // children: to the node array, and onto the stack when they hold more than one triangle
+            // (at most one entry per pending leaf: the stack never outgrows kSmall)
+            for (int side = 0; side < 2; ++side) {
+                const int cid = base + used + side, cn = side ? n - k : k;
+                BNode& ch = S.stack[top];
+                if (lane == 0) {
+                    ch.start = side ? nd.start + k : nd.start; ch.count = cn; ch.mesh = nd.mesh; ch.depth = nd.depth + 1;
+                    ch.rturns = nd.rturns + side; ch.parent = id; ch.side = side; ch.leaf = cn <= 1; ch.rank = -1; ch.pad = 0;
+                    for (int c = 0; c < 3; ++c) { ch.bmin[c] = S.lr[6 * side + c]; ch.bmax[c] = S.lr[6 * side + 3 + c]; }
+                    S.stack_id[top] = cid;
+                }
+                __syncwarp();
+                if (lane < kNodeWords) reinterpret_cast<int*>(&B.nodes[cid])[lane] = reinterpret_cast<const int*>(&ch)[lane];
+                __syncwarp();
+                if (cn > 1 && top < kSmall - 1) ++top;
             }
-            if (lane == 0) {
-                const int l = new_node(B, nd.start, k, nd.mesh, nd.depth + 1, nd.rturns, id, 0, S.lr);
-                const int rr = new_node(B, nd.start + k, n - k, nd.mesh, nd.depth + 1, nd.rturns + 1, id, 1, S.lr + 6);
-                S.choice[4] = l; S.choice[5] = rr;
-            }
-            __syncwarp();
-            const int l = S.choice[4], rr = S.choice[5];
-            // at most one stack entry per pending leaf: the stack never outgrows kSmall
-            if (l >= 0 && k > 1 && top < kSmall) { if (lane == 0) S.stack[top] = l; ++top; }
-            if (rr >= 0 && n - k > 1 && top < kSmall) { if (lane == 0) S.stack[top] = rr; ++top; }
-            __syncwarp();
+            used += 2;
         }
+        __syncwarp();
+        for (int x = lane; x < n0; x += 32) B.perm[start0 + x] = S.orig[S.ord[x]];
+        for (int i = used + lane; i < 2 * (n0 - 1); i += 32) {   // ids left over
+            B.nodes[base + i].mesh = -1;
+            B.nodes[base + i].leaf = 0;
+        }
+        __syncwarp();
     }
 }
 
@@ -668,7 +749,7 @@ __global__ void k_node_ranks(Build B) {
     const int n = min(*B.n_nodes, B.node_cap);
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const BNode nd = B.nodes[i];
-        if (nd.leaf) continue;
+        if (nd.leaf || nd.mesh < 0) continue;
         const int ms = B.meshes[nd.mesh].tri_start;
         B.nodes[i].rank = nd.depth + (B.lb[nd.start] - B.lb[ms]) - nd.rturns;
     }
@@ -678,6 +759,7 @@ __global__ void k_emit_nodes(Build B, TriNodeDev* out) {
     const int n = min(*B.n_nodes, B.node_cap);
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const BNode nd = B.nodes[i];
+        if (nd.mesh < 0) continue;
         const BuildMesh M = B.meshes[nd.mesh];
         const int id = nd.parent < 0 ? 0 : 2 * B.nodes[nd.parent].rank + 1 + nd.side;
         if (id < 0 || id >= max(1, 2 * M.tri_count - 1)) { atomicOr(B.err, 64); continue; }
@@ -706,17 +788,24 @@ __global__ void k_emit_tris(Build B, TriDev* out) {
 
 // ---------------------------------------------------------------- host
 
+// The build's device buffers in one allocation: add() every buffer, alloc() once.  (Some
+// forty cudaMalloc and cudaFree calls took 0.7 ms, whatever the mesh's size.)
 struct MeshBuildScratch {
-    std::vector<void*> ptrs;
+    std::vector<std::pair<void**, size_t>> want;
+    size_t bytes = 0;
+    char* mem = nullptr;
     template <class T>
-    cudaError_t get(T*& p, size_t n) {
-        void* q = nullptr;
-        cudaError_t e = cudaMalloc(&q, std::max<size_t>(1, n) * sizeof(T));
-        if (e == cudaSuccess) ptrs.push_back(q);
-        p = (T*)q;
+    void add(T*& p, size_t n) {
+        want.emplace_back(reinterpret_cast<void**>(&p), bytes);
+        bytes += (std::max<size_t>(1, n) * sizeof(T) + 255) / 256 * 256;
+    }
+    cudaError_t alloc() {
+        const cudaError_t e = cudaMalloc(&mem, bytes);
+        if (e == cudaSuccess)
+            for (auto& w : want) *w.first = mem + w.second;
         return e;
     }
-    ~MeshBuildScratch() { for (void* q : ptrs) cudaFree(q); }
+    ~MeshBuildScratch() { if (mem) cudaFree(mem); }
 };
 
 cudaError_t build_mesh_bvhs(const float4* verts, const int4* idx, const std::vector<BuildMesh>& meshes, TriDev* tris_out,
@@ -763,27 +852,54 @@ cudaError_t build_mesh_bvhs(const float4* verts, const int4* idx, const std::vec
     for (const BuildMesh& m : work) total += m.tri_count;
     B.node_cap = 2 * total + nm;
     BuildMesh* d_meshes;
-    MB_TRY(S.get(d_meshes, nm));
-    MB_TRY(cudaMemcpyAsync(d_meshes, work.data(), sizeof(BuildMesh) * nm, cudaMemcpyHostToDevice, st));
-    B.meshes = d_meshes;
-    MB_TRY(S.get(B.tri, n_tris));
-    MB_TRY(S.get(B.perm, n_tris));
-    MB_TRY(S.get(B.perm_tmp, n_tris));
-    MB_TRY(S.get(B.lab, n_tris));
-    MB_TRY(S.get(B.rnk, n_tris));
-    MB_TRY(S.get(B.fr, n_tris));
-    MB_TRY(S.get(B.bl, n_tris));
-    MB_TRY(S.get(B.nodes, B.node_cap));
-    MB_TRY(S.get(B.n_nodes, 1));
-    MB_TRY(S.get(B.small, B.node_cap));
-    MB_TRY(S.get(B.n_small, 1));
-    MB_TRY(S.get(B.mark, n_tris + 1));
-    MB_TRY(S.get(B.lb, n_tris + 1));
-    MB_TRY(S.get(B.err, 1));
+    S.add(d_meshes, nm);
+    S.add(B.tri, n_tris);
+    S.add(B.perm, n_tris);
+    S.add(B.perm_tmp, n_tris);
+    S.add(B.lab, n_tris);
+    S.add(B.rnk, n_tris);
+    S.add(B.fr, n_tris);
+    S.add(B.bl, n_tris);
+    S.add(B.nodes, B.node_cap);
+    S.add(B.n_nodes, 1);
+    S.add(B.small, B.node_cap);
+    S.add(B.n_small, 1);
+    S.add(B.mark, n_tris + 1);
+    S.add(B.lb, n_tris + 1);
+    S.add(B.err, 1);
     int* d_total;
-    MB_TRY(S.get(d_total, 1));
+    S.add(d_total, 1);
     int* scratch;
-    MB_TRY(S.get(scratch, scan_scratch_ints(n_tris + 1)));
+    S.add(scratch, scan_scratch_ints(n_tris + 1));
+    Level L[2];
+    const int slot_cap = total / kSmall + nm + 1;
+    const int chunk_cap = slot_cap + total / kChunk + 1;
+    for (Level& v : L) {
+        v.slot_cap = slot_cap;
+        v.chunk_cap = chunk_cap;
+        S.add(v.slots, slot_cap);
+        S.add(v.n_slots, 1);
+        S.add(v.keys, (size_t)slot_cap * kKeys);
+        S.add(v.zpos, (size_t)slot_cap * kKeys);
+        S.add(v.cnt, (size_t)slot_cap * kBins);
+        S.add(v.chunk_slot, chunk_cap);
+        S.add(v.chunk_k, chunk_cap);
+        S.add(v.n_chunks, 1);
+        S.add(v.chunk_cnt, chunk_cap);
+    }
+    // roots: bounds over each mesh's triangles in their original order
+    std::vector<int2> rc;
+    for (int m = 0; m < nm; ++m)
+        for (int c = 0; c * kChunk < work[m].tri_count; ++c) rc.push_back(make_int2(m, c));
+    int2* d_rc;
+    unsigned long long* d_rk;
+    int* d_mesh_nodes;
+    S.add(d_rc, rc.size());
+    S.add(d_rk, (size_t)nm * 6);
+    S.add(d_mesh_nodes, nm);
+    MB_TRY(S.alloc());
+    B.meshes = d_meshes;
+    MB_TRY(cudaMemcpyAsync(d_meshes, work.data(), sizeof(BuildMesh) * nm, cudaMemcpyHostToDevice, st));
     MB_TRY(cudaMemsetAsync(B.n_nodes, 0, sizeof(int), st));
     MB_TRY(cudaMemsetAsync(B.n_small, 0, sizeof(int), st));
     MB_TRY(cudaMemsetAsync(B.err, 0, sizeof(int), st));
@@ -791,77 +907,49 @@ cudaError_t build_mesh_bvhs(const float4* verts, const int4* idx, const std::vec
     // root nodes take ids 0 .. nm-1
     MB_TRY(cudaMemcpyAsync(B.n_nodes, &nm, sizeof(int), cudaMemcpyHostToDevice, st));
 
-    Level L[2];
-    const int slot_cap = total / kSmall + nm + 1;
-    const int chunk_cap = slot_cap + total / kChunk + 1;
     for (Level& v : L) {
-        v.slot_cap = slot_cap;
-        v.chunk_cap = chunk_cap;
-        MB_TRY(S.get(v.slots, slot_cap));
-        MB_TRY(S.get(v.n_slots, 1));
-        MB_TRY(S.get(v.keys, (size_t)slot_cap * kKeys));
-        MB_TRY(S.get(v.cnt, (size_t)slot_cap * kBins));
-        MB_TRY(S.get(v.chunk_slot, chunk_cap));
-        MB_TRY(S.get(v.chunk_k, chunk_cap));
-        MB_TRY(S.get(v.n_chunks, 1));
-        MB_TRY(S.get(v.chunk_cnt, chunk_cap));
-        MB_TRY(S.get(v.chunk_off, chunk_cap));
         MB_TRY(cudaMemsetAsync(v.n_slots, 0, sizeof(int), st));
         MB_TRY(cudaMemsetAsync(v.n_chunks, 0, sizeof(int), st));
     }
 
     const int grid = 152 * 4;
     k_tri_setup<<<grid, 256, 0, st>>>(B);
-    // roots: bounds over each mesh's triangles in their original order
-    std::vector<int2> rc;
-    for (int m = 0; m < nm; ++m)
-        for (int c = 0; c * kChunk < work[m].tri_count; ++c) rc.push_back(make_int2(m, c));
-    int2* d_rc;
-    unsigned long long* d_rk;
-    MB_TRY(S.get(d_rc, rc.size()));
-    MB_TRY(S.get(d_rk, (size_t)nm * 6));
     MB_TRY(cudaMemcpyAsync(d_rc, rc.data(), sizeof(int2) * rc.size(), cudaMemcpyHostToDevice, st));
-    {
-        std::vector<unsigned long long> init((size_t)nm * 6);
-        for (size_t i = 0; i < init.size(); ++i) init[i] = (i % 6) < 3 ? kMinInit : kMaxInit;
-        MB_TRY(cudaMemcpyAsync(d_rk, init.data(), sizeof(unsigned long long) * init.size(), cudaMemcpyHostToDevice, st));
-        k_root_keys<<<std::min<int>(grid, (int)rc.size()), kThreads, 0, st>>>(B, d_rc, (int)rc.size(), d_rk);
-        k_roots<<<(nm + 127) / 128, 128, 0, st>>>(B, nm, d_rk, L[0]);
-        MB_TRY(cudaStreamSynchronize(st));   // the host vectors above go out of scope
-    }
-    // top levels
-    int* h_cnt = nullptr;
-    MB_TRY(cudaMallocHost(&h_cnt, sizeof(int)));
-    cudaError_t le = cudaSuccess;
-    // every level lowers the largest remaining node by at least one triangle
+    std::vector<unsigned long long> init((size_t)nm * 6);   // (lives, as rc does, until the levels' first wait)
+    for (size_t i = 0; i < init.size(); ++i) init[i] = (i % 6) < 3 ? kMinInit : kMaxInit;
+    MB_TRY(cudaMemcpyAsync(d_rk, init.data(), sizeof(unsigned long long) * init.size(), cudaMemcpyHostToDevice, st));
+    k_root_keys<<<std::min<int>(grid, (int)rc.size()), kThreads, 0, st>>>(B, d_rc, (int)rc.size(), d_rk);
+    k_roots<<<(nm + 3) / 4, 128, 0, st>>>(B, nm, d_rk, L[0]);
+    // Top levels.  A split at best halves a node, so the first levels cannot be the last and
+    // are queued without asking; after them the host reads whether a level has nodes.
+    int sure = 0, largest = 0;
+    for (const BuildMesh& m : work) largest = std::max(largest, m.tri_count);
+    while (((long long)kSmall << sure) < largest) ++sure;
     bool done = false;
+    // every level lowers the largest remaining node by at least one triangle
     for (int lv = 0; lv <= total; ++lv) {
         Level& cur = L[lv & 1];
         Level& nxt = L[(lv + 1) & 1];
-        cudaMemcpyAsync(h_cnt, cur.n_slots, sizeof(int), cudaMemcpyDeviceToHost, st);
-        le = cudaStreamSynchronize(st);
-        if (le != cudaSuccess) break;
-        if (*h_cnt == 0) { done = true; break; }
-        k_level_bins<<<grid, kThreads, 0, st>>>(B, cur);
-        k_level_choose<<<(std::min(*h_cnt, slot_cap) + kChooseWarps - 1) / kChooseWarps, 32 * kChooseWarps, 0, st>>>(B, cur, nxt);
+        int nodes = lv < 31 ? (int)std::min<long long>((long long)nm << lv, slot_cap) : slot_cap;
+        if (lv >= sure) {
+            MB_TRY(cudaMemcpyAsync(&nodes, cur.n_slots, sizeof(int), cudaMemcpyDeviceToHost, st));
+            MB_TRY(cudaStreamSynchronize(st));
+            if (nodes == 0) { done = true; break; }
+            nodes = std::min(nodes, slot_cap);
+        }
+        k_level_bins<<<grid, kThreads, 0, st>>>(B, cur, nxt);
+        k_level_choose<<<(nodes + kChooseWarps - 1) / kChooseWarps, 32 * kChooseWarps, 0, st>>>(B, cur, nxt);
         k_level_count<<<grid, kThreads, 0, st>>>(B, cur);
-        k_level_scan<<<(std::min(*h_cnt, slot_cap) + 127) / 128, 128, 0, st>>>(cur, B.err);
         k_level_rank<<<grid, kThreads, 0, st>>>(B, cur);
         k_level_scatter<<<grid, kThreads, 0, st>>>(B, cur);
         k_level_copy<<<grid, kThreads, 0, st>>>(B, cur);
-        cudaMemsetAsync(cur.n_slots, 0, sizeof(int), st);
-        cudaMemsetAsync(cur.n_chunks, 0, sizeof(int), st);
     }
-    cudaFreeHost(h_cnt);
-    MB_TRY(le);
     if (!done) { *err_out = 4; return cudaSuccess; }
     k_small_subtrees<<<grid * 2, 32 * kWarpsSmall, 0, st>>>(B);
     // node ids
     k_leaf_marks<<<grid, 256, 0, st>>>(B);
     scan_exclusive(B.mark, B.lb, n_tris + 1, d_total, scratch, st);
     k_node_ranks<<<grid, 256, 0, st>>>(B);
-    int* d_mesh_nodes;
-    MB_TRY(S.get(d_mesh_nodes, nm));
     k_emit_nodes<<<grid, 256, 0, st>>>(B, nodes_out);
     k_mesh_node_counts<<<(nm + 127) / 128, 128, 0, st>>>(B, nm, d_mesh_nodes);
     k_emit_tris<<<grid, 256, 0, st>>>(B, tris_out);
