@@ -466,42 +466,75 @@ __device__ inline int collision_one(const World& w, V3 pos0, Q4 or0, GeomD g0, V
     return collideAnalytic(pos0, or0, g0, pos1, or1, g1, ms[0], err) ? 1 : 0;
 }
 
-// Scene::overlapWithMinTranslationalDistance (src/Physecs.cpp:653-688): every collider
-// whose bounds meet the query shape's; for each manifold with points of the collision
-// (collider first, shape second) its normal and the deepest point, max(0, max over the
-// points of dot(p0 - p1, n)).  Up to cap records a query: {world collider, n xyz, mtd}.
-// The MTD query of overlapWithMinTranslationalDistance: every collider of scene s whose
-// bounds meet the shape's, collided with the collider first; fn(collider, manifold, mtd)
-// for each manifold with points, mtd = max(0, deepest dot(p0 - p1, normal)).  The walk
-// visits the scene's tree left first.
+// The MTD query of Scene::overlapWithMinTranslationalDistance (src/Physecs.cpp:653-688):
+// every collider of scene s whose bounds meet the shape's, collided with the collider
+// first; fn(collider, normal, mtd, triangle) for each manifold with points, mtd = max(0,
+// deepest dot(p0 - p1, normal)), in the order of a walk of the scene's tree left first.
 // self_body (>= 0): a body whose colliders are posed at self_pos instead of its stored
 // position, while their bounds stay the stored ones (a character controller's entity,
 // moved in the registry but not yet patched).
-template <class F>
+//
+// WARP: a warp asks one query.  All lanes take the same walk; the colliders it reaches are
+// collided up to 32 at a time, one a lane, and their manifolds come out in the walk's order
+// (fn is called by all lanes with the same values).  Otherwise a thread asks one.
+template <bool WARP, class F>
 __device__ void for_each_mtd(const World& w, const FrameBuf& f, int s, V3 pos, Q4 ori, const GeomD& g, ManifoldL* ms,
                              TCI* cand, Polytope& poly, F&& fn, int self_body = -1, V3 self_pos = V3{0.f, 0.f, 0.f}) {
     const Bounds b = getBounds(w, pos, ori, g);
     const float4 qmin = make_float4(b.min.x, b.min.y, b.min.z, 0.f), qmax = make_float4(b.max.x, b.max.y, b.max.z, 0.f);
     const int cs = w.scene_col[s], nc = w.scene_col[s + 1] - cs;
-    auto leaf = [&](int q) {
-        const int c = f.order[q];
-        if (!boxes_meet(qmin, qmax, w.aabb_min[c], w.aabb_max[c])) return;
+    const int lane = threadIdx.x & 31;
+    auto collide = [&](int c) {
         V3 cp;
         Q4 co;
         GeomD cg;
         collider_pose(w, c, cp, co, cg);
         if (w.col_info[c].x == self_body) cp = self_pos + qrot(ld4(w.quat[self_body]), ld3(w.col_pos[c]));
-        const int nm = collision_one(w, cp, co, cg, pos, ori, g, ms, cand, poly, w.err);
-        for (int k = 0; k < nm; ++k) {
-            const ManifoldL& m = ms[k];
-            if (!m.numPoints) continue;
-            float mtd = 0.f;
-            for (int p = 0; p < m.numPoints; ++p) {
-                float dist = dot(m.points[p].p0 - m.points[p].p1, m.normal);
-                if (dist > mtd) mtd = dist;
-            }
-            fn(c, m, mtd);
+        return collision_one(w, cp, co, cg, pos, ori, g, ms, cand, poly, w.err);
+    };
+    auto deepest = [](const ManifoldL& m) {
+        float mtd = 0.f;
+        for (int p = 0; p < m.numPoints; ++p) {
+            float dist = dot(m.points[p].p0 - m.points[p].p1, m.normal);
+            if (dist > mtd) mtd = dist;
         }
+        return mtd;
+    };
+    int held = 0, mine = -1;   // WARP: colliders waiting, one in each of the first `held` lanes
+    auto flush = [&]() {
+        const int nm = lane < held ? collide(mine) : 0;
+        __syncwarp();
+        for (unsigned todo = __ballot_sync(~0u, nm > 0); todo; todo &= todo - 1) {
+            const int src = __ffs(todo) - 1;
+            const int n = __shfl_sync(~0u, nm, src), c = __shfl_sync(~0u, mine, src);
+            for (int k = 0; k < n; ++k) {
+                float v[4] = {0.f, 0.f, 0.f, 0.f};
+                int tri = 0, points = 0;
+                if (lane == src) {
+                    const ManifoldL& m = ms[k];
+                    v[0] = m.normal.x; v[1] = m.normal.y; v[2] = m.normal.z;
+                    v[3] = deepest(m);
+                    tri = m.triangleIndex;
+                    points = m.numPoints;
+                }
+                for (int i = 0; i < 4; ++i) v[i] = __shfl_sync(~0u, v[i], src);
+                tri = __shfl_sync(~0u, tri, src);
+                if (__shfl_sync(~0u, points, src)) fn(c, V3{v[0], v[1], v[2]}, v[3], tri);
+            }
+        }
+        held = 0;
+    };
+    auto leaf = [&](int q) {
+        const int c = f.order[q];
+        if (!boxes_meet(qmin, qmax, w.aabb_min[c], w.aabb_max[c])) return;
+        if (WARP) {
+            if (lane == held) mine = c;
+            if (++held == 32) flush();
+            return;
+        }
+        const int nm = collide(c);
+        for (int k = 0; k < nm; ++k)
+            if (ms[k].numPoints) fn(c, ms[k].normal, deepest(ms[k]), ms[k].triangleIndex);
     };
     if (nc == 1) {
         leaf(cs);
@@ -518,12 +551,16 @@ __device__ void for_each_mtd(const World& w, const FrameBuf& f, int s, V3 pos, Q
             stack[sp++] = f.bvh.left[c];
         }
     }
+    if (WARP && held) flush();
 }
 
+// Up to cap records a query: {world collider, n xyz, mtd}.
+template <bool WARP>
 __global__ void __launch_bounds__(64) k_overlap_mtd(World w, FrameBuf f, const ShapeIn* qs, int n, int cap, int* counts,
                                                     float4* hits, int* hit_col) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, i = WARP ? t >> 5 : t;
     if (i >= n) return;
+    const bool first = !WARP || (threadIdx.x & 31) == 0;
     const ShapeIn qi = qs[i];
     const V3 pos = {qi.px, qi.py, qi.pz};
     const Q4 ori = {qi.qx, qi.qy, qi.qz, qi.qw};
@@ -532,19 +569,61 @@ __global__ void __launch_bounds__(64) k_overlap_mtd(World w, FrameBuf f, const S
     TCI cand[kTriCandidates];
     Polytope poly;
     int count = 0;
-    for_each_mtd(w, f, qi.scene, pos, ori, g, ms, cand, poly, [&](int c, const ManifoldL& m, float mtd) {
-        if (count < cap) {
-            hits[(size_t)i * cap + count] = make_float4(m.normal.x, m.normal.y, m.normal.z, mtd);
+    for_each_mtd<WARP>(w, f, qi.scene, pos, ori, g, ms, cand, poly, [&](int c, V3 nrm, float mtd, int) {
+        if (first && count < cap) {
+            hits[(size_t)i * cap + count] = make_float4(nrm.x, nrm.y, nrm.z, mtd);
             hit_col[(size_t)i * cap + count] = c;
         }
         ++count;
     });
-    counts[i] = count;
+    if (first) counts[i] = count;
 }
 
-// CharacterController::move (src/CharacterController.cpp:5-45) for one controller a
-// thread.  The reference's step-up test calls Scene::raycastClosest without a filter,
-// which never reports a hit (src/Physecs.cpp:580, 615), so the translation stays as
+// a controller's hits in the order (collider, triangle), equal ones as they came
+constexpr int kCharHits = 32;
+template <bool WARP>
+struct CharHits {   // one thread's list
+    int n = 0, col[kCharHits], tri[kCharHits];
+    float4 hit[kCharHits];
+    __device__ bool add(int c, int t, float4 v) {
+        if (n == kCharHits) return false;
+        int k = n++;
+        while (k > 0 && (col[k - 1] > c || (col[k - 1] == c && tri[k - 1] > t))) {
+            col[k] = col[k - 1]; tri[k] = tri[k - 1]; hit[k] = hit[k - 1];
+            --k;
+        }
+        col[k] = c; tri[k] = t; hit[k] = v;
+        return true;
+    }
+    __device__ float4 at(int k) const { return hit[k]; }
+};
+template <>
+struct CharHits<true> {   // one entry a lane
+    static_assert(kCharHits == 32, "a lane an entry");
+    int n = 0, col = 0, tri = 0;
+    float4 hit = {0.f, 0.f, 0.f, 0.f};
+    __device__ bool add(int c, int t, float4 v) {
+        if (n == kCharHits) return false;
+        const int lane = threadIdx.x & 31;
+        const int k = __popc(__ballot_sync(~0u, lane < n && !(col > c || (col == c && tri > t))));
+        const int pc = __shfl_up_sync(~0u, col, 1), pt = __shfl_up_sync(~0u, tri, 1);
+        float4 pv;
+        pv.x = __shfl_up_sync(~0u, hit.x, 1); pv.y = __shfl_up_sync(~0u, hit.y, 1);
+        pv.z = __shfl_up_sync(~0u, hit.z, 1); pv.w = __shfl_up_sync(~0u, hit.w, 1);
+        if (lane > k) { col = pc; tri = pt; hit = pv; }
+        if (lane == k) { col = c; tri = t; hit = v; }
+        ++n;
+        return true;
+    }
+    __device__ float4 at(int k) const {
+        return make_float4(__shfl_sync(~0u, hit.x, k), __shfl_sync(~0u, hit.y, k), __shfl_sync(~0u, hit.z, k),
+                           __shfl_sync(~0u, hit.w, k));
+    }
+};
+
+// CharacterController::move (src/CharacterController.cpp:5-45) for one controller a warp
+// (WARP) or a thread.  The reference's step-up test calls Scene::raycastClosest without a
+// filter, which never reports a hit (src/Physecs.cpp:580, 615), so the translation stays as
 // given.  Each iteration collects the capsule's MTD hits and applies them in the order
 // (collider, triangle); the reference applies them in its tree's order, which only
 // changes the rounding of the summed moves.  Controllers of one batch see each other
@@ -552,10 +631,10 @@ __global__ void __launch_bounds__(64) k_overlap_mtd(World w, FrameBuf f, const S
 // pose in moved[i]; k_commit_characters writes them after every controller has moved.
 // A controller's own colliders move with it, as the registry's transform does in the
 // reference, while their bounds stay those before the move.
-constexpr int kCharHits = 32;
+template <bool WARP>
 __global__ void __launch_bounds__(64) k_move_characters(World w, FrameBuf f, const CharIn* cs, int n, unsigned char* flags_out,
                                                         float4* moved) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, i = WARP ? t >> 5 : t;
     if (i >= n) return;
     const CharIn ch = cs[i];
     const int b = ch.body;
@@ -567,34 +646,27 @@ __global__ void __launch_bounds__(64) k_move_characters(World w, FrameBuf f, con
     ManifoldL ms[kTriManifolds];
     TCI cand[kTriCandidates];
     Polytope poly;
-    int hc[kCharHits], ht[kCharHits];
-    float4 hv[kCharHits];
     int flags = 0;
     for (int it = 0; it < ch.iterations; ++it) {
-        int nh = 0;
-        for_each_mtd(w, f, w.info[b].w, p + up * (ch.height * 0.5f + ch.radius), q, g, ms, cand, poly,
-                     [&](int c, const ManifoldL& m, float mtd) {
-                         if (nh == kCharHits) { flags |= 0x80; return; }
-                         // insertion by (collider, triangle), stable
-                         int k = nh++;
-                         while (k > 0 && (hc[k - 1] > c || (hc[k - 1] == c && ht[k - 1] > m.triangleIndex))) {
-                             hc[k] = hc[k - 1]; ht[k] = ht[k - 1]; hv[k] = hv[k - 1];
-                             --k;
-                         }
-                         hc[k] = c; ht[k] = m.triangleIndex;
-                         hv[k] = make_float4(m.normal.x, m.normal.y, m.normal.z, mtd);
-                     }, b, p);
-        for (int k = 0; k < nh; ++k) {
-            const V3 nrm = ld3(hv[k]);
-            const float mtd = hv[k].w;
+        CharHits<WARP> hits;
+        for_each_mtd<WARP>(w, f, w.info[b].w, p + up * (ch.height * 0.5f + ch.radius), q, g, ms, cand, poly,
+                           [&](int c, V3 nrm, float mtd, int tri) {
+                               if (!hits.add(c, tri, make_float4(nrm.x, nrm.y, nrm.z, mtd))) flags |= 0x80;
+                           }, b, p);
+        for (int k = 0; k < hits.n; ++k) {
+            const float4 h = hits.at(k);
+            const V3 nrm = ld3(h);
+            const float mtd = h.w;
             const float d = dot(nrm, up);
             flags |= d > 0.001f ? 1 : (d < -0.001f ? 4 : 2);
             if (d > ch.slope_limit) p += up * mtd / d;
             else p += nrm * mtd;
         }
     }
-    moved[i] = st4(p);
-    flags_out[i] = (unsigned char)flags;
+    if (!WARP || (threadIdx.x & 31) == 0) {
+        moved[i] = st4(p);
+        flags_out[i] = (unsigned char)flags;
+    }
 }
 
 // The moved controllers' poses into the world, then registry.patch<TransformComponent> ->
@@ -620,10 +692,19 @@ __global__ void k_commit_characters(World w, const CharIn* cs, int n, const floa
     }
 }
 
+// Up to this many MTD queries or controllers a call, a warp takes each: a thread takes its
+// query's colliders one after the other (and its warp every kind of collision that some lane
+// has), so few queries are a long chain on a few SMs.  Above it the chip has enough threads
+// and the warps' idle lanes cost more.  A call that moves n controllers (each against its
+// scene of 100 balls and a ground), thread and warp: 128: 105 and 81 us, 1024: 129 and 81,
+// 4096: 203 and 181, 8192: 226 and 283, 32768: 480 and 909.
+constexpr int kWarpQueries = 4096;
+
 int launch_move_characters(const World& w, FrameBuf& f, const CharIn* cs, int n, unsigned char* flags, float4* moved,
                            cudaStream_t s) {
     if (n <= 0) return 0;
-    k_move_characters<<<(n + 63) / 64, 64, 0, s>>>(w, f, cs, n, flags, moved);
+    if (n <= kWarpQueries) k_move_characters<true><<<(n + 1) / 2, 64, 0, s>>>(w, f, cs, n, flags, moved);
+    else k_move_characters<false><<<(n + 63) / 64, 64, 0, s>>>(w, f, cs, n, flags, moved);
     k_commit_characters<<<(n + 127) / 128, 128, 0, s>>>(w, cs, n, moved);
     return 2;
 }
@@ -631,7 +712,8 @@ int launch_move_characters(const World& w, FrameBuf& f, const CharIn* cs, int n,
 int launch_overlap_mtd(const World& w, FrameBuf& f, const ShapeIn* qs, int n, int cap, int* counts, float4* hits,
                        int* hit_col, cudaStream_t s) {
     if (n <= 0) return 0;
-    k_overlap_mtd<<<(n + 63) / 64, 64, 0, s>>>(w, f, qs, n, cap, counts, hits, hit_col);
+    if (n <= kWarpQueries) k_overlap_mtd<true><<<(n + 1) / 2, 64, 0, s>>>(w, f, qs, n, cap, counts, hits, hit_col);
+    else k_overlap_mtd<false><<<(n + 63) / 64, 64, 0, s>>>(w, f, qs, n, cap, counts, hits, hit_col);
     return 1;
 }
 
