@@ -488,8 +488,7 @@ __device__ __forceinline__ bool overlap_incl(float4 amin, float4 amax, float4 bm
 }
 
 // SAP filters of src/Physecs.cpp:138-147
-__device__ __forceinline__ bool pair_ok(const World& w, int ca, int cb) {
-    int4 a = w.col_info[ca], b = w.col_info[cb];
+__device__ __forceinline__ bool pair_ok(const int4& a, const int4& b) {
     if (!(a.w & COL_ENABLE) || !(b.w & COL_ENABLE)) return false;
     if (a.x == b.x) return false;
     if (!((a.w & COL_DYNAMIC) || (b.w & COL_DYNAMIC))) return false;
@@ -497,13 +496,22 @@ __device__ __forceinline__ bool pair_ok(const World& w, int ca, int cb) {
 }
 
 // A warp takes 32 consecutive sorted leaves (Morton neighbours, so their bounds are
-// usually close) and walks their scene's tree together: a node is entered when it may
-// hold a partner of any lane, every lane reads the same node (one broadcast load), and
-// the walk stays warp-uniform; when the leaves lie far apart, each lane walks alone.  Each lane tests only its own leaf p against the leaves q > p
-// the walk reaches.  The walk is left-first depth-first, so each lane's partners come
-// out in increasing sorted position: an order that depends only on the scene (its
-// Morton codes), never on the tree's shape, the warp's other lanes or the batch.  A
-// warp whose leaves belong to two scenes walks them one after the other.
+// usually close) and asks for the partners of all of them with one walk of their scene's
+// tree: a node is entered when it may hold a partner of any of them.  The walk's stack is
+// kept in shared memory in left-to-right order, and a step takes its top 32 entries, a node
+// a lane, so a walk is about as many rounds of loads as the tree is deep.  Leaves it reaches
+// wait in order until there are 32; their bounds and identities then lie in shared memory
+// and each lane tests them against its own leaf p, q > p only.  A leaf much larger than the
+// warp's smallest (a ground) has a walk of its own, and where the leaves lie far apart, each
+// lane walks alone.  Each way a lane's partners come out in increasing sorted position: an
+// order that depends only on the scene (its Morton codes), never on the tree's shape, the
+// warp's other lanes or the batch.  A warp whose leaves belong to two scenes walks them one
+// after the other.
+//
+// Bound by the latency of dependent loads.  With one node a step (and the leaves tested as
+// they came, three dependent rounds each) the broadphase stage took 84 us on a pyramid of
+// 210 boxes, 194 on 2001 mixed colliders, 318 on 256 scenes and 1370 on 4096; now 61, 142,
+// 268 and 1025.
 //
 // The pairs of a leaf go to pairs[leaf_off[p] + k] for its k-th partner, and leaf_off is
 // the scan of the counts, so the walk runs before the scan (counting) and after it
@@ -515,11 +523,10 @@ enum TraverseMode { kCount = 0, kEmit = 1, kCollect = 2, kTail = 3 };
 
 __device__ __forceinline__ int2* trav_scratch(const FrameBuf& f) { return reinterpret_cast<int2*>(f.cat_list); }
 
-// the count-th partner cb of leaf p (collider ca): the pair in entity order, placed or kept
+// the count-th partner cb (entity eb) of leaf p (collider ca, entity ea): the pair in entity order, placed or kept
 template <int MODE>
-__device__ __forceinline__ void place_pair(const World& w, const FrameBuf& f, int ca, int cb, int p, int out, int count) {
+__device__ __forceinline__ void place_pair(const FrameBuf& f, int ca, uint32_t ea, int cb, uint32_t eb, int p, int out, int count) {
     if (MODE == kCount || (MODE == kTail && count < f.trav_k) || (MODE == kCollect && count >= f.trav_k)) return;
-    const uint32_t ea = (uint32_t)w.info[w.col_info[ca].x].x, eb = (uint32_t)w.info[w.col_info[cb].x].x;
     const int2 pr = ea < eb ? make_int2(ca, cb) : make_int2(cb, ca);
     if (MODE == kCollect) {
         trav_scratch(f)[(size_t)p * f.trav_k + count] = pr;
@@ -534,62 +541,142 @@ __device__ __forceinline__ void check_pairs(const World& w, const FrameBuf& f) {
     if (*f.n_pairs > f.pair_cap) { atomicOr(w.err, ERR_PAIR_CAPACITY); *f.n_pairs = f.pair_cap; }
 }
 
+constexpr int kTravThreads = 128;
+// A warp with at most this many leaves after its first one tests all of them, without the
+// tree: their loads depend on nothing, while a walk is a chain of them.  Broadphase stage at
+// 0, 128, 256 and 512: 76, 75, 64 and 64 us (251 colliders), 122, 123, 124 and 98 (901); a
+// batch of 4096 scenes of 16 to 2048 bodies 1091, 1077, 1059 and 1054.
+constexpr int kTravDirect = 512;
+// A joint walk is taken while the lanes' union is at most this many times the largest of
+// them.  At 4, 8, 16 and 32: 159, 150, 173 and 173 us (2001 colliders), 475, 429, 641 and
+// 1761 (65536 on a mesh), 1270, 1052, 1055 and 1063 (the batch).  Splitting a scattered warp
+// into up to 2, 4 or 8 joint walks of near lanes took 150, 171 and 171 (2001), 570 (65536).
+constexpr float kTravSpread = 8.f;
+constexpr int kTravWide = 512;                 // a step takes one entry above this, so that depth bounds the rest
+constexpr int kTravStack = kTravWide + 64;     // a tree is at most 64 deep: 32 code bits, then position bits
+
 template <int MODE>
-__global__ void __launch_bounds__(256) k_traverse(World w, FrameBuf f) {
+__global__ void __launch_bounds__(kTravThreads) k_traverse(World w, FrameBuf f) {
     constexpr bool EMIT = MODE == kEmit || MODE == kTail;
     if (MODE == kEmit && blockIdx.x == 0 && threadIdx.x == 0) check_pairs(w, f);
     if (MODE == kTail && *f.trav_tail == 0) return;
     if (MODE == kCollect && blockIdx.x == 0 && threadIdx.x == 0) *f.trav_tail = 0;
+    __shared__ int s_stack[kTravThreads / 32][kTravStack], s_cand[kTravThreads / 32][64];
+    __shared__ float4 s_lo[kTravThreads / 32][32], s_hi[kTravThreads / 32][32];
+    __shared__ int4 s_id[kTravThreads / 32][32];
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    const int lane = threadIdx.x & 31;
-    int ca = 0, s = -1, root = 0;
+    const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
+    int* const stk = s_stack[wi];
+    int* const cand = s_cand[wi];
+    int ca = 0, s = -1, root = 0, stop = 0;
+    uint32_t ea = 0;
+    int4 ai = make_int4(-1, 0, 0, 0);
     float4 qmin = make_float4(0.f, 0.f, 0.f, 0.f), qmax = qmin;
     bool want = false;
     if (p < w.n_colliders) {
         ca = f.order[p];
-        s = w.info[w.col_info[ca].x].w;
-        int cs = w.scene_col[s], n = w.scene_col[s + 1] - cs;
-        bool active = !w.scene_active || w.scene_active[s];
-        want = n >= 2 && active && (w.col_info[ca].w & COL_ENABLE);
-        if (MODE == kTail) want = want && f.leaf_cnt[p] > f.trav_k;
-        root = cs - s;   // root of this scene's tree
+        ai = w.col_info[ca];
         qmin = w.aabb_min[ca];
         qmax = w.aabb_max[ca];
+        const int4 bi = w.info[ai.x];
+        s = bi.w;
+        ea = (uint32_t)bi.x;
+        int cs = w.scene_col[s], n = w.scene_col[s + 1] - cs;
+        bool active = !w.scene_active || w.scene_active[s];
+        want = n >= 2 && active && (ai.w & COL_ENABLE);
+        if (MODE == kTail) want = want && f.leaf_cnt[p] > f.trav_k;
+        root = cs - s;   // root of this scene's tree
+        stop = cs + n;
     }
+    const float own = fmaxf(fmaxf(qmax.x - qmin.x, qmax.y - qmin.y), qmax.z - qmin.z);
+    float least = want ? own : FLT_MAX;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) least = fminf(least, __shfl_xor_sync(~0u, least, o));
+    const bool large = own > 8.f * least;
     int count = 0;
     const int out = (EMIT && p < w.n_colliders) ? f.leaf_off[p] : 0;
+    // leaf q (collider cb), one a lane, for the tests
+    auto stage = [&](int q, int cb, float4 mn, float4 mx, const int4& ci) {
+        mn.w = __int_as_float(q);
+        s_lo[wi][lane] = mn;
+        s_hi[wi][lane] = mx;
+        s_id[wi][lane] = make_int4(ci.x, w.info[ci.x].x, cb, ci.w);
+    };
+    // the first k staged leaves against the lanes of the group
+    auto test = [&](bool mine, int k) {
+        unsigned hits = 0;   // without branches, so that the loads of several leaves are in flight
+#pragma unroll 8
+        for (int j = 0; j < k; ++j) {
+            const float4 mn = s_lo[wi][j], mx = s_hi[wi][j];
+            hits |= (unsigned)(__float_as_int(mn.w) > p && overlap_incl(qmin, qmax, mn, mx)) << j;
+        }
+        for (hits = mine ? hits : 0; hits; hits &= hits - 1) {
+            const int j = __ffs(hits) - 1;
+            const int4 id = s_id[wi][j];
+            if (!pair_ok(ai, id)) continue;
+            place_pair<MODE>(f, ca, ea, id.z, (uint32_t)id.y, p, out, count);
+            ++count;
+        }
+        __syncwarp();
+    };
+    // the first k leaves that wait
+    auto take = [&](int k) {
+        __syncwarp();
+        if (lane < k) {
+            const int q = cand[lane], cb = f.order[q];
+            stage(q, cb, w.aabb_min[cb], w.aabb_max[cb], w.col_info[cb]);
+        }
+        __syncwarp();
+    };
     unsigned pending = __ballot_sync(~0u, want);
     while (pending) {
         const int leader = __ffs(pending) - 1;
+        {   // few leaves after the first lane's: all of them, 32 at a time, without the tree
+            const int q0 = p - lane + leader + 1, end = __shfl_sync(~0u, stop, leader), same = __shfl_sync(~0u, s, leader);
+            if (end - q0 <= kTravDirect) {
+                const bool mine = (pending >> lane & 1) && s == same;
+                pending &= ~__ballot_sync(~0u, mine);
+                int q = q0 + lane, cb = q < end ? f.order[q] : -1;
+                for (; q - lane < end; q += 32) {
+                    const int k = min(32, end - (q - lane));
+                    if (lane < k) stage(q, cb, w.aabb_min[cb], w.aabb_max[cb], w.col_info[cb]);
+                    cb = q + 32 < end ? f.order[q + 32] : -1;
+                    __syncwarp();
+                    test(mine, k);
+                }
+                continue;
+            }
+        }
         const int gs = __shfl_sync(~0u, s, leader);
         const int groot = __shfl_sync(~0u, root, leader);
-        const bool mine = want && s == gs;
-        pending &= ~__ballot_sync(~0u, mine);
+        const bool alone = __shfl_sync(~0u, large, leader);
+        const bool mine = (pending >> lane & 1) && s == gs && (alone ? lane == leader : !large);
+        const unsigned group = __ballot_sync(~0u, mine);
+        pending &= ~group;
         // The joint walk pays for the union of the lanes' bounds.  Leaves that are Morton
         // neighbours but far apart (scattered bodies, where the curve jumps) make that union
-        // much larger than any lane's own bounds; each lane then walks alone.  Either walk
-        // reaches each lane's partners in increasing sorted position, so the output is the
-        // same.
-        float ulo[3] = {qmin.x, qmin.y, qmin.z}, uhi[3] = {qmax.x, qmax.y, qmax.z};
-        float own = fmaxf(fmaxf(qmax.x - qmin.x, qmax.y - qmin.y), qmax.z - qmin.z);
+        // much larger than any lane's own bounds; each lane then walks alone.
+        float4 umin = qmin, umax = qmax;
+        float most = own;
         if (!mine) {
-            ulo[0] = ulo[1] = ulo[2] = FLT_MAX;
-            uhi[0] = uhi[1] = uhi[2] = -FLT_MAX;
-            own = 0.f;
+            umin = make_float4(FLT_MAX, FLT_MAX, FLT_MAX, 0.f);
+            umax = make_float4(-FLT_MAX, -FLT_MAX, -FLT_MAX, 0.f);
+            most = 0.f;
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                ulo[k] = fminf(ulo[k], __shfl_xor_sync(~0u, ulo[k], o));
-                uhi[k] = fmaxf(uhi[k], __shfl_xor_sync(~0u, uhi[k], o));
-            }
-            own = fmaxf(own, __shfl_xor_sync(~0u, own, o));
+            umin.x = fminf(umin.x, __shfl_xor_sync(~0u, umin.x, o));
+            umin.y = fminf(umin.y, __shfl_xor_sync(~0u, umin.y, o));
+            umin.z = fminf(umin.z, __shfl_xor_sync(~0u, umin.z, o));
+            umax.x = fmaxf(umax.x, __shfl_xor_sync(~0u, umax.x, o));
+            umax.y = fmaxf(umax.y, __shfl_xor_sync(~0u, umax.y, o));
+            umax.z = fmaxf(umax.z, __shfl_xor_sync(~0u, umax.z, o));
+            most = fmaxf(most, __shfl_xor_sync(~0u, most, o));
         }
-        const float spread = fmaxf(fmaxf(uhi[0] - ulo[0], uhi[1] - ulo[1]), uhi[2] - ulo[2]);
-        int stack[64];
-        int sp = 0;
-        if (!(spread <= 8.f * own)) {   // scattered leaves (or a NaN bound): one walk per lane
+        const float spread = fmaxf(fmaxf(umax.x - umin.x, umax.y - umin.y), umax.z - umin.z);
+        if (!(spread <= kTravSpread * most)) {   // scattered leaves (or a NaN bound): one walk per lane
+            int stack[64];
+            int sp = 0;
             if (mine) stack[sp++] = groot;
             while (sp) {
                 const int c = stack[--sp];
@@ -597,9 +684,10 @@ __global__ void __launch_bounds__(256) k_traverse(World w, FrameBuf f) {
                     const int q = ~c;
                     if (q <= p) continue;
                     const int cb = f.order[q];
+                    const int4 ci = w.col_info[cb];
                     if (!overlap_incl(qmin, qmax, w.aabb_min[cb], w.aabb_max[cb])) continue;
-                    if (!pair_ok(w, ca, cb)) continue;
-                    place_pair<MODE>(w, f, ca, cb, p, out, count);
+                    if (!pair_ok(ai, ci)) continue;
+                    place_pair<MODE>(f, ca, ea, cb, (uint32_t)w.info[ci.x].x, p, out, count);
                     ++count;
                 } else {
                     // the node's fields in one round of loads (c is a node of the lane's tree)
@@ -615,33 +703,62 @@ __global__ void __launch_bounds__(256) k_traverse(World w, FrameBuf f) {
                     }
                 }
             }
+            __syncwarp();
             continue;
         }
-        // the joint walk: the stack is the same in every lane
-        stack[sp++] = groot;
+        const int pmin = p - lane + __ffs(group) - 1;
+        int sp = 1, held = 0;
+        if (lane == 0) stk[0] = groot;
+        __syncwarp();
         while (sp) {
-            const int c = stack[--sp];
-            if (c < 0) {
-                const int q = ~c;
-                if (!mine || q <= p) continue;
-                const int cb = f.order[q];
-                if (!overlap_incl(qmin, qmax, w.aabb_min[cb], w.aabb_max[cb])) continue;
-                if (!pair_ok(w, ca, cb)) continue;
-                place_pair<MODE>(w, f, ca, cb, p, out, count);
-                ++count;
-            } else {
-                // the node's fields in one round of loads, children before the vote
-                const int last = f.bvh.last[c], L = f.bvh.left[c], R = f.bvh.right[c];
-                const float4 bmn = f.bvh.bmin[c], bmx = f.bvh.bmax[c];
-                const bool go = mine && last > p && overlap_incl(qmin, qmax, bmn, bmx);
-                if (!__any_sync(~0u, go)) continue;
-                if (sp + 2 <= 64) {
-                    stack[sp++] = R;
-                    stack[sp++] = L;
-                } else if (lane == 0) {
-                    atomicOr(w.err, ERR_STACK_CAPACITY);
+            const int m = min(min(32, sp), max(1, kTravWide - sp)), base = sp - m;
+            int c = 0, L = 0, R = 0, push = 0;   // push: entries that take this one's place
+            if (lane < m) {
+                c = stk[sp - 1 - lane];
+                if (c < 0) {
+                    push = ~c > pmin;
+                } else {
+                    const int last = f.bvh.last[c];
+                    L = f.bvh.left[c];
+                    R = f.bvh.right[c];
+                    const float4 bmn = f.bvh.bmin[c], bmx = f.bvh.bmax[c];
+                    push = last > pmin && overlap_incl(umin, umax, bmn, bmx) ? 2 : 0;
                 }
             }
+            const unsigned two = __ballot_sync(~0u, push == 2);
+            const int first = two ? __ffs(two) - 1 : 32;   // the leaves before the first entered node are next
+            const unsigned next = __ballot_sync(~0u, push == 1 && lane < first);
+            const unsigned one = __ballot_sync(~0u, push == 1 && lane > first);
+            if (sp + m > kTravStack) {   // deeper than any tree
+                if (lane == 0) atomicOr(w.err, ERR_STACK_CAPACITY);
+                break;
+            }
+            if (push == 1 && lane < first) cand[held + __popc(next & ((1u << lane) - 1))] = ~c;
+            held += __popc(next);
+            const unsigned under = ~((2u << lane) - 1);    // entries after this one lie below it
+            const int at = base + 2 * __popc(two & under) + __popc(one & under);
+            __syncwarp();
+            if (push == 2) {
+                stk[at] = R;
+                stk[at + 1] = L;
+            } else if (push == 1 && lane > first) {
+                stk[at] = c;
+            }
+            sp = base + 2 * __popc(two) + __popc(one);
+            __syncwarp();
+            if (held >= 32) {
+                take(32);
+                test(mine, 32);
+                held -= 32;
+                const int c2 = lane < held ? cand[32 + lane] : 0;
+                __syncwarp();
+                if (lane < held) cand[lane] = c2;
+                __syncwarp();
+            }
+        }
+        if (held) {
+            take(held);
+            test(mine, held);
         }
     }
     if (!EMIT && p < w.n_colliders) f.leaf_cnt[p] = count;
@@ -809,18 +926,18 @@ int launch_bvh_build(const World& w, FrameBuf& f, int scene_bits, int scene_sort
 int launch_broadphase(const World& w, FrameBuf& f, int scene_bits, int scene_sort_pmax, cudaStream_t s) {
     int n = w.n_colliders;
     if (n == 0) return 0;
-    int nb = (n + 255) / 256;
+    const int nb = (n + 255) / 256, nt = (n + kTravThreads - 1) / kTravThreads;
     int k = launch_bvh_build(w, f, scene_bits, scene_sort_pmax, false, s);
     if (f.trav_k > 0) {   // one walk, the kept pairs placed after the scan, a second walk only for long lists
-        k_traverse<kCollect><<<nb, 256, 0, s>>>(w, f);
+        k_traverse<kCollect><<<nt, kTravThreads, 0, s>>>(w, f);
         k += scan_exclusive(f.leaf_cnt, f.leaf_off, n, f.n_pairs, f.scan_scratch, s);
         k_pairs_place<<<std::min(nb, 152 * 8), 256, 0, s>>>(w, f);
-        k_traverse<kTail><<<nb, 256, 0, s>>>(w, f);
+        k_traverse<kTail><<<nt, kTravThreads, 0, s>>>(w, f);
         return k + 3;
     }
-    k_traverse<kCount><<<nb, 256, 0, s>>>(w, f);
+    k_traverse<kCount><<<nt, kTravThreads, 0, s>>>(w, f);
     k += scan_exclusive(f.leaf_cnt, f.leaf_off, n, f.n_pairs, f.scan_scratch, s);
-    k_traverse<kEmit><<<nb, 256, 0, s>>>(w, f);
+    k_traverse<kEmit><<<nt, kTravThreads, 0, s>>>(w, f);
     return k + 2;
 }
 
