@@ -107,7 +107,7 @@ __global__ void __launch_bounds__(256) k_narrow_analytic(World w, FrameBuf f) {
 }
 
 // convex-mesh pairs, part 1: GJK, then EPA for the pairs GJK finds overlapping.  The
-// EPA normal and closest points (or "no contact") are staged in the pair's manifold slot.
+// EPA normal and closest points are staged in the pair's manifold slot.
 
 __device__ __forceinline__ bool convex_pair_ordered(const World& w, int2 pr, V3& pos0, Q4& or0, GeomD& g0, V3& pos1,
                                                     Q4& or1, GeomD& g1) {
@@ -144,19 +144,13 @@ __global__ void __launch_bounds__(128, 4) k_convex_gjk(World w, FrameBuf f) {
         convexOrderedSupports(w, pos0, or0, g0, pos1, or1, g1, a, b);
         GjkSimplex s;
         const bool hit = gjk(a, b, pos1 - pos0, s);
-        Manifold& m = f.man_pair[p];
         if (hit) {
-            m.np = 1;
+            Manifold& m = f.man_pair[p];
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 m.p0[i] = make_float4(s.v[i].sp0.x, s.v[i].sp0.y, s.v[i].sp0.z, 0.f);
                 m.p1[i] = make_float4(s.v[i].sp1.x, s.v[i].sp1.y, s.v[i].sp1.z, 0.f);
             }
-        } else {
-            m.np = -1;
-            m.n = make_float4(0.f, 0.f, 0.f, 0.f);
-            m.p0[0] = m.n;
-            m.p1[0] = m.n;
         }
         const unsigned act = __activemask();
         const unsigned hm = __ballot_sync(act, hit);
@@ -400,27 +394,61 @@ __global__ void __launch_bounds__(32) k_convex_epa_full(World w, FrameBuf f, int
 }
 
 // convex-mesh pairs, part 2: contact generation after EPA (face selection and
-// clipping, Collision.cpp:352-887), one thread per pair.
+// clipping, Collision.cpp:352-887), one thread per overlapping pair.  Bound by the latency
+// of its local arrays and by divergence: a convex mesh clipped against another takes far
+// longer than against a box or a capsule, and a sphere takes nothing.  So a warp takes 128
+// pairs at a time where there are enough and works through them by the kind of the other
+// shape.
+constexpr int kConChunk = 128;
 __global__ void __launch_bounds__(256) k_convex_contacts(World w, FrameBuf f) {
-    const int n = f.cat_count[1];
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
-        const int p = f.cat_list[f.pair_cap + t];
-        Manifold& m = f.man_pair[p];
-        if (m.np < 0) { f.pair_nman[p] = 0; continue; }
-        V3 pos0, pos1;
-        Q4 or0, or1;
-        GeomD g0, g1;
-        bool swap = convex_pair_ordered(w, f.pairs[p], pos0, or0, g0, pos1, or1, g1);
-        ManifoldL r;
-        r.numPoints = 0;
-        r.triangleIndex = -1;
-        r.normal = ld3(m.n);
-        r.points[0] = {ld3(m.p0[0]), ld3(m.p1[0])};
-        convexOrderedContacts(w, pos0, or0, g0, pos1, or1, g1, r, w.err);
-        if (swap) flipM(r);
-        int cnt = r.numPoints ? 1 : 0;
-        if (cnt) store_manifold(m, r, p);
-        f.pair_nman[p] = cnt;
+    __shared__ int s_order[8][kConChunk];
+    const int n = f.cat_count[3];
+    const int lane = threadIdx.x & 31;
+    int* const order = s_order[threadIdx.x >> 5];
+    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, warps = (gridDim.x * blockDim.x) >> 5;
+    const int chunk = n <= warps ? 1 : min(kConChunk, max(32, (n + warps - 1) / warps));
+    for (int base = warp * chunk; base < n; base += warps * chunk) {
+        const int k = min(chunk, n - base);
+        int kind[kConChunk / 32], item[kConChunk / 32];
+#pragma unroll
+        for (int j = 0; j < kConChunk / 32; ++j) {
+            kind[j] = -1;
+            if (j * 32 + lane >= k) continue;
+            item[j] = f.cat_list[3 * (size_t)f.pair_cap + base + j * 32 + lane];
+            const int2 pr = f.pairs[f.cat_list[f.pair_cap + item[j]]];
+            const int t0 = w.col_info[pr.x].y, t1 = w.col_info[pr.y].y;
+            const int other = t1 == G_CONVEX ? t0 : t1;
+            kind[j] = other == G_CONVEX ? 0 : other == G_BOX ? 1 : other == G_CAPSULE ? 2 : 3;
+        }
+        int at = 0;
+        for (int c = 0; c < 4; ++c) {
+#pragma unroll
+            for (int j = 0; j < kConChunk / 32; ++j) {
+                const unsigned m = __ballot_sync(0xffffffffu, kind[j] == c);
+                if (kind[j] == c) order[at + __popc(m & ((1u << lane) - 1u))] = item[j];
+                at += __popc(m);
+            }
+        }
+        __syncwarp();
+        for (int i = lane; i < k; i += 32) {
+            const int p = f.cat_list[f.pair_cap + order[i]];
+            Manifold& m = f.man_pair[p];
+            V3 pos0, pos1;
+            Q4 or0, or1;
+            GeomD g0, g1;
+            bool swap = convex_pair_ordered(w, f.pairs[p], pos0, or0, g0, pos1, or1, g1);
+            ManifoldL r;
+            r.numPoints = 0;
+            r.triangleIndex = -1;
+            r.normal = ld3(m.n);
+            r.points[0] = {ld3(m.p0[0]), ld3(m.p1[0])};
+            convexOrderedContacts(w, pos0, or0, g0, pos1, or1, g1, r, w.err);
+            if (swap) flipM(r);
+            int cnt = r.numPoints ? 1 : 0;
+            if (cnt) store_manifold(m, r, p);
+            f.pair_nman[p] = cnt;   // k_classify left 0 for the pairs that do not overlap
+        }
+        __syncwarp();
     }
 }
 
