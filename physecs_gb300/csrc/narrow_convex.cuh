@@ -167,41 +167,55 @@ __device__ inline void completeFromLine(MK& mk, GjkSimplex& s) {
     if (distPointToPlane(f3(s.v[3].pos), f3(s.v[0].pos), f3(dir)) < 0.0001f) s.v[3] = mk(f3(-dir));
 }
 
-// GJK.h:226-292
+// GJK.h:226-292, up to the first full simplex
+enum GjkState { kGjkApart = 0, kGjkOverlap = 1, kGjkGoOn = 2 };
 template <class MK>
-__device__ inline bool gjkT(MK& mk, V3 startDir, GjkSimplex& s) {
+__device__ inline GjkState gjkBegin(MK& mk, V3 startDir, GjkSimplex& s) {
     D3 dir = d3(normalize(startDir));
     s.v[0] = mk(f3(dir));
     if (isZeroF(f3(s.v[0].pos))) {
         dir = -dir;
         s.v[1] = mk(f3(dir));
         completeFromLine(mk, s);
-        return true;
+        return kGjkOverlap;
     }
     dir = -s.v[0].pos;
-    if (!checkDirection(mk, dir, s.v[1])) return false;
+    if (!checkDirection(mk, dir, s.v[1])) return kGjkApart;
     dir = cross(cross(s.v[0].pos - s.v[1].pos, -s.v[1].pos), s.v[0].pos - s.v[1].pos);
-    if (isZeroF(f3(dir))) { completeFromLine(mk, s); return true; }
-    if (!checkDirection(mk, dir, s.v[2])) return false;
+    if (isZeroF(f3(dir))) { completeFromLine(mk, s); return kGjkOverlap; }
+    if (!checkDirection(mk, dir, s.v[2])) return kGjkApart;
     dir = cross(s.v[1].pos - s.v[0].pos, s.v[2].pos - s.v[0].pos);
     double sg = signD(dot(-s.v[0].pos, dir));
     if (!sg) {
         dir = normalize(dir);
         s.v[3] = mk(f3(dir));
         if (distPointToPlane(f3(s.v[3].pos), f3(s.v[0].pos), f3(dir)) < 0.0001f) s.v[3] = mk(f3(-dir));
-        return true;
+        return kGjkOverlap;
     }
     dir = sg * dir;
-    if (!checkDirection(mk, dir, s.v[3])) return false;
+    if (!checkDirection(mk, dir, s.v[3])) return kGjkApart;
+    return kGjkGoOn;
+}
+// one step of its loop over simplices
+constexpr int kGjkSteps = 100;
+template <class MK>
+__device__ inline GjkState gjkStep(MK& mk, GjkSimplex& s) {
+    D3 dir;
     int fi;
-    for (int i = 0; i < 100; ++i) {
-        if (mk.containsOrigin(s, dir, fi)) return true;
-        if (!checkDirection(mk, dir, s.v[fi])) return false;
-        GjkVertex t = s.v[fi];
-        s.v[fi] = s.v[3];
-        s.v[3] = t;
-    }
-    return false;
+    if (mk.containsOrigin(s, dir, fi)) return kGjkOverlap;
+    GjkVertex v;
+    if (!checkDirection(mk, dir, v)) return kGjkApart;
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+        if (i == fi) s.v[i] = s.v[3];
+    s.v[3] = v;
+    return kGjkGoOn;
+}
+template <class MK>
+__device__ inline bool gjkT(MK& mk, V3 startDir, GjkSimplex& s) {
+    GjkState st = gjkBegin(mk, startDir, s);
+    for (int i = 0; i < kGjkSteps && st == kGjkGoOn; ++i) st = gjkStep(mk, s);
+    return st == kGjkOverlap;
 }
 
 struct PairMink {

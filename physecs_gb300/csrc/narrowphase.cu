@@ -124,43 +124,146 @@ __device__ __forceinline__ bool convex_pair_ordered(const World& w, int2 pr, V3&
     return swap;
 }
 
-// GJK with one thread per pair.  Its simplex arithmetic is f64, and the FP64 pipe costs
-// the same for a warp instruction whatever the number of lanes that use it, so 32 pairs
-// per warp instruction is where GJK is cheapest; the support searches are f32.  Most
-// pairs end here without contact (their bounds overlap, their shapes do not).  For an
-// overlapping pair the final simplex is kept in the pair's manifold slot (the f32
-// support points; each Minkowski vertex is their difference widened to f64, so it is
-// rebuilt exactly) and the pair joins the list that EPA works through.
+// GJK with a lane per pair.  Its simplex arithmetic is f64, and the FP64 pipe costs the
+// same for a warp instruction whatever the number of lanes that use it, so full warps are
+// where GJK is cheapest; the support searches are f32.  For an overlapping pair the final
+// simplex is kept in the pair's manifold slot (the f32 support points; each Minkowski vertex
+// is their difference widened to f64, so it is rebuilt exactly) and the pair joins the list
+// that EPA works through.
+//
+// k_convex_gjk: a pair a lane to its end.  A warp waits for its slowest lane, so few pairs
+// are spread over 608 warps (4 an SM): 1475 pairs took 83 us in full warps and take 68.
+// Fewer than 32 a warp where there are more pairs was slower (narrowphase stage of 64
+// scenes, 21,000 pairs, at 32, 9 and 5 a warp: 578, 617 and 666 us).
+//
+// k_convex_gjk_refill: of the pairs of a large batch 46 % end without contact before there
+// is a full simplex, the others go through the loop over simplices 2.6 times on average, and
+// the longest of 32 six or seven times.  So a warp takes up to 256 pairs: first it brings all
+// of them to the full simplex, 32 at a time, leaving those that go on in their manifold
+// slots, then it runs the loop with idle lanes taking the next ones when there are
+// kGjkIdle of them (8: 1 % faster than 16).  4096 scenes, 1.36 M pairs: 2360 us in the first
+// form, 1420 in this one.  It needs more registers, and 256 scenes (111,000 colliders, 85,000
+// pairs) took 206 and 230 us, so it is for worlds of more than kGjkRefill colliders.
+constexpr int kGjkBatch = 256, kGjkIdle = 8, kGjkRefill = 1 << 17;
+struct GjkPair { Support a, b; GjkSimplex s; };
+
+__device__ __forceinline__ void gjk_load(const World& w, const FrameBuf& f, int p, GjkPair& g, V3& start) {
+    V3 pos0, pos1;
+    Q4 or0, or1;
+    GeomD g0, g1;
+    convex_pair_ordered(w, f.pairs[p], pos0, or0, g0, pos1, or1, g1);
+    convexOrderedSupports(w, pos0, or0, g0, pos1, or1, g1, g.a, g.b);
+    start = pos1 - pos0;
+}
+__device__ __forceinline__ void gjk_keep(Manifold& m, const GjkSimplex& s) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        m.p0[i] = st4(s.v[i].sp0);
+        m.p1[i] = st4(s.v[i].sp1);
+    }
+}
+__device__ __forceinline__ void gjk_restore(const Manifold& m, GjkSimplex& s) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const V3 sa = ld3(m.p0[i]), sb = ld3(m.p1[i]);
+        s.v[i] = {d3(sa - sb), sa, sb};
+    }
+}
+
+// the warp's overlapping pairs (t of each lane with hit) onto EPA's list
+__device__ __forceinline__ void gjk_overlapping(const FrameBuf& f, bool hit, int t) {
+    const int lane = threadIdx.x & 31;
+    const unsigned hm = __ballot_sync(~0u, hit);
+    if (!hm) return;
+    const int leader = __ffs(hm) - 1;
+    int first = 0;
+    if (lane == leader) first = atomicAdd(&f.cat_count[3], __popc(hm));
+    first = __shfl_sync(~0u, first, leader);
+    if (hit) f.cat_list[3 * (size_t)f.pair_cap + first + __popc(hm & ((1u << lane) - 1u))] = t;
+}
+
 __global__ void __launch_bounds__(128, 4) k_convex_gjk(World w, FrameBuf f) {
     const int n = f.cat_count[1];
     const int lane = threadIdx.x & 31;
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
-        const int p = f.cat_list[f.pair_cap + t];
-        V3 pos0, pos1;
-        Q4 or0, or1;
-        GeomD g0, g1;
-        convex_pair_ordered(w, f.pairs[p], pos0, or0, g0, pos1, or1, g1);
-        Support a, b;
-        convexOrderedSupports(w, pos0, or0, g0, pos1, or1, g1, a, b);
-        GjkSimplex s;
-        const bool hit = gjk(a, b, pos1 - pos0, s);
-        if (hit) {
-            Manifold& m = f.man_pair[p];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                m.p0[i] = make_float4(s.v[i].sp0.x, s.v[i].sp0.y, s.v[i].sp0.z, 0.f);
-                m.p1[i] = make_float4(s.v[i].sp1.x, s.v[i].sp1.y, s.v[i].sp1.z, 0.f);
+    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, warps = (gridDim.x * blockDim.x) >> 5;
+    const int batch = min(32, (n + 607) / 608);
+    for (int base = warp * batch; base < n; base += warps * batch) {
+        const int t = base + lane;
+        bool hit = false;
+        if (lane < batch && t < n) {
+            const int p = f.cat_list[f.pair_cap + t];
+            GjkPair g;
+            V3 start;
+            gjk_load(w, f, p, g, start);
+            hit = gjk(g.a, g.b, start, g.s);
+            if (hit) gjk_keep(f.man_pair[p], g.s);
+        }
+        __syncwarp();
+        gjk_overlapping(f, hit, t);
+    }
+}
+
+__global__ void __launch_bounds__(128, 4) k_convex_gjk_refill(World w, FrameBuf f) {
+    __shared__ int s_wait[4][kGjkBatch];
+    const int n = f.cat_count[1];
+    const int lane = threadIdx.x & 31;
+    const unsigned below = (1u << lane) - 1u;
+    int* const wait = s_wait[threadIdx.x >> 5];
+    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, warps = (gridDim.x * blockDim.x) >> 5;
+    const int batch = min(kGjkBatch, max(32, (n + 2431) / 2432));   // at least 16 warps an SM
+    for (int base = warp * batch; base < n; base += warps * batch) {
+        const int end = min(base + batch, n);
+        GjkPair g;
+        PairMink mk{g.a, g.b};
+        int t = -1, p = 0, step = 0, held = 0, next = 0;   // t: the pair in this lane's registers
+        GjkState st = kGjkApart;                           // kGjkOverlap: not yet on the list
+        for (int at = base; at < end; at += 32) {
+            st = kGjkApart;
+            t = at + lane;
+            if (t < end) {
+                p = f.cat_list[f.pair_cap + t];
+                V3 start;
+                gjk_load(w, f, p, g, start);
+                st = gjkBegin(mk, start, g.s);
+                if (st == kGjkOverlap || (st == kGjkGoOn && at + 32 < end)) gjk_keep(f.man_pair[p], g.s);
+            }
+            __syncwarp();
+            if (at + 32 < end) {   // the last 32 go on from here
+                gjk_overlapping(f, st == kGjkOverlap, t);
+                const unsigned m = __ballot_sync(~0u, st == kGjkGoOn);
+                if (st == kGjkGoOn) wait[held + __popc(m & below)] = t;
+                held += __popc(m);
             }
         }
-        const unsigned act = __activemask();
-        const unsigned hm = __ballot_sync(act, hit);
-        int first = 0;
-        if (hm) {
-            const int leader = __ffs(hm) - 1;
-            if (lane == leader) first = atomicAdd(&f.cat_count[3], __popc(hm));
-            first = __shfl_sync(act, first, leader);
-            if (hit) f.cat_list[3 * (size_t)f.pair_cap + first + __popc(hm & ((1u << lane) - 1u))] = t;
+        __syncwarp();
+        while (true) {
+            const unsigned idle = __ballot_sync(~0u, st != kGjkGoOn);
+            if (next < held && __popc(idle) >= kGjkIdle) {
+                gjk_overlapping(f, st == kGjkOverlap, t);
+                const int k = next + __popc(idle & below);
+                if (st == kGjkOverlap) st = kGjkApart;
+                if (st != kGjkGoOn && k < held) {
+                    st = kGjkGoOn;
+                    t = wait[k];
+                    p = f.cat_list[f.pair_cap + t];
+                    V3 start;
+                    gjk_load(w, f, p, g, start);
+                    gjk_restore(f.man_pair[p], g.s);
+                    step = 0;
+                }
+                next += __popc(idle);
+            } else if (idle == ~0u) {
+                break;
+            }
+            if (st == kGjkGoOn) {
+                st = gjkStep(mk, g.s);
+                if (st == kGjkOverlap) gjk_keep(f.man_pair[p], g.s);
+                else if (st == kGjkGoOn && ++step == kGjkSteps) st = kGjkApart;
+            }
+            __syncwarp();
         }
+        gjk_overlapping(f, st == kGjkOverlap, t);
+        __syncwarp();
     }
 }
 
@@ -195,11 +298,7 @@ __device__ __forceinline__ int epa_pair(const World& w, FrameBuf& f, int t, PT& 
     convexOrderedSupports(w, pos0, or0, g0, pos1, or1, g1, a, b);
     Manifold& m = f.man_pair[p];
     GjkSimplex s;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const V3 sa = ld3(m.p0[i]), sb = ld3(m.p1[i]);
-        s.v[i] = {d3(sa - sb), sa, sb};
-    }
+    gjk_restore(m, s);
     V3 nrm, c0, c1;
     const int r = group_epa<G, PT, kSpill>(a, b, s, nrm, c0, c1, P, g, w.err, resume);   // ends with a group barrier
     if (r <= 0) return r;
@@ -543,7 +642,8 @@ int launch_narrowphase(const World& w, FrameBuf& f, const StreamPair& sp, const 
     if (w.may_convex) {
         cudaEventRecord(sp.fork, s);
         cudaStreamWaitEvent(sp.aux, sp.fork, 0);
-        k_convex_gjk<<<152 * ns.gjk_blocks_per_sm, 128, 0, sp.aux>>>(w, f);
+        if (w.n_colliders > kGjkRefill) k_convex_gjk_refill<<<152 * ns.gjk_blocks_per_sm, 128, 0, sp.aux>>>(w, f);
+        else k_convex_gjk<<<152 * ns.gjk_blocks_per_sm, 128, 0, sp.aux>>>(w, f);
         // epa_lanes 1: a lane per pair first; the pairs that outgrow it go to the grouped
         // kernel (16 lanes), or with epa_full_only straight to the full polytope.
         // (Generating the finished pairs' contacts on another stream beside the longer passes
