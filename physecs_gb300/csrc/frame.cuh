@@ -166,6 +166,7 @@ int launch_move_characters(const World& w, FrameBuf& f, const CharIn* cs, int n,
 int launch_overlap_mtd(const World& w, FrameBuf& f, const ShapeIn* qs, int n, int cap, int* counts, float4* hits,
                        int* hit_col, cudaStream_t s);
 // a second stream with a fork / join event pair, for kernels that may overlap
+// (mid: the aux stream goes on once the main one got that far)
 struct StreamPair {
     cudaStream_t aux;
     cudaEvent_t fork, join, mid;

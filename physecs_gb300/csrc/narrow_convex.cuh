@@ -888,13 +888,15 @@ __device__ inline bool collideAnalyticT(V3 pos0, Q4 or0, const GeomD& g0, V3 pos
     if constexpr (BOXES == 2) {
         return boxBox(pos0, or0, gv(g0), pos1, or1, gv(g1), r, err);
     } else if constexpr (BOXES == 1) {
-        if (g1.type == G_BOX) {
-            if (g0.type == G_SPHERE) return sphereBox(pos0, g0.p[0], pos1, or1, gv(g1), r);
-            return capsuleBox(pos0, or0, g0.p[0], g0.p[1], pos1, or1, gv(g1), r);
-        }
-        if (g1.type == G_SPHERE) { bool h = sphereBox(pos1, g1.p[0], pos0, or0, gv(g0), r); flipM(r); return h; }
-        bool h = capsuleBox(pos1, or1, g1.p[0], g1.p[1], pos0, or0, gv(g0), r);
-        flipM(r);
+        // the box second; one copy of each routine, so that a warp's lanes part two ways only
+        const bool flip = g1.type != G_BOX;
+        const V3 pa = flip ? pos1 : pos0, pb = flip ? pos0 : pos1;
+        const Q4 oa = flip ? or1 : or0, ob = flip ? or0 : or1;
+        const int ta = flip ? g1.type : g0.type;
+        const float a0 = flip ? g1.p[0] : g0.p[0], a1 = flip ? g1.p[1] : g0.p[1];
+        const V3 he = flip ? gv(g0) : gv(g1);
+        const bool h = ta == G_SPHERE ? sphereBox(pa, a0, pb, ob, he, r) : capsuleBox(pa, oa, a0, a1, pb, ob, he, r);
+        if (flip) flipM(r);
         return h;
     } else {
         if (g0.type == G_SPHERE) {

@@ -2,10 +2,11 @@
 //
 // The pair list is split by kind so each kernel runs one code path: analytic
 // pairs (sphere / capsule / box), convex-mesh pairs (GJK + EPA + face clipping)
-// and triangle-mesh pairs (BVH midphase + per-triangle tests).  Every pair is one
-// thread; every kernel writes its manifolds into per-pair slots, and a count /
-// scan / compact pass produces the manifold list in pair order, so the output is
-// deterministic.  Pair geometry follows src/Physecs.cpp:188-213: collider world
+// and triangle-mesh pairs (BVH midphase + per-triangle tests).  A pair is one lane's
+// work in most kernels, a group of lanes' where one pair's chain is long, and a warp's
+// against a triangle mesh; which lane takes which pair never shows in the output: every
+// kernel writes its manifolds into per-pair slots, and a count / scan / compact pass
+// produces the manifold list in pair order.  Pair geometry follows src/Physecs.cpp:188-213: collider world
 // pose = body pose composed with the collider's local pose.
 #include <algorithm>
 #include "frame.cuh"
@@ -85,13 +86,17 @@ __global__ void k_classify(World w, FrameBuf f) {
 }
 
 // analytic pairs: sphere / capsule / box, one kernel per list (BOXES boxes in the pair:
-// list 5 for two, 4 for one, 0 for none), so that each kernel holds only its routines
+// list 5 for two, 4 for one, 0 for none), so that each kernel holds only its routines.
+// A capsule against a box takes several times as long as a sphere, so with one box a warp
+// takes up to 128 pairs where there are enough and works through the spheres first.
+// 4096 scenes: 1136 us with a thread per pair in the list's order, 769 so (with one copy of
+// each routine for both orders of the pair).
+constexpr int kAnaChunk = 128;
 template <int BOXES>
 __global__ void __launch_bounds__(256) k_narrow_analytic(World w, FrameBuf f) {
     constexpr int lst = BOXES == 2 ? 5 : (BOXES == 1 ? 4 : 0);
     const int n = f.cat_count[lst];
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
-        int p = f.cat_list[lst * (size_t)f.pair_cap + t];
+    auto pair = [&](int p) {
         int2 pr = f.pairs[p];
         V3 pos0, pos1;
         Q4 or0, or1;
@@ -103,6 +108,40 @@ __global__ void __launch_bounds__(256) k_narrow_analytic(World w, FrameBuf f) {
         int cnt = (hit && m.numPoints) ? 1 : 0;
         if (cnt) store_manifold(f.man_pair[p], m, p);
         f.pair_nman[p] = cnt;
+    };
+    if constexpr (BOXES == 1) {
+        __shared__ int s_order[8][kAnaChunk];
+        int* const order = s_order[threadIdx.x >> 5];
+        const int lane = threadIdx.x & 31;
+        const unsigned below = (1u << lane) - 1u;
+        const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, warps = (gridDim.x * blockDim.x) >> 5;
+        const int chunk = min(kAnaChunk, max(32, n / warps));
+        for (int base = warp * chunk; base < n; base += warps * chunk) {
+            const int k = min(chunk, n - base);
+            int front = 0, back = k;
+            for (int at = 0; at < k; at += 32) {
+                int p = -1;
+                bool sphere = false;
+                if (at + lane < k) {
+                    p = f.cat_list[lst * (size_t)f.pair_cap + base + at + lane];
+                    if (chunk > 32) {
+                        const int2 pr = f.pairs[p];
+                        sphere = w.col_info[pr.x].y == G_SPHERE || w.col_info[pr.y].y == G_SPHERE;
+                    }
+                }
+                const unsigned ms = __ballot_sync(~0u, sphere), mo = __ballot_sync(~0u, p >= 0 && !sphere);
+                if (sphere) order[front + __popc(ms & below)] = p;
+                else if (p >= 0) order[back - 1 - __popc(mo & below)] = p;
+                front += __popc(ms);
+                back -= __popc(mo);
+            }
+            __syncwarp();
+            for (int i = lane; i < k; i += 32) pair(order[i]);
+            __syncwarp();
+        }
+    } else {
+        for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x)
+            pair(f.cat_list[lst * (size_t)f.pair_cap + t]);
     }
 }
 

@@ -11,8 +11,9 @@
 // One persistent kernel runs a whole frame of a scene: colouring, then every
 // substep's row update, velocity integration, preSolve, iterations, position
 // integration, relaxation and write-back.  Small scenes run one per CTA with
-// __syncthreads between phases; large scenes run on the whole grid with a
-// bounded grid barrier.
+// __syncthreads between phases; large scenes run on a cluster, or on the whole grid,
+// where bodies count their finished solves and contacts wait for their turn on both of
+// theirs (solve_flow), with grid barriers between phases.  Every wait is bounded.
 #include <cooperative_groups.h>
 #include "libm_f32.cuh"
 #include <algorithm>

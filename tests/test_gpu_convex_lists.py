@@ -1,6 +1,7 @@
-"""Convex pairs in worlds of few and many: how a warp takes its pairs in GJK and in the
-contact pass depends on their number in the world, the result of a scene does not.  One
-scene alone equals the oracle (lockstep); every copy of it in a larger world equals it."""
+"""Pairs in worlds of few and many: how a warp takes its pairs in GJK, in the convex contact
+pass and in the one-box routines depends on their number in the world, the result of a scene
+does not.  One scene alone equals the oracle (lockstep); every copy of it in a larger world
+equals it."""
 import numpy as np
 import pytest
 
@@ -31,7 +32,7 @@ def alone(gpu_lib, oracle_lib):
     return s, st
 
 
-@pytest.mark.parametrize("copies", [2, 40, 400, 3000])
+@pytest.mark.parametrize("copies", [2, 40, 400, 3000, 8000])
 def test_copies_equal_the_scene_alone(alone, copies):
     from physecs_gb300.api import World
     s, want = alone
