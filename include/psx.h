@@ -163,20 +163,21 @@ typedef struct psx_launch_config {
     int32_t large_scene_solver;      /* scenes above the block limit: 1 one thread-block cluster each (those whose
                                       * velocities fit the cluster's shared memory), 2 the whole grid, one scene
                                       * after another (default: clusters when two or more scenes fit them) */
-    int32_t gjk_blocks_per_sm;       /* GJK (one thread per convex pair): 128-thread blocks per SM, 1-16 (default 16) */
+    int32_t gjk_blocks_per_sm;       /* GJK (a lane per convex pair): 128-thread blocks per SM, 1-16 (default 16) */
     int32_t epa_lanes;               /* EPA: lanes per overlapping pair, 1, 8, 16 or 32 (default 1); below 32 a block
                                       * is one warp holding 32 / epa_lanes pairs.  1: one lane per pair with the
                                       * warp's new faces built by all of its lanes, and 16 lanes per pair for the
                                       * pairs that need more than 12 steps */
     int32_t solver_threads_min;      /* smallest solver block: 32 or 64 (scenes up to 96 dynamic bodies on 32 or 64
-                                      * threads, up to 384 on 128), 128 or 256 (default: 64 for worlds of more block
-                                      * scenes than two per SM, else 256) */
+                                      * threads, up to 384 on 128), 128 or 256 (default: 128 for worlds with more of
+                                      * these scenes than SMs, else 256) */
     int32_t epa_full_only;           /* 1: no grouped small-polytope pass: the pairs go to the full polytope
                                       * directly, or with epa_lanes 1 after the lane-per-pair pass (lowest latency
                                       * for the slowest pair); 2: the grouped pass between them (highest
                                       * throughput; default) */
-    int32_t large_threads;           /* block scenes above 1024 dynamic bodies: threads per block, 128 (four blocks
-                                      * an SM), 256 (two) or 512 (one, with the most shared memory; default) */
+    int32_t large_threads;           /* block scenes above 1024 dynamic bodies (above 192 in a world with no more such
+                                      * scenes than SMs): threads per block, 128 (four blocks an SM), 256 (two) or
+                                      * 512 (one, with the most shared memory; default) */
 } psx_launch_config;
 
 typedef struct psx_world_opts {
@@ -211,7 +212,8 @@ PSX_API psx_status psx_world_step_timed(psx_world* w, float dt, int32_t frames, 
 /* Waits for queued work and reports a device-side error (capacity, timeout). */
 PSX_API psx_status psx_world_synchronize(psx_world* w);
 /* The reference has no device waits.  Here a scene above the block limit that is solved
- * by the whole grid (a cooperative launch) waits at a grid barrier between colour steps.
+ * by the whole grid (a cooperative launch) waits at grid barriers and, between contacts, for
+ * both bodies' turns.
  * Each wait polls at most `polls` times, 64 ns apart (0: the default, 2^23 polls, about
  * half a second), then gives up: every block leaves the solver, the frame's results are
  * not valid, and psx_world_synchronize returns PSX_ERR_TIMEOUT.  Takes effect from the
