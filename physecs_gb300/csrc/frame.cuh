@@ -91,7 +91,7 @@ struct FrameBuf {
     int* pt_group;        // [man_cap] first of the slots of each contact's group
     int2* cbody;          // [man_cap] colouring: scene-local dynamic bodies of each contact; then
                           // (solve_flow, solve order) its places among its bodies' solves
-    int* bdeg;            // [n_dyn] solve_flow: a body's contacts | its solves per iteration << 16
+    int* bdeg;            // [n_dyn] solve_flow: a body's contacts and its solves per iteration (flow_degree)
     uint4* cmask;         // [n_dyn] colouring: colours each dynamic body carries (128 bits)
     SHdr* s_hdr;          // [man_cap]
     SPt* s_pts;           // [4 * man_cap]

@@ -16,6 +16,7 @@
 // theirs (solve_flow), with grid barriers between phases.  Every wait is bounded.
 #include <cooperative_groups.h>
 #include "libm_f32.cuh"
+#include "solver_words.cuh"
 #include <algorithm>
 #include "frame.cuh"
 
@@ -1207,7 +1208,7 @@ __device__ void solve_flow(const World& w, FrameBuf& f, int s, const GridSync& s
     };
     for (int d = slot; d < nd; d += nth) {
         const int n = carried(d, kMaxColors);
-        f.bdeg[ds + d] = n | (n + w.body_nj[ds + d]) << 16;
+        f.bdeg[ds + d] = flow_degree(n, w.body_nj[ds + d]);
     }
     for (int k = slot; k < ncl; k += nth) {
         SHdr& H = Hg[k];
@@ -1263,12 +1264,12 @@ __device__ void solve_flow(const World& w, FrameBuf& f, int s, const GridSync& s
                 b0 = J.b0 >= 0 ? J.b0 - ds : -1;
                 b1 = J.b1 >= 0 ? J.b1 - ds : -1;
                 const int d0 = b0 >= 0 && it >= 0 ? f.bdeg[J.b0] : 0, d1 = b1 >= 0 && it >= 0 ? f.bdeg[J.b1] : 0;
-                e0 = J.rank0 + (d0 & 0xffff) + max(it, 0) * (d0 >> 16);
-                e1 = J.rank1 + (d1 & 0xffff) + max(it, 0) * (d1 >> 16);
+                e0 = J.rank0 + flow_contacts(d0) + max(it, 0) * flow_solves(d0);
+                e1 = J.rank1 + flow_contacts(d1) + max(it, 0) * flow_solves(d1);
             } else {
                 const int deg = f.bdeg[ds + idx];
                 b0 = idx; b1 = -1;
-                e0 = iterations * (deg >> 16) + (kind == FLOW_OUT ? 1 + (deg & 0xffff) : 0);
+                e0 = iterations * flow_solves(deg) + (kind == FLOW_OUT ? 1 + flow_contacts(deg) : 0);
                 e1 = w.body_nj[ds + idx];   // preSolves the position integration waits for
             }
         };
@@ -1280,15 +1281,15 @@ __device__ void solve_flow(const World& w, FrameBuf& f, int s, const GridSync& s
             int lag = 0;
             if (kind == FLOW_DONE) {
             } else if (kind == FLOW_JOINT && it < 0) {
-                // pseudo velocities: the rows applied so far + 256 x the preSolves done, and the latter
+                // pseudo velocities: the rows applied so far with the preSolves done, and the latter
                 auto ready_pseudo = [&](int b, int want, float4& a, float4& c) {
                     V3 x, y;
                     int s0, s1;
                     ld_stamped(w.pv_v + ds + b, x, s0);
                     ld_stamped(w.pv_w + ds + b, y, s1);
-                    a = st4(x, (float)(s0 & 255));
+                    a = st4(x, (float)flow_pseudo_rows(s0));
                     c = st4(y, 0.f);
-                    return s0 >> 8 == want && s1 == want;
+                    return flow_pseudo_joints(s0) == want && s1 == want;
                 };
                 if (b0 >= 0) ready &= ready_pseudo(b0, e0, ps0, pw0);
                 if (b1 >= 0) ready &= ready_pseudo(b1, e1, ps1, pw1);
@@ -1300,8 +1301,8 @@ __device__ void solve_flow(const World& w, FrameBuf& f, int s, const GridSync& s
                     int s0, s1;
                     ld_stamped(w.pv_v + ds + b0, x, s0);
                     ld_stamped(w.pv_w + ds + b0, y, s1);
-                    ready = s0 >> 8 == e1 && s1 == e1;
-                    ps0 = st4(x, (float)(s0 & 255));
+                    ready = flow_pseudo_joints(s0) == e1 && s1 == e1;
+                    ps0 = st4(x, (float)flow_pseudo_rows(s0));
                     pw0 = st4(y);
                 }
             }
@@ -1319,8 +1320,8 @@ __device__ void solve_flow(const World& w, FrameBuf& f, int s, const GridSync& s
                     w.ang[ds + b0] = st4(pv.w0);
                 }
                 if (kind == FLOW_JOINT && it < 0) {
-                    if (b0 >= 0) { st_stamped(w.pv_v + ds + b0, ld3(ps0), (int)ps0.w | (e0 + 1) << 8); st_stamped(w.pv_w + ds + b0, ld3(pw0), e0 + 1); }
-                    if (b1 >= 0) { st_stamped(w.pv_v + ds + b1, ld3(ps1), (int)ps1.w | (e1 + 1) << 8); st_stamped(w.pv_w + ds + b1, ld3(pw1), e1 + 1); }
+                    if (b0 >= 0) { st_stamped(w.pv_v + ds + b0, ld3(ps0), flow_pseudo((int)ps0.w, e0 + 1)); st_stamped(w.pv_w + ds + b0, ld3(pw0), e0 + 1); }
+                    if (b1 >= 0) { st_stamped(w.pv_v + ds + b1, ld3(ps1), flow_pseudo((int)ps1.w, e1 + 1)); st_stamped(w.pv_w + ds + b1, ld3(pw1), e1 + 1); }
                 } else if (kind != FLOW_OUT) {
                     if (b0 >= 0) { st_stamped(vt + 2 * b0, pv.v0, e0 + 1); st_stamped(vt + 2 * b0 + 1, pv.w0, e0 + 1); }
                     if (b1 >= 0) { st_stamped(vt + 2 * b1, pv.v1, e1 + 1); st_stamped(vt + 2 * b1 + 1, pv.w1, e1 + 1); }
@@ -1459,8 +1460,9 @@ __device__ void solve_scene(const World& w, FrameBuf& f, int s, const S& sy, int
         if (6 * per <= 4 * smem_f4) solve_substeps<false>(w, f, s, sy, sc, 0, 0, ClusterVel{sy.bases, per, sy.lg});
         else solve_substeps<false>(w, f, s, sy, sc, 0, 0, GlobVel{w.vt + 2 * (size_t)ds});
     } else {
-        // a colour beyond the limit is solved in contact order, which the counts do not express
-        if (serial_last || w.self_joint) solve_substeps<false>(w, f, s, sy, sc, 0, 0, GlobVel{w.vt + 2 * (size_t)ds});
+        // a colour beyond the limit is solved in contact order, which the counts do not express,
+        // and a body of very many joints outgrows them
+        if (serial_last || w.no_flow) solve_substeps<false>(w, f, s, sy, sc, 0, 0, GlobVel{w.vt + 2 * (size_t)ds});
         else solve_flow(w, f, s, sy, sc);
     }
 }

@@ -172,7 +172,8 @@ struct World {
     float4* bq;          // 2 per dynamic body: world centre of mass and orientation of the substep
     float4* sv;          // 2 per dynamic body: the substep's integrated velocities (solve_flow)
     int* body_nj;        // joints of each dynamic body
-    int self_joint;      // some joint has one body at both ends
+    int no_flow;         // solve_flow does not apply: a joint has one body at both ends, or a body
+                         // more than kFlowJoints joints
     // colliders
     int4* col_info;      // body, type, mesh, flags
     float4* col_pos;

@@ -16,6 +16,7 @@
 #include <vector>
 #include "meshbvh.cuh"
 #include "runtime.cuh"
+#include "solver_words.cuh"
 
 using namespace psx;
 
@@ -374,8 +375,9 @@ psx_status psx::rt::build_world(psx_world* W, const psx_scene_desc* scenes, int 
             const int d0 = W->h_body_dyn[J.body0], d1 = W->h_body_dyn[J.body1];
             J.rank0 = d0 >= 0 ? nj[d0]++ : 0;
             J.rank1 = d1 >= 0 ? nj[d1]++ : 0;
-            if (J.body0 == J.body1) w.self_joint = 1;
+            if (J.body0 == J.body1) w.no_flow = 1;
         }
+        for (int n : nj) if (n > kFlowJoints) w.no_flow = 1;
         PSX_TRY(W->upload(w.body_nj, nj));
     }
     PSX_TRY(W->upload(w.joints, joints));
