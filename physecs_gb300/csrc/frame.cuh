@@ -80,14 +80,14 @@ struct FrameBuf {
     int* man_scene_cnt;   // [S]
     int* scene_man;       // [S+1]
     // colouring
-    unsigned long long* claim;  // [2 * n_dyn] (colour << 40 | hashed priority << 24 | contact index), two sets a scene
+    unsigned long long* claim;  // [2 * n_dyn] claims on each body (claim_word), two sets a scene
     int* color_of;        // [man_cap]
     int* corder;          // [man_cap] manifolds sorted by (scene, colour, points)
     int* scene_ncolor;    // [S]
     int* color_start;     // [S * kColorBins] contacts per bin of a scene solved by several blocks
     int* claim_pos;       // [S * kColorBins] scatter counters of the same scenes
     // per-substep contact records of scenes whose records do not fit in shared memory
-    int* pt_off;          // [man_cap] point slots of each contact, solve order: first slot, step - 1 from bit 28
+    int* pt_off;          // [man_cap] point slots of each contact, solve order (slot_word)
     int* pt_group;        // [man_cap] first of the slots of each contact's group
     int2* cbody;          // [man_cap] colouring: scene-local dynamic bodies of each contact; then
                           // (solve_flow, solve order) its places among its bodies' solves

@@ -592,7 +592,7 @@ __device__ __forceinline__ M3 world_invI(const World& w, int d) {
 __device__ void contact_header(const World& w, const Contact& c, int ds, int slots, SHdr& H) {
     H.n = c.n;
     H.m = make_float4(c.b0 >= 0 ? w.com[c.b0].w : 0.f, c.b1 >= 0 ? w.com[c.b1].w : 0.f, c.frequency, c.damping);
-    H.i = make_int4(c.b0 >= 0 ? c.b0 - ds : -1, c.b1 >= 0 ? c.b1 - ds : -1, c.np | (c.soft << 8) | (((slots >> 28) + 1) << 9), slots & 0xfffffff);
+    H.i = make_int4(c.b0 >= 0 ? c.b0 - ds : -1, c.b1 >= 0 ? c.b1 - ds : -1, c.np | (c.soft << 8) | (slot_step(slots) << 9), slot_first(slots));
 }
 
 // A contact's rows for one substep: the row update (src/Physecs.cpp:366-427), which reads
@@ -994,9 +994,7 @@ __device__ int colour_contacts(const World& w, FrameBuf& f, int ms, int nc, int 
             for (int q = 0; q < 4; ++q)
                 if (~u[q]) { c = 32 * q + __ffs(~u[q]) - 1; break; }
             if (c >= kMaxColors - 1) { col[k] = -2; continue; }   // no colour left: the serial colour takes it
-            unsigned long long v = ((unsigned long long)c << 40) |
-                                   ((unsigned long long)(cache_hash((unsigned long long)k * 0x9E3779B97F4A7C15ull + round) & 0xffffu) << 24) |
-                                   (unsigned)k;
+            const unsigned long long v = claim_word(c, cache_hash((unsigned long long)k * 0x9E3779B97F4A7C15ull + round), k);
             if (b.x >= 0) atomicMin(&claim[b.x], v);
             if (b.y >= 0) atomicMin(&claim[b.y], v);
         }
@@ -1006,10 +1004,10 @@ __device__ int colour_contacts(const World& w, FrameBuf& f, int ms, int nc, int 
             if (col[k] != -1) continue;
             const int2 b = cb[k];
             const unsigned long long v0 = b.x >= 0 ? claim[b.x] : kFree, v1 = b.y >= 0 ? claim[b.y] : kFree;
-            const bool mine0 = b.x < 0 || (unsigned)(v0 & 0xffffffu) == (unsigned)k;
-            const bool mine1 = b.y < 0 || (unsigned)(v1 & 0xffffffu) == (unsigned)k;
+            const bool mine0 = b.x < 0 || claim_of(v0, k);
+            const bool mine1 = b.y < 0 || claim_of(v1, k);
             if (mine0 && mine1) {
-                int c = (int)((b.x >= 0 ? v0 : v1) >> 40);
+                int c = claim_colour(b.x >= 0 ? v0 : v1);
                 col[k] = c;
                 // each body accepted only this contact this round: plain updates suffice
                 unsigned bit = 1u << (c & 31);
@@ -1436,8 +1434,8 @@ __device__ void solve_scene(const World& w, FrameBuf& f, int s, const S& sy, int
     // Point slots: eight contacts of a bin side by side (fewer at its end), point by point,
     // so that the lanes of a warp read a point of theirs at 112-byte steps, which hit every
     // bank once; a contact's points in a row (448 bytes a contact) put sixteen lanes on
-    // four banks.  pt_off: the contact's first slot and, above bit 28, the step between its
-    // points less one; pt_group: the first of its eight contacts' slots.
+    // four banks.  pt_off: the contact's first slot and the step between its points
+    // (slot_word); pt_group: the first of its eight contacts' slots.
     for (int k = tid; k < ncl; k += nth) {
         const int m = f.corder[ms + k] - ms, b = bin_of(f.color_of[ms + m], m), per = 4 - (b & (kPointBins - 1));
         // in block mode the cursors have moved on to each bin's end
@@ -1445,7 +1443,7 @@ __device__ void solve_scene(const World& w, FrameBuf& f, int s, const S& sy, int
         const int c0 = serial ? colstart[ncol - 1] : (S::kBlock ? (b ? bin_a[b - 1] : 0) : bin_a[b]);
         const int c1 = serial ? ncl : (S::kBlock ? bin_a[b] : (b + 1 < nbins ? bin_a[b + 1] : ncl));
         const int i = k - c0, t8 = i & ~7, step = min(8, c1 - c0 - t8);
-        f.pt_off[ms + k] = (bin_b[b] + t8 * per + (i & 7)) | (step - 1) << 28;
+        f.pt_off[ms + k] = slot_word(bin_b[b] + t8 * per + (i & 7), step);
         f.pt_group[ms + k] = bin_b[b] + t8 * per;
     }
     sy.sync();

@@ -401,7 +401,7 @@ psx_status psx::rt::build_world(psx_world* W, const psx_scene_desc* scenes, int 
     int ppc = o.pairs_per_collider > 0 ? o.pairs_per_collider : 8;
     int mpc = o.manifolds_per_collider > 0 ? o.manifolds_per_collider : 4;
     f.pair_cap = std::max(1024, ppc * n);
-    f.man_cap = std::max(1024, mpc * n);
+    f.man_cap = contact_room(mpc, n);
     int tri_pairs = 0;
     for (int s = 0; s < S; ++s) if (scenes[s].n_trimesh) tri_pairs += scenes[s].n_bodies;
     f.tri_cap = std::max(64, 2 * tri_pairs);

@@ -2,7 +2,8 @@
 
 csrc/solver_words.cuh compiles as plain C++; tests/words/check_words.cpp packs and reads
 back every field where it is widest: a body's joint rows and finished joints up to the
-joints that solve_flow takes."""
+joints that solve_flow takes, a colouring claim's contact index above 2^24, and the point
+slots of the most contacts a world has room for."""
 import os
 import shutil
 import subprocess
