@@ -214,9 +214,12 @@ PSX_API psx_status psx_world_synchronize(psx_world* w);
 /* The reference has no device waits.  Here a scene above the block limit that is solved
  * by the whole grid (a cooperative launch) waits at grid barriers and, between contacts, for
  * both bodies' turns.
- * Each wait polls at most `polls` times, 64 ns apart (0: the default, 2^23 polls, about
- * half a second), then gives up: every block leaves the solver, the frame's results are
- * not valid, and psx_world_synchronize returns PSX_ERR_TIMEOUT.  Takes effect from the
+ * A wait at a barrier polls at most `polls` times, pausing 64 ns after each (0: the
+ * default, 2^23 polls, half a second and the polls' own time), then gives up: every block
+ * leaves the solver, the frame's results are not valid, and psx_world_synchronize returns
+ * PSX_ERR_TIMEOUT.  A wait for a turn (its polls 40 or 400 ns apart) or for the end of a
+ * substep's turns may rightly last through all sweeps of the substep; it gives up when
+ * nothing in the scene was solved through `polls` of its polls.  Takes effect from the
  * next frame. */
 PSX_API psx_status psx_world_set_wait_limit(psx_world* w, int64_t polls);
 /* Scene::setNumSubSteps / setNumIterations / setGravity (src/Physecs.cpp:100-110) for one scene (-1: all). */

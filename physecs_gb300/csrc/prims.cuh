@@ -31,13 +31,16 @@ constexpr long long kDefaultWaitPolls = 1ll << 23;
 // a barrier that the grid did not complete, and after a timeout every block ends
 // within one more bounded wait.  A kernel that uses it must leave nothing behind that
 // a later launch relies on besides *err; the barrier words themselves are reset
-// before each launch.
+// before each launch.  progress(): a number that changes while the blocks still to arrive
+// get on; a wait whose polls reached the limit starts over if it changed.
 struct GridBarrier {
     unsigned int* count;
     unsigned int* gen;
     int* err;
     long long limit;
-    __device__ __forceinline__ void sync() const {
+    __device__ __forceinline__ void sync() const { sync([] { return 0u; }); }
+    template <class P>
+    __device__ __forceinline__ void sync(P&& progress) const {
         __shared__ int leave;
         __syncthreads();
         if (threadIdx.x == 0) {
@@ -54,10 +57,16 @@ struct GridBarrier {
                     atomicAdd(gen, 1u);
                 } else {
                     long long polls = 0;
+                    unsigned int seen = 0;
                     while (*vgen == g) {
                         __nanosleep(64);
                         if (*verr & kBarrierTimeoutBit) { out = 1; break; }
-                        if (++polls > limit) { atomicOr(err, kBarrierTimeoutBit); out = 1; break; }
+                        if (++polls > limit) {
+                            const unsigned int now = progress();
+                            if (now == seen) { atomicOr(err, kBarrierTimeoutBit); out = 1; break; }
+                            seen = now;
+                            polls = 0;
+                        }
                     }
                 }
                 __threadfence();

@@ -1153,6 +1153,12 @@ __device__ void solve_substeps(const World& w, FrameBuf& f, int s, const S& sy, 
 // of its lane's list and ready; all blocks are resident (cooperative launch).  The lanes of
 // a warp poll together and none waits inside a divergent branch.
 //
+// A wait is bounded by what the grid does, not by its own length: a lane may rightly wait
+// through every sweep of a substep (for the position of a body whose solves are other
+// lanes'), and a block without work at the barrier after the last sweep, many times what a
+// barrier after each colour waits.  So a wait whose polls reach the limit adds up the
+// bodies' counts, and gives up only if none has moved since it last did so.
+//
 // Bound by the longest chain of solves on shared bodies, each a poll, a solve and a store
 // through L2.  With a grid barrier after every colour and joint step, an iteration took
 // 77.6 us on 65,536 bodies landing on a terrain (61,000 contacts in nine colours) and 104 us
@@ -1217,7 +1223,12 @@ __device__ void solve_flow(const World& w, FrameBuf& f, int s, const GridSync& s
         const int n1 = b1 >= 0 ? carried(b1, kMaxColors) + w.body_nj[ds + b1] : 0, r1 = b1 >= 0 ? carried(b1, c) : 0;
         f.cbody[ms + k] = make_int2(r0 | n0 << 8, r1 | n1 << 8);   // place, and solves of the body per iteration
     }
-    const long long limit = max(1ll, sy.bar.limit >> 3);   // a poll here takes some eight of the barrier's
+    auto counts = [&](int first, int step) {   // of the bodies first, first + step, ...: solves and preSolves done
+        unsigned all = 0;
+        for (int d = first; d < nd; d += step)
+            all += *(volatile unsigned*)&vt[2 * d].w + *(volatile unsigned*)&w.pv_w[ds + d].w;
+        return all;
+    };
     for (int sub = 0; sub < substeps; ++sub) {
         for (int q = jq0 + slot; q < jq1; q += nth) make_joint_rows(w, q);
         for (int d = slot; d < nd; d += nth) integrate_velocity<true>(w, ds + d, ds, h, g, GlobVel{vt});
@@ -1272,6 +1283,7 @@ __device__ void solve_flow(const World& w, FrameBuf& f, int s, const GridSync& s
             }
         };
         settle();
+        unsigned seen = 0;   // the counts when this warp last added them up
         for (long long polls = 0; __any_sync(~0u, kind != FLOW_DONE);) {
             PairVel pv = {};
             float4 ps0 = make_float4(0, 0, 0, 0), pw0 = ps0, ps1 = ps0, pw1 = ps0;
@@ -1328,19 +1340,25 @@ __device__ void solve_flow(const World& w, FrameBuf& f, int s, const GridSync& s
                 settle();
                 polls = 0;
             } else if (kind != FLOW_DONE) {
-                ++polls;
-                const bool over = polls > limit;
-                if (over) atomicOr(w.err, ERR_BARRIER_TIMEOUT);
-                // a wait that ran out here or elsewhere ends the lane's list; the grid leaves at the next barrier
-                if (over || ((polls & 63) == 0 && (*(volatile int*)w.err & ERR_BARRIER_TIMEOUT))) kind = FLOW_DONE;
+                // a wait that ran out, here or elsewhere, ends the lane's list; the grid leaves at the next barrier
+                if ((++polls & 63) == 0 && (*(volatile int*)w.err & ERR_BARRIER_TIMEOUT)) kind = FLOW_DONE;
             }
             if (!__any_sync(~0u, ready)) {
-                // nothing to do yet: the further the nearest solve, the longer the pause
-                const int near = __reduce_min_sync(~0u, kind == FLOW_DONE ? 1 << 20 : lag);
+                // nothing to do yet: the further the nearest solve, the longer the pause (-1: a wait at its limit)
+                const int near = __reduce_min_sync(~0u, kind == FLOW_DONE ? 1 << 20 : polls > sy.bar.limit ? -1 : lag);
+                if (near < 0) {
+                    const unsigned all = __reduce_add_sync(~0u, counts(slot & 31, 32));
+                    if (all == seen && kind != FLOW_DONE && polls > sy.bar.limit) {
+                        atomicOr(w.err, ERR_BARRIER_TIMEOUT);
+                        kind = FLOW_DONE;
+                    }
+                    if (all != seen) polls = 0;
+                    seen = all;
+                }
                 __nanosleep(near > 3 ? 400 : 40);
             }
         }
-        sy.sync();
+        sy.bar.sync([&] { return counts(0, 1); });
     }
     // accumulated impulses back into the frame's contacts (inspection only)
     for (int k = slot; k < ncl; k += nth) {

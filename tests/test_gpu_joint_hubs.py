@@ -113,3 +113,21 @@ def test_hub_at_the_limit_of_the_counts(n, gpu_lib):
 def test_kinematic_toggles_of_jointed_bodies(gpu_lib, oracle_lib):
     s = scenes.joint_chains(n_chains=6, links=9, substeps=3, iterations=3)
     _lockstep(s, 24, deltas=delta_schedule(s, 24, seed=11, every=2))
+
+
+def test_a_wait_through_many_sweeps_is_not_a_timeout(gpu_lib):
+    """The position of a body whose joints other lanes solve waits for every iteration of the
+    substep; a limit that each barrier keeps does not end it."""
+    from physecs_gb300.api import World
+    s = _hub(40, scenes.JOINT_SPHERICAL)
+    s.num_substeps, s.num_iterations = 1, 400
+    g, b = World([s], **GRID), World([s], block_scene_max_dyn=1 << 20)
+    g.set_wait_limit(4096)
+    g.step()
+    g.synchronize()
+    b.step()
+    x, y = g.read_bodies(), b.read_bodies()
+    for k in x:
+        assert np.array_equal(x[k].view(np.uint32), y[k].view(np.uint32)), k
+    g.close()
+    b.close()
