@@ -903,7 +903,13 @@ PSX_API psx_status psx_world_raycast(psx_world* W, int32_t n, const psx_ray* ray
                 const int b = W->h_col_body[c];
                 ids[c] = make_int4(b - W->h_scene_body[s], W->h_col_local[c], (int)W->h_entity[b], 0);
             }
-        PSX_TRY(W->upload(W->hit_ids, ids));
+        // on the world's stream, which orders it before the kernel that reads it (a pageable copy
+        // on the legacy stream may return with the data only staged)
+        int4* table = nullptr;
+        PSX_TRY(W->alloc(table, ids.size()));
+        if (!ids.empty()) PSX_CUDA(cudaMemcpyAsync(table, ids.data(), sizeof(int4) * ids.size(), cudaMemcpyHostToDevice, W->stream));
+        PSX_CUDA(cudaStreamSynchronize(W->stream));   // ids goes out of scope
+        W->hit_ids = table;
     }
     const size_t in_b = align256(sizeof(RayIn) * n), acc_b = accept ? align256(nb) : 0, out_b = sizeof(RayOut) * n;
     char* buf = nullptr;
@@ -916,9 +922,10 @@ PSX_API psx_status psx_world_raycast(psx_world* W, int32_t n, const psx_ray* ray
     if (accept) PSX_CUDA(cudaMemcpyAsync(d_acc, accept, nb, cudaMemcpyHostToDevice, st));
     query_trees(W);
     launch_raycast(W->w, W->f, d_in, n, d_acc, W->hit_ids, d_out, st);
+    PSX_CUDA(cudaStreamSynchronize(st));
+    PSX_TRY(check_err(W));   // before the caller's array is written
     PSX_CUDA(cudaMemcpyAsync(hits, d_out, sizeof(RayOut) * n, cudaMemcpyDeviceToHost, st));
     PSX_CUDA(cudaStreamSynchronize(st));
-    PSX_TRY(check_err(W));
     return PSX_OK;
 }
 
