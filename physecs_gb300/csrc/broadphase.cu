@@ -11,6 +11,7 @@
 // partner collider.
 #include "frame.cuh"
 #include "ordkey.cuh"
+#include "smem_limit.cuh"
 #include "narrow_convex.cuh"
 
 namespace psx {
@@ -879,15 +880,11 @@ __global__ void __launch_bounds__(1024) k_scene_tree(World w, FrameBuf f, int pm
 
 template <bool ALL>
 static void launch_scene_tree(const World& w, FrameBuf& f, int pmax, cudaStream_t s) {
-    constexpr int kMaxDevices = 64;
-    static int done[kMaxDevices] = {};
+    static SmemLimit limit;
     const int bytes = (int)scene_tree_bytes(pmax);
     int dev = 0;
     cudaGetDevice(&dev);
-    if (dev >= 0 && dev < kMaxDevices && done[dev] < bytes) {
-        cudaFuncSetAttribute(k_scene_tree<ALL>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-        done[dev] = bytes;
-    }
+    limit.raise(dev, bytes, [](int b) { cudaFuncSetAttribute(k_scene_tree<ALL>, cudaFuncAttributeMaxDynamicSharedMemorySize, b); });
     // few scenes: a block as wide as its sort has pairs, for latency
     const int threads = w.n_scenes <= 152 ? std::max(kBoundsThreads, std::min(1024, pmax / 2)) : kBoundsThreads;
     k_scene_tree<ALL><<<w.n_scenes, threads, bytes, s>>>(w, f, pmax);

@@ -16,6 +16,7 @@
 // theirs (solve_flow), with grid barriers between phases.  Every wait is bounded.
 #include <cooperative_groups.h>
 #include "libm_f32.cuh"
+#include "smem_limit.cuh"
 #include "solver_words.cuh"
 #include <algorithm>
 #include "frame.cuh"
@@ -1533,24 +1534,16 @@ int solver_grid_blocks() {
     return sms * per;
 }
 
-// The dynamic shared memory a kernel may use is a per-device attribute: it is set on
-// the current device whenever a launch there asks for more than was set before.
-constexpr int kMaxDevices = 64;
-
-static void set_kernel_smem(const void* fn, int* done, int bytes) {
+static void set_kernel_smem(const void* fn, SmemLimit& limit, int bytes) {
     int dev = 0;
     cudaGetDevice(&dev);
-    if (dev < 0 || dev >= kMaxDevices) return;
-    if (done[dev] < bytes) {
-        cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-        done[dev] = bytes;
-    }
+    limit.raise(dev, bytes, [fn](int b) { cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, b); });
 }
 
 template <int NT>
 static void set_smem(int bytes) {
-    static int done[kMaxDevices] = {};
-    set_kernel_smem((const void*)k_solve_block<NT>, done, bytes);
+    static SmemLimit limit;
+    set_kernel_smem((const void*)k_solve_block<NT>, limit, bytes);
 }
 
 // A solver launch at a scheduling priority: `rank` 0 is the device's highest, each step
@@ -1632,7 +1625,7 @@ int launch_solver(const World& w, FrameBuf& f, const SolverLaunch& L, cudaStream
     if (L.n_tier[1]) cudaStreamWaitEvent(s, L.tjoin[1], 0);
     if (L.n_large) cudaStreamWaitEvent(s, L.join, 0);
     if (L.n_cluster) {
-        static int cluster_smem[kMaxDevices] = {};
+        static SmemLimit cluster_smem;
         set_kernel_smem((const void*)k_solve_cluster<512>, cluster_smem, L.smem_large);
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(kClusterBlocks * L.n_cluster);
