@@ -593,7 +593,7 @@ __device__ __forceinline__ M3 world_invI(const World& w, int d) {
 __device__ void contact_header(const World& w, const Contact& c, int ds, int slots, SHdr& H) {
     H.n = c.n;
     H.m = make_float4(c.b0 >= 0 ? w.com[c.b0].w : 0.f, c.b1 >= 0 ? w.com[c.b1].w : 0.f, c.frequency, c.damping);
-    H.i = make_int4(c.b0 >= 0 ? c.b0 - ds : -1, c.b1 >= 0 ? c.b1 - ds : -1, c.np | (c.soft << 8) | (slot_step(slots) << 9), slot_first(slots));
+    H.i = make_int4(c.b0 >= 0 ? c.b0 - ds : -1, c.b1 >= 0 ? c.b1 - ds : -1, c.np | (c.soft ? HDR_SOFT : 0) | (slot_step(slots) << HDR_STEP), slot_first(slots));
 }
 
 // A contact's rows for one substep: the row update (src/Physecs.cpp:366-427), which reads
@@ -601,10 +601,10 @@ __device__ void contact_header(const World& w, const Contact& c, int ds, int slo
 // (src/ContactConstraints.cpp:4-31) and the per-substep constants of solve (:33-101), which
 // read the integrated ones (vr).  `last`: the substep's separations stay with the contact.
 template <class V>
-__device__ void contact_rows(const World& w, Contact& c, const SHdr& H, SPt* __restrict__ P, float h, bool last, const V vr) {
+__device__ void contact_rows(const World& w, Contact& c, SHdr& H, SPt* __restrict__ P, float h, bool last, const V vr) {
     const int4 id = *reinterpret_cast<const int4*>(&c.b0);   // b0, b1, body0, body1
-    const int b0 = id.x, b1 = id.y, np = H.i.z & 0xff, step = H.i.z >> 9;
-    const bool soft = (H.i.z & 0x100) != 0;
+    const int b0 = id.x, b1 = id.y, np = H.i.z & 0xff, step = H.i.z >> HDR_STEP;
+    const bool soft = (H.i.z & HDR_SOFT) != 0;
     const float im0 = H.m.x, im1 = H.m.y;
     V3 com0 = {0, 0, 0}, v0 = {0, 0, 0}, w0 = {0, 0, 0}, com1 = {0, 0, 0}, v1 = {0, 0, 0}, w1 = {0, 0, 0};
     V3 nv0 = {0, 0, 0}, nw0 = {0, 0, 0}, nv1 = {0, 0, 0}, nw1 = {0, 0, 0};
@@ -623,6 +623,7 @@ __device__ void contact_rows(const World& w, Contact& c, const SHdr& H, SPt* __r
         vr.ld(H.i.y, nv1, nw1);
     } else q1 = ld4(w.quat[id.w]);
     const V3 n = ld3(H.n);
+    bool whole = np == 4;   // every row of the widest form is live
     for (int k = 0; k < np; ++k) {
         const float4 l0 = c.p[k].r0;
         const V3 r0 = qrot(q0, ld3(l0)), r1 = qrot(q1, ld3(c.p[k].r1));
@@ -658,6 +659,7 @@ __device__ void contact_rows(const World& w, Contact& c, const SHdr& H, SPt* __r
             lamT = rv / invT;
         }
         const int live = (invN ? 1 : 0) | (invT ? 2 : 0);
+        whole &= live == 3;
         SPt& p = P[k * step];
         p.a = make_float4(-r0xn.x, r1xn.x, -r0xn.y, r1xn.y);
         p.b = make_float4(-r0xn.z, r1xn.z, r0xnt.x, -r1xnt.x);
@@ -668,6 +670,10 @@ __device__ void contact_rows(const World& w, Contact& c, const SHdr& H, SPt* __r
         p.g = make_float4(r0xtt.z, -r1xtt.z, lamT, __int_as_float(live));
         if (last) c.p[k].r1.w = cc;
     }
+    // a -0 among the velocities; no sweep makes one that was not there (its bits are the least integer)
+    auto least = [](const V3& a) { return min(min(__float_as_int(a.x), __float_as_int(a.y)), __float_as_int(a.z)); };
+    const bool minus0 = !whole && min(min(least(nv0), least(nw0)), min(least(nv1), least(nw1))) == (int)0x80000000;
+    if (minus0 != ((H.i.z & HDR_MINUS0) != 0)) H.i.z ^= HDR_MINUS0;
 }
 
 // Two floats in one 64-bit register; the packed operations round each lane as the scalar
@@ -690,7 +696,7 @@ __device__ __forceinline__ F2 dot(const F2x3& a, const F2x3& b) { return a.x * b
 __device__ __forceinline__ void axpy(F2x3& a, F2 s, const F2x3& b) { a = {a.x + s * b.x, a.y + s * b.y, a.z + s * b.z}; }
 
 // ContactConstraints::solve (src/ContactConstraints.cpp:33-124) of a contact with at most
-// N points; SOFT: the contact may be soft.  No other thread touches the contact's bodies
+// N points; ANY: the contact may be soft or hold a -0 (below).  No other thread touches the contact's bodies
 // within its colour, so their velocities stay in registers from the first point to the
 // last; every value equals a reload after each point.
 // The step is one dependent chain of up to 2 N rows, so it is written for latency and
@@ -703,13 +709,17 @@ __device__ __forceinline__ void axpy(F2x3& a, F2 s, const F2x3& b) { a = {a.x + 
 //     live (the reference skips a row whose inverse effective mass is zero; a contact may
 //     have fewer than N points) or a side has no simulated body, so the chain has no
 //     branches.  A live row's operations and their order are the reference's (x - l * n
-//     is formed as x + l * (-n), which rounds the same).
+//     is formed as x + l * (-n), which rounds the same).  Adding a row of zeros changes
+//     one value, a -0 to +0, so a contact that starts the substep with a -0 among its
+//     velocities (HDR_MINUS0) takes the form that branches around rows that are not live.
+//     (Selects there took registers from every form: 2.4 % of a frame of 2000 bodies; the
+//     branches nothing.)
 struct PairVel { V3 v0, w0, v1, w1; };   // a contact's or joint's velocities; zero on a side that is not simulated
-template <int N, bool SOFT>
+template <int N, bool ANY>
 __device__ __forceinline__ bool contact_solve(const SHdr& H, SPt* __restrict__ P, bool useBias, PairVel& pv) {
     const float friction = H.n.w;
-    const int np = H.i.z & 0xff, step = H.i.z >> 9;
-    const bool soft = SOFT && (H.i.z & 0x100) != 0;
+    const int np = H.i.z & 0xff, step = H.i.z >> HDR_STEP;
+    const bool soft = ANY && (H.i.z & HDR_SOFT) != 0;
     const bool sim0 = H.i.x >= 0, sim1 = H.i.y >= 0;
     const F2 im = f2(H.m.x, H.m.y);
     const F2x3 nm = {f2(-H.n.x, H.n.x), f2(-H.n.y, H.n.y), f2(-H.n.z, H.n.z)};
@@ -746,8 +756,10 @@ __device__ __forceinline__ bool contact_solve(const SHdr& H, SPt* __restrict__ P
         lamN[i] = on ? tot : prev;
         lambda = tot - prev;
         const F2 l = f2(on && sim0 ? lambda : 0.f, on && sim1 ? lambda : 0.f);
-        axpy(v, l * im, np3);
-        axpy(o, l, F2x3{f2(B[i].z, B[i].w), f2(C[i].x, C[i].y), f2(C[i].z, C[i].w)});
+        if (!ANY || on) {
+            axpy(v, l * im, np3);
+            axpy(o, l, F2x3{f2(B[i].z, B[i].w), f2(C[i].x, C[i].y), f2(C[i].z, C[i].w)});
+        }
         touched |= on;
     }
     float4 E[N], F[N], G[N];
@@ -767,8 +779,10 @@ __device__ __forceinline__ bool contact_solve(const SHdr& H, SPt* __restrict__ P
         lamT[i] = tot;
         lambda = tot - prev;
         const F2 l = f2(on && sim0 ? lambda : 0.f, on && sim1 ? lambda : 0.f);
-        axpy(v, l * im, F2x3{f2(E[i].x, -E[i].x), f2(E[i].y, -E[i].y), f2(E[i].z, -E[i].z)});
-        axpy(o, l, F2x3{f2(F[i].x, F[i].y), f2(F[i].z, F[i].w), f2(G[i].x, G[i].y)});
+        if (!ANY || on) {
+            axpy(v, l * im, F2x3{f2(E[i].x, -E[i].x), f2(E[i].y, -E[i].y), f2(E[i].z, -E[i].z)});
+            axpy(o, l, F2x3{f2(F[i].x, F[i].y), f2(F[i].z, F[i].w), f2(G[i].x, G[i].y)});
+        }
         touched |= on;
     }
 #pragma unroll
@@ -787,9 +801,9 @@ __device__ __forceinline__ bool contact_solve(const SHdr& H, SPt* __restrict__ P
 // The vote only chooses among forms that all give this contact's result.
 __device__ __forceinline__ bool contact_forms(const SHdr& H, SPt* __restrict__ P, bool useBias, PairVel& pv) {
     const int np = H.i.z & 0xff;
-    const bool soft = (H.i.z & 0x100) != 0;
+    const bool any = (H.i.z & (HDR_SOFT | HDR_MINUS0)) != 0;
     const unsigned lanes = __activemask();
-    if (__any_sync(lanes, soft)) return contact_solve<4, true>(H, P, useBias, pv);
+    if (__any_sync(lanes, any)) return contact_solve<4, true>(H, P, useBias, pv);
     if (!__any_sync(lanes, np > 1)) return contact_solve<1, false>(H, P, useBias, pv);
     if (!__any_sync(lanes, np > 2)) return contact_solve<2, false>(H, P, useBias, pv);
     return contact_solve<4, false>(H, P, useBias, pv);
@@ -798,7 +812,7 @@ __device__ __forceinline__ bool contact_forms(const SHdr& H, SPt* __restrict__ P
 template <class V>
 __device__ __forceinline__ void contact_step(const SHdr* __restrict__ Hp, SPt* __restrict__ points, bool useBias, const V vr) {
     const SHdr H = *Hp;
-    if ((H.i.z & 0x100) && !useBias) return;   // the relaxation skips soft contacts
+    if ((H.i.z & HDR_SOFT) && !useBias) return;   // the relaxation skips soft contacts
     const int b0 = H.i.x, b1 = H.i.y;
     PairVel pv = {};
     if (b0 >= 0) vr.ld(b0, pv.v0, pv.w0);
@@ -1085,7 +1099,7 @@ __device__ void solve_substeps(const World& w, FrameBuf& f, int s, const S& sy, 
         for (int d = ds + tid; d < de; d += nth) integrate_velocity<false>(w, d, ds, h, g, vr);
         sy.sync();
         for (int k = tid; k < ncl; k += nth) {
-            const SHdr& H = HK(k);
+            SHdr& H = HK(k);
             contact_rows(w, f.contacts[f.corder[ms + k]], H, PK(k) + H.i.w, h, sub == substeps - 1, vr);
         }
         for (int st = js0; st < js1; ++st) {
@@ -1133,7 +1147,7 @@ __device__ void solve_substeps(const World& w, FrameBuf& f, int s, const S& sy, 
         Contact& c = f.contacts[f.corder[ms + k]];
         const SHdr& H = HK(k);
         const SPt* q = PK(k) + H.i.w;
-        const int step = H.i.z >> 9;
+        const int step = H.i.z >> HDR_STEP;
         for (int i = 0; i < c.np; ++i) c.lambda[i] = make_float2(q[i * step].d.x, q[i * step].e.w);
     }
 }
@@ -1320,7 +1334,7 @@ __device__ void solve_flow(const World& w, FrameBuf& f, int s, const GridSync& s
             if (ready) {
                 if (kind == FLOW_CONTACT) {
                     const bool bias = it < iterations;
-                    if (bias || !(hi.z & 0x100)) contact_forms(Hg[idx], Pg + hi.w, bias, pv);
+                    if (bias || !(hi.z & HDR_SOFT)) contact_forms(Hg[idx], Pg + hi.w, bias, pv);
                 } else if (kind == FLOW_JOINT) {
                     if (it < 0) joint_rows_presolve(w, idx, ps0, pw0, ps1, pw1);
                     else joint_rows_solve(w, idx, w.jruns[idx], h, joint_bias, it == 0, pv.v0, pv.w0, pv.v1, pv.w1);
@@ -1366,7 +1380,7 @@ __device__ void solve_flow(const World& w, FrameBuf& f, int s, const GridSync& s
         Contact& c = f.contacts[f.corder[ms + k]];
         const SHdr& H = Hg[k];
         const SPt* q = Pg + H.i.w;
-        const int step = H.i.z >> 9;
+        const int step = H.i.z >> HDR_STEP;
         for (int i = 0; i < c.np; ++i) c.lambda[i] = make_float2(q[i * step].d.x, q[i * step].e.w);
     }
 }

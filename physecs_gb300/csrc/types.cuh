@@ -110,8 +110,10 @@ struct JointDev {
 // Per-substep solver record of one contact (ContactConstraints, src/ContactConstraints.h:31-48),
 // written in colour order:
 //   n = {normal, friction}   m = {invMass0, invMass1, frequency, damping}
-//   i = {scene-local dynamic body 0 or -1, body 1 or -1, numPoints | soft << 8 | step << 9, first
-//        point slot}; the contact's points lie `step` slots apart
+//   i = {scene-local dynamic body 0 or -1, body 1 or -1, numPoints | HDR_* | step << HDR_STEP,
+//        first point slot}; the contact's points lie `step` slots apart
+// HDR_MINUS0: a velocity component of its bodies is -0 as the substep's sweeps begin
+enum : int { HDR_SOFT = 1 << 8, HDR_MINUS0 = 1 << 9, HDR_STEP = 10 };
 struct SHdr {
     float4 n, m;
     int4 i;
