@@ -90,7 +90,7 @@ def prepare_tree():
 
 def build(jobs=8, verbose=False, portable=None):
     """portable: emulate SSE on GCC vector extensions (default: on hosts other than x86)."""
-    if os.path.isdir(REFERENCE):
+    if os.path.isdir(os.path.join(REFERENCE, "src")):   # an empty directory is no checkout
         prepare_tree()
     elif not os.path.isdir(TREE):
         raise RuntimeError("reference sources unavailable: neither %s nor %s exist" % (REFERENCE, TREE))
