@@ -429,7 +429,6 @@ __global__ void k_karras(World w, FrameBuf f) {
     int right = (hi == gamma + 1) ? ~(cs + gamma + 1) : ibase + gamma + 1;
     f.bvh.left[node] = left;
     f.bvh.right[node] = right;
-    f.bvh.first[node] = cs + lo;
     f.bvh.last[node] = cs + hi;
     f.bvh.visits[node] = 0;
     if (left >= 0) f.bvh.parent[left] = node; else f.bvh.leaf_parent[~left] = node;

@@ -30,7 +30,6 @@ struct BVHNodes {
     int* right;
     int* parent;      // parent of internal nodes (global internal index), -1 for roots
     int* leaf_parent; // parent of each sorted leaf
-    int* first;       // sorted-leaf range covered by each internal node
     int* last;
     float4* bmin;
     float4* bmax;

@@ -416,7 +416,7 @@ psx_status psx::rt::build_world(psx_world* W, const psx_scene_desc* scenes, int 
     PSX_TRY(W->alloc(f.radix_hist, radix_hist_ints(n)));
     BVHNodes& v = f.bvh;
     PSX_TRY(W->alloc(v.left, n)); PSX_TRY(W->alloc(v.right, n)); PSX_TRY(W->alloc(v.parent, n));
-    PSX_TRY(W->alloc(v.leaf_parent, n)); PSX_TRY(W->alloc(v.first, n)); PSX_TRY(W->alloc(v.last, n));
+    PSX_TRY(W->alloc(v.leaf_parent, n)); PSX_TRY(W->alloc(v.last, n));
     PSX_TRY(W->alloc(v.bmin, n)); PSX_TRY(W->alloc(v.bmax, n)); PSX_TRY(W->alloc(v.visits, n));
     PSX_TRY(W->alloc(f.leaf_cnt, n));
     PSX_TRY(W->alloc(f.leaf_off, n));
