@@ -498,8 +498,9 @@ PSX_API psx_status psx_world_trigger_events(psx_world* w, psx_trigger_event* out
 PSX_API psx_status psx_world_counts(psx_world* w, int32_t* counts);
 /* counts[4] = {convex-mesh pairs, of them overlapping after GJK (EPA runs on these), of
  *             those the ones that outgrew the lane-per-pair EPA (12 steps), and of those
- *             the ones that outgrew the grouped EPA (36 steps)} of the last frame; EPA
- *             schedules that skip a tier report 0 for it */
+ *             the ones that outgrew the grouped EPA (36 steps)} of the last frame; a tier
+ *             that is skipped reports 0: by the EPA schedule, or, with epa_lanes 1, by a
+ *             frame of at most 1216 overlapping pairs, which all take the full polytope */
 PSX_API psx_status psx_world_narrow_counts(psx_world* w, int32_t* counts);
 /* Inspection of the last frame (synchronises):
  *   pairs: {scene, entity0, collider0, entity1, collider1} per broadphase pair

@@ -230,8 +230,8 @@ class World:
         _check(load().psx_world_set_joint_params(self.h, scene, joint, _p(p)))
 
     def set_wait_limit(self, polls):
-        """psx_world_set_wait_limit: polls of a grid-barrier wait before it gives up
-        (0: the default, about half a second)."""
+        """psx_world_set_wait_limit: polls of a wait in the grid's solver before it gives up
+        (0: the default, 2^23; include/psx.h says what a wait is)."""
         _check(load().psx_world_set_wait_limit(self.h, int(polls)))
 
     def tune(self, frames=2):

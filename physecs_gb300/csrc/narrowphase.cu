@@ -386,12 +386,13 @@ __global__ void __launch_bounds__(32 * WARPS) k_convex_epa(World w, FrameBuf f, 
 // polytope, a warp each: narrowphase stage of 2000 mixed bodies (285 overlapping pairs) 261
 // against 414 us, of 250 bodies 288 against 403.  With 13,000 (65,536 bodies) the warps take
 // 1190 us against 960, with 240,000 (4096 scenes) twice the time.
+constexpr int kFewPairs = 1216;
+
 // EPA for the overlapping pairs (list 3) with one lane per pair and the faces built by the
 // whole warp (narrow_epa_flat.cuh).  Each warp takes pairs from a shared counter as its
 // lanes free up; a pair whose polytope would outgrow the lane's room goes to list 8 for
 // the grouped kernel.  One block of WARPS warps per SM: the polytopes take about 54 KB of
 // shared memory a warp.
-constexpr int kFewPairs = 1216;
 template <int WARPS>
 __global__ void __launch_bounds__(32 * WARPS, 1) k_convex_epa_flat(World w, FrameBuf f) {
     extern __shared__ __align__(16) unsigned char epa_smem[];

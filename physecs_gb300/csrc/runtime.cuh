@@ -78,14 +78,14 @@ struct psx_world {
     long long frames_run = 0;        // frames queued since creation
     int frame_kernels = 0;           // kernels in one frame
     int solver_smem_large = 0;       // the same for the 512-thread blocks of large scenes
-    std::vector<int> large_scenes_h; // block scenes above 1024 dynamic bodies
+    std::vector<int> large_scenes_h; // block scenes above 1024 dynamic bodies, or above 192 (build_world)
     int* large_scenes = nullptr;
     std::vector<int> big_scenes_h;     // scenes above the block limit
     std::vector<int> cluster_scenes_h; // ... solved by a thread-block cluster each
     int* cluster_scenes = nullptr;     // (grid_scenes: the rest; both sized for every big scene)
     int large_mode = 0;                // 1: clusters where they fit, 2: the whole grid
     long long wait_limit = 0;          // polls of a grid-barrier wait before it gives up (0: the default)
-    int large_nt = 512;                // threads per block of the scenes above 1024 dynamic bodies
+    int large_nt = 512;                // threads per block of large_scenes
     psx_world_opts opts_used{};        // the creation options (launch shapes: current_launch)
     std::vector<const int32_t*> forced_colors;   // per scene, while building: joint colours given by the caller
     // block scenes by solver block size (64, 128, 256 threads), each longest first

@@ -1498,7 +1498,8 @@ __device__ void solve_scene(const World& w, FrameBuf& f, int s, const S& sy, int
     }
 }
 
-// one scene per block; NT = 32 or 64, 128 or 256 for scenes up to 1024 dynamic bodies (by size), 512 above
+// one scene per block; by size NT = 32 or 64, 128 or 256, and 512 for the world's large scenes: above
+// 1024 dynamic bodies, or above 192 where no more scenes than SMs are (build_world)
 template <int NT>
 __global__ void __launch_bounds__(NT, 512 / NT) k_solve_block(World w, FrameBuf f, const int* scenes, int smem_f4) {
     BlockSync sy;
